@@ -3,7 +3,7 @@
 A case is a dict of plain values.  ``listed`` gives the named ones, ``draw`` one more of the same
 ranges, ``prepare`` what a program holds before the call (model, engine, batch on the GPU), ``run``
 one pass, ``work`` the bytes and operations that the pass cannot do without, ``tolerance`` how far
-two correct implementations at the same precision may be apart.
+two correct implementations at the same precision may be apart, ``exact`` the outputs in 64 bits.
 
 Kinds: whole training steps of the decoder and convolution models through ``TrainEngine``, the
 forward / backward of a pipeline stage's slice of a model, evaluation passes that return logits,
@@ -14,6 +14,8 @@ from __future__ import annotations
 import math
 
 import torch
+import torch.nn.functional as F
+from torch.utils.checkpoint import checkpoint
 
 from necklace_b200.comm.symm import SymmetricHeap
 from necklace_b200.models.gpt2 import GPT2, GPT2Config
@@ -407,3 +409,198 @@ def tolerance(case: dict):
             "resnet_infer": {"rel": 1.6e-2, "max": 0.07}, "llama_stage": {"rel": 1.2e-2, "max": 0.16},
             "llama_step": {"rel": 3e-2, "max": 0.99}, "attention": {"rel": 1e-2, "max": 0.28},
             "codec": "exact"}[case["kind"]]
+
+
+# -------------------------------------------------------------------------------------- exact
+def exact(case: dict, seed: int):
+    """The outputs of ``run`` in plain torch and 64 bits.  Inputs, weights and the layout of the
+    flat gradient come from the state of ``prepare``.  The updated weights of an optimizer step are
+    left out: Adam's first update is the sign of the gradient.  So is the whole convolution step,
+    whose gradients have no digits to compare (see ``tolerance``)."""
+    kind = case["kind"]
+    if kind == "resnet_step":
+        return None
+    st = prepare(case, seed)
+    with torch.enable_grad():
+        return _EXACT[kind](case, st)
+
+
+def _leaves64(flat):
+    return {n: p.detach().double().requires_grad_(True) for n, p in zip(flat.names, flat.params)}
+
+
+def _flat_grad64(flat, w):
+    """The gradients at their places in the flat buffer."""
+    out = torch.zeros(flat.numel, dtype=torch.float64, device=DEV)
+    for n, o in zip(flat.names, flat.offsets):
+        if w[n].grad is not None:
+            out[o:o + w[n].numel()] = w[n].grad.reshape(-1)
+    return out
+
+
+def _softmax_attention64(q, k, v, causal):
+    s = (q @ k.transpose(-1, -2)) / math.sqrt(q.shape[-1])
+    if causal:
+        s = s.masked_fill(~torch.ones(s.shape[-2:], dtype=torch.bool, device=DEV).tril(),
+                          float("-inf"))
+    return torch.softmax(s, -1) @ v
+
+
+def _attention64(qkv, H, causal, rotate=False):
+    B, S, C3 = qkv.shape
+    q, k, v = qkv.view(B, S, 3, H, C3 // 3 // H).permute(2, 0, 3, 1, 4)
+    if rotate:
+        half = q.shape[-1] // 2
+        a = torch.arange(S, dtype=torch.float64, device=DEV)[:, None] * 10000.0 ** (
+            -torch.arange(half, dtype=torch.float64, device=DEV) / half)
+        cos, sin = a.cos(), a.sin()
+        q, k = (torch.cat([t[..., :half] * cos - t[..., half:] * sin,
+                           t[..., half:] * cos + t[..., :half] * sin], -1) for t in (q, k))
+    # a head of every sample at a time: the score matrices of all heads take too much memory
+    out = [checkpoint(_softmax_attention64, q[:, h], k[:, h], v[:, h], causal, use_reentrant=False)
+           for h in range(H)]
+    return torch.stack(out, 2).reshape(B, S, C3 // 3)
+
+
+def _gpt2_block64(x, w, pre, H):
+    C = x.shape[-1]
+
+    def ln(t, n):
+        return F.layer_norm(t, (C,), w[pre + n + ".weight"], w[pre + n + ".bias"], 1e-5)
+
+    def lin(t, n):
+        return t @ w[pre + "w_" + n].t() + w[pre + "b_" + n]
+
+    x = x + lin(_attention64(lin(ln(x, "ln1"), "qkv"), H, True), "proj")
+    return x + lin(F.gelu(lin(ln(x, "ln2"), "fc1"), approximate="tanh"), "fc2")
+
+
+def _gpt2_logits64(c, w, idx):
+    table = w["embed.emb.wte"]
+    x = table[idx] + w["embed.emb.wpe"][:idx.shape[1]]
+    for i in range(c["n_layer"]):
+        x = checkpoint(_gpt2_block64, x, w, f"blocks.{i}.", c["n_head"], use_reentrant=False)
+    x = F.layer_norm(x, x.shape[-1:], w["head.ln_f.weight"], w["head.ln_f.bias"], 1e-5)
+    return x @ table[:c["vocab"]].t()
+
+
+def _llama_block64(x, w, pre, H):
+    def rms(t, n):
+        return t * torch.rsqrt(t.square().mean(-1, keepdim=True) + 1e-6) * w[pre + n + ".weight"]
+
+    x = x + _attention64(rms(x, "ln1") @ w[pre + "w_qkv"].t(), H, True, True) @ w[pre + "w_o"].t()
+    g, u = (rms(x, "ln2") @ w[pre + "w_gu"].t()).chunk(2, -1)
+    return x + (F.silu(g) * u) @ w[pre + "w_down"].t()
+
+
+def _llama_blocks64(c, w, x):
+    for i in range(c["n_layer"]):
+        x = checkpoint(_llama_block64, x, w, f"blocks.{i}.", c["n_head"], use_reentrant=False)
+    return x
+
+
+def _llama_logits64(c, w, idx):
+    x = _llama_blocks64(c, w, w["embed.wte"][idx])
+    x = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * w["head.norm.weight"]
+    return x @ w["head.w_out"][:c["vocab"]].t()
+
+
+def _exact_step(c, st):
+    flat = st["engine"].flat
+    w, total = _leaves64(flat), 0.0
+    logits = _gpt2_logits64 if c["kind"] == "gpt2_step" else _llama_logits64
+    k = c.get("micro", 1)
+    for x, y in zip(st["x"].chunk(k), st["y"].chunk(k)):
+        loss = F.cross_entropy(logits(c, w, x).flatten(0, 1), y.reshape(-1), ignore_index=-100)
+        loss.backward()
+        total = total + loss.detach() / k
+    return {"loss": total, "grads": _flat_grad64(flat, w), "weights": None}
+
+
+def _exact_gpt2_logits(c, st):
+    with torch.no_grad():
+        w = {n: p.double() for n, p in st["model"].named_parameters()}
+        return _gpt2_logits64(c, w, st["x"])
+
+
+def _there_and_back64(st, w, fn):
+    x = st["x"].detach().double().requires_grad_(True)
+    y = fn(x)
+    y.backward(st["dy"].double())
+    return {"y": y.detach(), "dx": x.grad, "grads": _flat_grad64(st["flat"], w)}
+
+
+def _exact_llama_stage(c, st):
+    if not c["backward"]:
+        with torch.no_grad():
+            w = {n: p.double() for n, p in st["model"].named_parameters()}
+            return _llama_blocks64(c, w, st["x"].double())
+    w = _leaves64(st["flat"])
+    return _there_and_back64(st, w, lambda x: _llama_blocks64(c, w, x))
+
+
+def _conv64(x, w, k, stride, pad):
+    """``x`` [N, H, W, C], ``w`` [out, (kh, kw, c) and padding]."""
+    N, H, W, C = x.shape
+    t = F.pad(x, (0, 0, pad, pad, pad, pad))
+    h, v = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1
+    taps = [t[:, i:i + (h - 1) * stride + 1:stride, j:j + (v - 1) * stride + 1:stride]
+            for i in range(k) for j in range(k)]
+    return torch.cat(taps, -1) @ w[:, :k * k * C].t()
+
+
+def _exact_conv_unit(c, st):
+    w = _leaves64(st["flat"])
+
+    def fn(x):
+        y = _conv64(x, w["0.weight"], c["k"], c["stride"], c["k"] // 2)
+        var, mean = torch.var_mean(y, (0, 1, 2), unbiased=False)
+        return torch.relu((y - mean) * torch.rsqrt(var + 1e-5) * w["1.weight"] + w["1.bias"])
+
+    return _there_and_back64(st, w, fn)
+
+
+def _exact_resnet_infer(c, st):
+    net = st["model"]
+
+    def unit(x, conv, bn):
+        y = _conv64(x, conv.weight.double(), conv.k, conv.stride, conv.pad)
+        a = bn.weight.double() * torch.rsqrt(bn.running_var.double() + 1e-5)
+        return (y - bn.running_mean.double()) * a + bn.bias.double()
+
+    def features(x):
+        x = torch.relu(unit(x, net.conv1, net.bn1)).permute(0, 3, 1, 2)
+        x = F.max_pool2d(x, 3, 2, 1).permute(0, 2, 3, 1)
+        for layer in (net.layer1, net.layer2, net.layer3, net.layer4):
+            for b in layer:
+                idt = x if b.down_conv is None else unit(x, b.down_conv, b.down_bn)
+                y = torch.relu(unit(torch.relu(unit(x, b.conv1, b.bn1)), b.conv2, b.bn2))
+                x = torch.relu(unit(y, b.conv3, b.bn3) + idt)
+        return x.mean((1, 2))
+
+    with torch.no_grad():
+        f = torch.cat([features(x.double()) for x in st["x"].split(32)])
+        return f @ net.fc_weight.double()[:1000].t() + net.fc_bias.double()[:1000]
+
+
+def _exact_attention(c, st):
+    qkv = st["qkv"].detach().double().requires_grad_(c["backward"])
+    out = _attention64(qkv, c["H"], c["causal"])
+    if not c["backward"]:
+        return out
+    out.backward(st["dout"].double())
+    return {"out": out.detach(), "dqkv": qkv.grad}
+
+
+def _exact_codec(c, st):
+    # which value is over the threshold is decided on the 32-bit sum
+    a = st["grad"].float() + (st["residual"] if not c["ncol"] else 0.0)
+    thr = float(torch.tensor(st["thr"], dtype=torch.float32))
+    dec = (a >= thr).double().mul_(thr) - (a <= -thr).double().mul_(thr)
+    return {"codes": None, "residual": a.double() - dec, "decoded": dec}
+
+
+_EXACT = {"gpt2_step": _exact_step, "llama_step": _exact_step, "gpt2_logits": _exact_gpt2_logits,
+          "llama_stage": _exact_llama_stage, "conv_unit": _exact_conv_unit,
+          "resnet_infer": _exact_resnet_infer, "attention": _exact_attention,
+          "codec": _exact_codec}
