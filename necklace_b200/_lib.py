@@ -72,6 +72,11 @@ _SIGS = {
     "nkb_swiglu_bwd": [vp, vp, vp, i64, i32, vp],
     "nkb_im2col_nhwc": [vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp],
     "nkb_col2im_nhwc": [vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp],
+    "nkb_conv_fwd": [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp],
+    "nkb_conv_dgrad": [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp],
+    "nkb_conv_wgrad_split": [i32, i32, i32, i32, i32, i32, i32, i32, i32],
+    "nkb_conv_wgrad": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp,
+                       vp],
     "nkb_bn_fwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, f32, i32, vp],
     "nkb_bn_apply": [vp, vp, vp, vp, vp, vp, i64, i32, i32, vp],
     "nkb_bn_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, vp, i64, i32, i32, vp],

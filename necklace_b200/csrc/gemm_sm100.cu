@@ -1422,6 +1422,26 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* base, long long inner, long 
   return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
 }
 
+// bf16 tensor map of any rank: extents and box in elements, strides (of dimension 1 and up) in
+// bytes, traversal strides; 128-byte swizzle, zero outside.
+int make_tmap_bf16_nd(CUtensorMap* out, const void* base, int rank, const long long* dims,
+                      const long long* strides, const int* box, const int* estr) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return -1;
+  cuuint64_t gdim[5], gstride[4];
+  cuuint32_t b[5], e[5];
+  for (int i = 0; i < rank; ++i) {
+    gdim[i] = (cuuint64_t)dims[i];
+    b[i] = (cuuint32_t)box[i];
+    e[i] = (cuuint32_t)estr[i];
+    if (i + 1 < rank) gstride[i] = (cuuint64_t)strides[i];
+  }
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base),
+                  gdim, gstride, b, e, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
+}
+
 static int g_num_sms = 0;
 static int g_pair_enabled = 1;
 static int g_splitk_enabled = 1;

@@ -73,7 +73,7 @@ def set_wait_cycles(cycles: int) -> None:
     flag, on a readiness flag.  The default is about two seconds; a wait that runs out makes
     its kernel record a status code and return (see ``check_status``)."""
     lib = _lib.load()
-    for tu in ("gemm", "attn", "comm"):
+    for tu in ("gemm", "attn", "comm", "conv"):
         fn = getattr(lib, f"nkb_set_wait_cycles_{tu}")
         fn.argtypes = [_lib.i64]
         fn.restype = _lib.i32

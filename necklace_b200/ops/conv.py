@@ -1,8 +1,9 @@
 """Convolution, batch norm (+ residual + ReLU) and pooling on channels-last bf16 tensors.
 
 Tensors are ``[N, H, W, C]`` (NHWC) everywhere, so a 1x1 convolution is a GEMM on the
-activation matrix as it is and every other convolution is a GEMM on a gathered ``col``
-matrix; all GEMMs run on the tcgen05 kernel (``ops.gemm``).  Weights are stored
+activation matrix as it is (``ops.gemm``).  Every other convolution whose channel counts are
+multiples of 8 runs on the tcgen05 convolution kernels, which read shifted boxes of the image
+through 4-D tensor maps; the rest (a 3-channel stem) is a GEMM on a gathered ``col`` matrix.  Weights are stored
 ``[C_out, KH*KW*C_in]`` with the input channel innermost, which is what that GEMM wants as
 its K-major B operand.  CPU tensors take PyTorch reference paths (``F.conv2d`` and friends
 on permuted views), which the CPU test-suite and the GPU numerics tests compare against.
@@ -18,7 +19,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ._common import on_gpu, ptr, scratch, scratch_zero
+from ._common import on_gpu, ptr, scratch_zero, status_word
 from .gemm import _deliver_grad, gemm
 
 
@@ -69,6 +70,53 @@ def col2im(dcol: torch.Tensor, shape, KH: int, KW: int, stride: int, pad: int) -
     return dx
 
 
+def _image_kernels(x, w, KH, KW, stride, pad) -> bool:
+    """Whether the kernels that read the image itself take this layer (else: gather).  The
+    tensor maps want channel counts that are multiples of 8 (16-byte strides) and aligned
+    bases; the data gradient is written for strides 1 and 2; 64 taps fit the argument block."""
+    C, Cout = x.shape[-1], w.shape[0]
+    return (x.is_cuda and C % 8 == 0 and Cout % 8 == 0 and stride <= 2 and KH * KW <= 64
+            and pad < 64 and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+            and x.is_contiguous() and w.is_contiguous() and w.shape[1] == KH * KW * C
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and x.numel() > 0)
+
+
+def _conv_fwd(x, w, KH, KW, stride, pad):
+    N, H, W, C = x.shape
+    y = torch.empty(N, *_out_hw(H, W, KH, KW, stride, pad), w.shape[0], dtype=x.dtype,
+                    device=x.device)
+    _lib.call("nkb_conv_fwd", x.data_ptr(), w.data_ptr(), y.data_ptr(), N, H, W, C, w.shape[0],
+              KH, KW, stride, pad, status_word(x.device).data_ptr(), _lib.stream_ptr())
+    _lib.count_launch()
+    return y
+
+
+def _conv_dgrad(dy, w, shape, KH, KW, stride, pad):
+    N, H, W, C = shape
+    dx = torch.empty(shape, dtype=dy.dtype, device=dy.device)
+    _lib.call("nkb_conv_dgrad", dy.data_ptr(), w.data_ptr(), dx.data_ptr(), N, H, W, C,
+              w.shape[0], KH, KW, stride, pad, status_word(dy.device).data_ptr(),
+              _lib.stream_ptr())
+    _lib.count_launch(min(stride, KH) * min(stride, KW))
+    return dx
+
+
+def _conv_wgrad(x, dy, w, KH, KW, stride, pad, out, acc):
+    N, H, W, C = x.shape
+    geom = (N, H, W, C, w.shape[0], KH, KW, stride, pad)
+    split = _lib.load().nkb_conv_wgrad_split(*geom)
+    ws = torch.empty(max(split, 1), w.numel(), dtype=torch.float32, device=x.device)
+    direct = out is not None and out.dtype == torch.bfloat16 and out.is_contiguous() \
+        and out.data_ptr() % 16 == 0
+    dst = out if direct else torch.empty_like(w)
+    _lib.call("nkb_conv_wgrad", x.data_ptr(), dy.data_ptr(), dst.data_ptr(), ws.data_ptr(), split,
+              *geom, int(acc and direct), status_word(x.device).data_ptr(), _lib.stream_ptr())
+    _lib.count_launch(2)
+    if out is None or direct:
+        return dst
+    return out.add_(dst) if acc else out.copy_(dst)
+
+
 class Conv2dFn(torch.autograd.Function):
     """``y[N,Ho,Wo,Cout] = conv(x[N,H,W,Cin], w[Cout, KH*KW*Cin (padded to 8)])``, no bias."""
 
@@ -80,6 +128,11 @@ class Conv2dFn(torch.autograd.Function):
         ctx.xshape = tuple(x.shape)
         direct = KH == 1 and KW == 1 and stride == 1 and pad == 0 and C % 8 == 0
         ctx.direct = direct
+        ctx.image = not direct and _image_kernels(x, w, KH, KW, stride, pad)
+        if ctx.image:
+            ctx.keep_col = False
+            ctx.save_for_backward(x, w)
+            return _conv_fwd(x, w, KH, KW, stride, pad)
         a = x.reshape(-1, C) if direct else im2col(x, KH, KW, stride, pad)
         y = gemm(a, w)
         # the gathered matrix is kept for the weight gradient unless it would be very large
@@ -105,6 +158,11 @@ class Conv2dFn(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
+        if ctx.image and x.is_contiguous() and \
+                not (x.data_ptr() | w.data_ptr() | dy2.data_ptr()) % 16:
+            dx = _conv_dgrad(dy2, w, ctx.xshape, *ctx.geom) if ctx.needs_input_grad[0] else None
+            dw = _deliver_grad(w, lambda out, acc: _conv_wgrad(x, dy2, w, *ctx.geom, out, acc))
+            return dx, dw, None, None, None, None
         dx = None
         if ctx.needs_input_grad[0]:
             d = gemm(dy2, w, b_mn=True)                       # [M, Kpad]
