@@ -172,13 +172,20 @@ col2im_kernel(const __nv_bfloat16* __restrict__ dcol, __nv_bfloat16* __restrict_
 // Per-channel sums over the rows of a [M, C] matrix (C % 8 == 0):
 //   MODE 0: acc[0][c] += sum x,        acc[1][c] += sum x^2            (forward statistics)
 //   MODE 1: acc[0][c] += sum dy',      acc[1][c] += sum dy' * xhat     (backward sums)
-// with dy' = dy * (y > 0) when relu (y = the layer's output), xhat = (x - mean) * rstd.
+// with dy' = dy * (y > 0) when relu, xhat = (x - mean) * rstd.  The signs of the layer's output
+// are kept as one bit per element (`mask`, one byte per thread and row): the backward kernels
+// are bound by memory and the output itself would be a third of what they read.
 // Threads: 8 channels each; a block covers `cx` channel chunks x `ry` row lanes.
+//
+// Each thread loads BN_ROWS rows before it uses the first: with one row in flight the 1024
+// threads of an SM (64 registers) kept 32 KB on the way, less than the latency of the
+// memory times its rate.
+constexpr int BN_ROWS = 4;
 template <int MODE>
 __global__ void __launch_bounds__(256)
 bn_sums_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ x,
-               const __nv_bfloat16* __restrict__ y, const float* __restrict__ stats,
-               float* __restrict__ acc, long long M, int C, int cx, int relu) {
+               const uint8_t* __restrict__ mask, const float* __restrict__ stats,
+               float* __restrict__ acc, long long M, int C, int cx) {
   __shared__ float sh[2][256][8 + 1];
   const int ry = 256 / cx;
   const int tx = threadIdx.x % cx, ty = threadIdx.x / cx;
@@ -187,48 +194,56 @@ bn_sums_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restr
 #pragma unroll
   for (int j = 0; j < 8; ++j) s0[j] = s1[j] = 0.f;
   if (c < C && ty < ry) {
-    float mean[8], rstd[8];
+    float mean[8];
     if (MODE == 1) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { mean[j] = stats[c + j]; rstd[j] = stats[C + c + j]; }
+      for (int j = 0; j < 8; ++j) mean[j] = stats[c + j];
     }
-    for (long long r = (long long)blockIdx.y * ry + ty; r < M; r += (long long)gridDim.y * ry) {
-      uint4 va = *reinterpret_cast<const uint4*>(a + r * C + c);
-      uint32_t ua[4] = {va.x, va.y, va.z, va.w};
-      float fa[8];
+    const long long step = (long long)gridDim.y * ry;
+    for (long long r = (long long)blockIdx.y * ry + ty; r < M; r += BN_ROWS * step) {
+      uint4 va[BN_ROWS], vx[BN_ROWS];
+      uint32_t m[BN_ROWS];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float2 f = unpack_bf16x2(ua[j]);
-        fa[2 * j] = f.x; fa[2 * j + 1] = f.y;
-      }
-      if (MODE == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { s0[j] += fa[j]; s1[j] += fa[j] * fa[j]; }
-      } else {
-        uint4 vx = *reinterpret_cast<const uint4*>(x + r * C + c);
-        uint32_t ux[4] = {vx.x, vx.y, vx.z, vx.w};
-        float fx[8];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float2 f = unpack_bf16x2(ux[j]);
-          fx[2 * j] = f.x; fx[2 * j + 1] = f.y;
-        }
-        if (relu) {
-          uint4 vy = *reinterpret_cast<const uint4*>(y + r * C + c);
-          uint32_t uy[4] = {vy.x, vy.y, vy.z, vy.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float2 f = unpack_bf16x2(uy[j]);
-            if (!(f.x > 0.f)) fa[2 * j] = 0.f;
-            if (!(f.y > 0.f)) fa[2 * j + 1] = 0.f;
+      for (int u = 0; u < BN_ROWS; ++u) {
+        const long long off = (r + u * step) * C + c;
+        va[u] = vx[u] = make_uint4(0, 0, 0, 0);
+        m[u] = 0xffu;
+        if (r + u * step < M) {
+          va[u] = *reinterpret_cast<const uint4*>(a + off);
+          if (MODE == 1) {
+            vx[u] = *reinterpret_cast<const uint4*>(x + off);
+            if (mask) m[u] = mask[off >> 3];
           }
         }
+      }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          s0[j] += fa[j];
-          s1[j] += fa[j] * (fx[j] - mean[j]) * rstd[j];
+      for (int u = 0; u < BN_ROWS; ++u) {
+        const uint32_t ua[4] = {va[u].x, va[u].y, va[u].z, va[u].w};
+        const uint32_t ux[4] = {vx[u].x, vx[u].y, vx[u].z, vx[u].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float2 f = unpack_bf16x2(ua[j]);
+          if (MODE == 0) {
+            s0[2 * j] += f.x;
+            s0[2 * j + 1] += f.y;
+            s1[2 * j] += f.x * f.x;
+            s1[2 * j + 1] += f.y * f.y;
+          } else {
+            const float2 g = unpack_bf16x2(ux[j]);
+            if (!(m[u] & (1u << (2 * j)))) f.x = 0.f;
+            if (!(m[u] & (2u << (2 * j)))) f.y = 0.f;
+            s0[2 * j] += f.x;
+            s0[2 * j + 1] += f.y;
+            // rows behind the last one have f = 0
+            s1[2 * j] += f.x * (g.x - mean[2 * j]);
+            s1[2 * j + 1] += f.y * (g.y - mean[2 * j + 1]);
+          }
         }
       }
+    }
+    if (MODE == 1) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s1[j] *= stats[C + c + j];
     }
   }
 #pragma unroll
@@ -277,8 +292,8 @@ __global__ void bn_finalize_kernel(float* __restrict__ acc, float* __restrict__ 
 __global__ void __launch_bounds__(256)
 bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
                 const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
-                const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ y, long long M,
-                int C, int cx, int relu) {
+                const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ y,
+                uint8_t* __restrict__ mask, long long M, int C, int cx, int relu) {
   const int ry = 256 / cx;
   const int tx = threadIdx.x % cx, ty = threadIdx.x / cx;
   const int c = (blockIdx.x * cx + tx) * 8;
@@ -297,25 +312,40 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ s
       sh[2 * j + 1] = fb.y - stats[c + 2 * j + 1] * sc[2 * j + 1];
     }
   }
-  for (long long r = (long long)blockIdx.y * ry + ty; r < M; r += (long long)gridDim.y * ry) {
-    const long long off = r * C + c;
-    uint4 vx = *reinterpret_cast<const uint4*>(x + off);
-    uint32_t ux[4] = {vx.x, vx.y, vx.z, vx.w};
-    uint32_t ur[4] = {0, 0, 0, 0};
-    if (res) {
-      uint4 vr = *reinterpret_cast<const uint4*>(res + off);
-      ur[0] = vr.x; ur[1] = vr.y; ur[2] = vr.z; ur[3] = vr.w;
-    }
-    uint32_t o[4];
+  const long long step = (long long)gridDim.y * ry;
+  for (long long r = (long long)blockIdx.y * ry + ty; r < M; r += BN_ROWS * step) {
+    uint4 vx[BN_ROWS], vr[BN_ROWS];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 fx = unpack_bf16x2(ux[j]), fr = unpack_bf16x2(ur[j]);
-      float a = fx.x * sc[2 * j] + sh[2 * j] + fr.x;
-      float b = fx.y * sc[2 * j + 1] + sh[2 * j + 1] + fr.y;
-      if (relu) { a = fmaxf(a, 0.f); b = fmaxf(b, 0.f); }
-      o[j] = pack_bf16x2(a, b);
+    for (int u = 0; u < BN_ROWS; ++u) {
+      const long long off = (r + u * step) * C + c;
+      vr[u] = make_uint4(0, 0, 0, 0);
+      if (r + u * step < M) {
+        vx[u] = *reinterpret_cast<const uint4*>(x + off);
+        if (res) vr[u] = *reinterpret_cast<const uint4*>(res + off);
+      }
     }
-    *reinterpret_cast<uint4*>(y + off) = make_uint4(o[0], o[1], o[2], o[3]);
+#pragma unroll
+    for (int u = 0; u < BN_ROWS; ++u) {
+      if (r + u * step >= M) break;
+      const long long off = (r + u * step) * C + c;
+      const uint32_t ux[4] = {vx[u].x, vx[u].y, vx[u].z, vx[u].w};
+      const uint32_t ur[4] = {vr[u].x, vr[u].y, vr[u].z, vr[u].w};
+      uint32_t o[4];
+      uint32_t m = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float2 fx = unpack_bf16x2(ux[j]), fr = unpack_bf16x2(ur[j]);
+        float a = fx.x * sc[2 * j] + sh[2 * j] + fr.x;
+        float b = fx.y * sc[2 * j + 1] + sh[2 * j + 1] + fr.y;
+        if (relu) { a = fmaxf(a, 0.f); b = fmaxf(b, 0.f); }
+        o[j] = pack_bf16x2(a, b);
+        // signs of the rounded values: what a comparison of the stored output with zero gives
+        const float2 f = unpack_bf16x2(o[j]);
+        m |= (f.x > 0.f ? 1u : 0u) << (2 * j) | (f.y > 0.f ? 1u : 0u) << (2 * j + 1);
+      }
+      *reinterpret_cast<uint4*>(y + off) = make_uint4(o[0], o[1], o[2], o[3]);
+      if (mask) mask[off >> 3] = (uint8_t)m;
+    }
   }
 }
 
@@ -323,10 +353,10 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ s
 // sums = [2][C] from bn_sums_kernel<1>.  Same thread layout.
 __global__ void __launch_bounds__(256)
 bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                    const __nv_bfloat16* __restrict__ y, const float* __restrict__ stats,
+                    const uint8_t* __restrict__ mask, const float* __restrict__ stats,
                     const float* __restrict__ sums, const __nv_bfloat16* __restrict__ gamma,
                     __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dres, long long M,
-                    int C, int cx, int relu) {
+                    int C, int cx) {
   const int ry = 256 / cx;
   const int tx = threadIdx.x % cx, ty = threadIdx.x / cx;
   const int c = (blockIdx.x * cx + tx) * 8;
@@ -349,31 +379,40 @@ bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
       k3[j] = -k1[j] * (a0 - mean * rstd * a1);
     }
   }
-  for (long long r = (long long)blockIdx.y * ry + ty; r < M; r += (long long)gridDim.y * ry) {
-    const long long off = r * C + c;
-    uint4 vd = *reinterpret_cast<const uint4*>(dy + off);
-    uint4 vx = *reinterpret_cast<const uint4*>(x + off);
-    uint32_t ud[4] = {vd.x, vd.y, vd.z, vd.w}, ux[4] = {vx.x, vx.y, vx.z, vx.w};
-    uint32_t uy[4] = {0, 0, 0, 0};
-    if (relu) {
-      uint4 vy = *reinterpret_cast<const uint4*>(y + off);
-      uy[0] = vy.x; uy[1] = vy.y; uy[2] = vy.z; uy[3] = vy.w;
-    }
-    uint32_t o[4], rr[4];
+  constexpr int U = BN_ROWS / 2;
+  const long long step = (long long)gridDim.y * ry;
+  for (long long r = (long long)blockIdx.y * ry + ty; r < M; r += U * step) {
+    uint4 vd[U], vx[U];
+    uint32_t mk[U];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 fd = unpack_bf16x2(ud[j]), fx = unpack_bf16x2(ux[j]);
-      if (relu) {
-        float2 fy = unpack_bf16x2(uy[j]);
-        if (!(fy.x > 0.f)) fd.x = 0.f;
-        if (!(fy.y > 0.f)) fd.y = 0.f;
+    for (int u = 0; u < U; ++u) {
+      const long long off = (r + u * step) * C + c;
+      if (r + u * step < M) {
+        vd[u] = *reinterpret_cast<const uint4*>(dy + off);
+        vx[u] = *reinterpret_cast<const uint4*>(x + off);
+        mk[u] = mask ? mask[off >> 3] : 0xffu;
       }
-      o[j] = pack_bf16x2(k1[2 * j] * fd.x + k2[2 * j] * fx.x + k3[2 * j],
-                         k1[2 * j + 1] * fd.y + k2[2 * j + 1] * fx.y + k3[2 * j + 1]);
-      rr[j] = pack_bf16x2(fd.x, fd.y);
     }
-    *reinterpret_cast<uint4*>(dx + off) = make_uint4(o[0], o[1], o[2], o[3]);
-    if (dres) *reinterpret_cast<uint4*>(dres + off) = make_uint4(rr[0], rr[1], rr[2], rr[3]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (r + u * step >= M) break;
+      const long long off = (r + u * step) * C + c;
+      const uint32_t ud[4] = {vd[u].x, vd[u].y, vd[u].z, vd[u].w};
+      const uint32_t ux[4] = {vx[u].x, vx[u].y, vx[u].z, vx[u].w};
+      const uint32_t m = mk[u];
+      uint32_t o[4], rr[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float2 fd = unpack_bf16x2(ud[j]), fx = unpack_bf16x2(ux[j]);
+        if (!(m & (1u << (2 * j)))) fd.x = 0.f;
+        if (!(m & (2u << (2 * j)))) fd.y = 0.f;
+        o[j] = pack_bf16x2(k1[2 * j] * fd.x + k2[2 * j] * fx.x + k3[2 * j],
+                           k1[2 * j + 1] * fd.y + k2[2 * j + 1] * fx.y + k3[2 * j + 1]);
+        rr[j] = pack_bf16x2(fd.x, fd.y);
+      }
+      *reinterpret_cast<uint4*>(dx + off) = make_uint4(o[0], o[1], o[2], o[3]);
+      if (dres) *reinterpret_cast<uint4*>(dres + off) = make_uint4(rr[0], rr[1], rr[2], rr[3]);
+    }
   }
 }
 
@@ -601,7 +640,8 @@ static void bn_sums_dims(long long M, int C, int& cx, dim3& grid) {
        (chunks >= 2 ? 2 : 1))));
   const int gx = (chunks + cx - 1) / cx;
   const int ry = 256 / cx;
-  long long gy = (148LL * 8) / gx;
+  // six blocks per SM: one round of the forward sums (40 registers), two of the others (80)
+  long long gy = (148LL * 6) / gx;
   const long long need = (M + ry - 1) / ry;
   if (gy > need) gy = need;
   if (gy < 1) gy = 1;
@@ -610,9 +650,10 @@ static void bn_sums_dims(long long M, int C, int& cx, dim3& grid) {
 }
 
 // Forward: batch statistics of x [M, C], then y = act(bn(x) (+ res)).  acc: fp32 [2][C], zero on
-// entry, left zero.  stats out: fp32 [2][C] (mean, rstd).
+// entry, left zero.  stats out: fp32 [2][C] (mean, rstd).  mask (optional): one bit per element,
+// y > 0, in [M * C / 8] bytes, bit j of byte i for element 8 i + j.
 extern "C" int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, const void* res,
-                          void* y, float* stats, float* acc, float* run_mean, float* run_var,
+                          void* y, void* mask, float* stats, float* acc, float* run_mean, float* run_var,
                           long long M, int C, float eps, float momentum, int relu, void* stream) {
   if (C % 8) return -3;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) |
@@ -624,13 +665,13 @@ extern "C" int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, co
   dim3 grid;
   bn_sums_dims(M, C, cx, grid);
   bn_sums_kernel<0><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), nullptr, nullptr,
-                                         nullptr, acc, M, C, cx, 0);
+                                         nullptr, acc, M, C, cx);
   bn_finalize_kernel<<<(C + 127) / 128, 128, 0, s>>>(acc, stats, run_mean, run_var, M, C, eps,
                                                      momentum);
   bn_apply_kernel<<<grid, 256, 0, s>>>(
       static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
       static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
-      static_cast<__nv_bfloat16*>(y), M, C, cx, relu);
+      static_cast<__nv_bfloat16*>(y), static_cast<uint8_t*>(mask), M, C, cx, relu);
   return (int)cudaGetLastError();
 }
 
@@ -644,32 +685,31 @@ extern "C" int nkb_bn_apply(const void* x, const float* stats, const void* gamma
   bn_apply_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
       static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
-      static_cast<__nv_bfloat16*>(y), M, C, cx, relu);
+      static_cast<__nv_bfloat16*>(y), nullptr, M, C, cx, relu);
   return (int)cudaGetLastError();
 }
 
-// Backward: dx (and dres = relu-masked dy when given), dgamma / dbeta written or accumulated.
-extern "C" int nkb_bn_bwd(const void* dy, const void* x, const void* y, const float* stats,
+// Backward: dx (and dres = dy masked by the ReLU when given), dgamma / dbeta written or
+// accumulated.  mask: what the forward wrote, null without a ReLU.
+extern "C" int nkb_bn_bwd(const void* dy, const void* x, const void* mask, const float* stats,
                           const void* gamma, void* dx, void* dres, void* dgamma, void* dbeta,
-                          int acc_g, int acc_b, float* acc, long long M, int C, int relu,
-                          void* stream) {
+                          int acc_g, int acc_b, float* acc, long long M, int C, void* stream) {
   if (C % 8) return -3;
   if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) |
        reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(gamma)) & 15)
     return -3;
-  if (relu && (y == nullptr || (reinterpret_cast<uintptr_t>(y) & 15))) return -3;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int cx;
   dim3 grid;
   bn_sums_dims(M, C, cx, grid);
   bn_sums_kernel<1><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(dy),
                                          static_cast<const __nv_bfloat16*>(x),
-                                         static_cast<const __nv_bfloat16*>(y), stats, acc, M, C,
-                                         cx, relu);
+                                         static_cast<const uint8_t*>(mask), stats, acc, M, C,
+                                         cx);
   bn_bwd_apply_kernel<<<grid, 256, 0, s>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
-      static_cast<const __nv_bfloat16*>(y), stats, acc, static_cast<const __nv_bfloat16*>(gamma),
-      static_cast<__nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(dres), M, C, cx, relu);
+      static_cast<const uint8_t*>(mask), stats, acc, static_cast<const __nv_bfloat16*>(gamma),
+      static_cast<__nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(dres), M, C, cx);
   bn_param_grad_kernel<<<(C + 127) / 128, 128, 0, s>>>(acc, static_cast<__nv_bfloat16*>(dgamma),
                                                        static_cast<__nv_bfloat16*>(dbeta), C,
                                                        acc_g, acc_b);

@@ -86,15 +86,16 @@ int nkb_conv_wgrad(const void* x, const void* dy, void* dw, float* ws, int split
                    int W, int C, int Cout, int KH, int KW, int stride, int pad, int accumulate,
                    int* status, void* stream);
 // Training-mode batch norm over the rows of x [M, C] (+ residual, + ReLU).  acc: fp32 [2][C]
-// scratch, zero on entry and on exit; stats: fp32 [2][C] = (mean, rstd).
+// scratch, zero on entry and on exit; stats: fp32 [2][C] = (mean, rstd); mask (may be null): the
+// bits y > 0, M * C / 8 bytes, which the backward of a ReLU takes.
 int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, const void* res, void* y,
-               float* stats, float* acc, float* run_mean, float* run_var, long long M, int C,
+               void* mask, float* stats, float* acc, float* run_mean, float* run_var, long long M, int C,
                float eps, float momentum, int relu, void* stream);
 int nkb_bn_apply(const void* x, const float* stats, const void* gamma, const void* beta,
                  const void* res, void* y, long long M, int C, int relu, void* stream);
-int nkb_bn_bwd(const void* dy, const void* x, const void* y, const float* stats, const void* gamma,
-               void* dx, void* dres, void* dgamma, void* dbeta, int acc_g, int acc_b, float* acc,
-               long long M, int C, int relu, void* stream);
+int nkb_bn_bwd(const void* dy, const void* x, const void* mask, const float* stats,
+               const void* gamma, void* dx, void* dres, void* dgamma, void* dbeta, int acc_g,
+               int acc_b, float* acc, long long M, int C, void* stream);
 int nkb_maxpool3x3s2_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C,
                          void* stream);
 int nkb_maxpool3x3s2_bwd(const void* dy, const void* idx, void* dx, int N, int H, int W, int C,

@@ -35,8 +35,9 @@ class Bottleneck(nn.Module):
             self.down_bn = BatchNorm2d(width * 4, device=device)
 
     def forward(self, x):
+        x, out = self.conv1.split(x)     # the residual path's gradient is added in conv1's
         idt = x if self.down_conv is None else self.down_bn(self.down_conv(x))
-        out = self.bn1(self.conv1(x))
+        out = self.bn1(out)
         out = self.bn2(self.conv2(out))
         return self.bn3(self.conv3(out), residual=idt)
 

@@ -174,6 +174,33 @@ class Conv2dFn(torch.autograd.Function):
         return dx, dw, None, None, None, None
 
 
+class Conv1x1SplitFn(torch.autograd.Function):
+    """``(x_alias, y) = (x, conv1x1(x))`` for a block whose input also goes along a residual
+    path, which takes ``x_alias``: both gradients arrive in one backward call and the
+    residual one is added in the epilogue of the data-gradient GEMM."""
+
+    @staticmethod
+    def forward(ctx, x, w):
+        ctx.save_for_backward(x, w)
+        return x.view_as(x), gemm(x.reshape(-1, x.shape[-1]), w).view(*x.shape[:-1], w.shape[0])
+
+    @staticmethod
+    def backward(ctx, dres, dy):
+        x, w = ctx.saved_tensors
+        if dy is None:      # only the residual path was used
+            return dres, None
+        a, dy2 = x.reshape(-1, x.shape[-1]), dy.reshape(-1, dy.shape[-1])
+        if not dy2.is_contiguous():
+            dy2 = dy2.contiguous()
+        dx = None
+        if ctx.needs_input_grad[0]:
+            r2 = dres.reshape(a.shape) if dres is not None else None
+            dx = gemm(dy2, w, b_mn=True, res=r2).view(x.shape)
+        dw = _deliver_grad(w, lambda out, acc: gemm(dy2, a, a_mn=True, b_mn=True, out=out,
+                                                    accumulate=acc))
+        return dx, dw
+
+
 def conv2d(x, w, KH, KW, stride=1, pad=0):
     return Conv2dFn.apply(x, w, KH, KW, stride, pad)
 
@@ -197,6 +224,14 @@ class Conv2d(nn.Module):
 
     def forward(self, x):
         return conv2d(x, self.weight, self.k, self.k, self.stride, self.pad)
+
+    def split(self, x):
+        """``(x, conv(x))`` at the head of a residual block (see ``Conv1x1SplitFn``)."""
+        hooked = self._forward_hooks or self._forward_pre_hooks or self._backward_hooks \
+            or self._backward_pre_hooks         # they see calls of the module
+        if (self.k, self.stride, self.pad) == (1, 1, 0) and x.shape[-1] % 8 == 0 and not hooked:
+            return Conv1x1SplitFn.apply(x, self.weight)
+        return x, self(x)
 
 
 # ------------------------------------------------------------------------ batch norm
@@ -228,24 +263,26 @@ class BatchNormFn(torch.autograd.Function):
                 run_mean.mul_(1 - momentum).add_(momentum * mean)
                 run_var.mul_(1 - momentum).add_(momentum * var * (M / max(M - 1, 1)))
             stats = torch.stack([mean, rstd])
-            y = y.to(x.dtype)
+            y = mask = y.to(x.dtype)
         else:
             assert x.dtype == torch.bfloat16 and x2.is_contiguous() and C % 8 == 0 and C <= 8192
             y = torch.empty_like(x2)
+            mask = torch.empty(M, C // 8, dtype=torch.uint8, device=x.device) if relu else None
             stats = torch.empty(2, C, dtype=torch.float32, device=x.device)
             _lib.call("nkb_bn_fwd", x2.data_ptr(), gamma.data_ptr(), beta.data_ptr(), ptr(r2),
-                      y.data_ptr(), stats.data_ptr(), _bn_acc(C, x.device).data_ptr(),
+                      y.data_ptr(), ptr(mask), stats.data_ptr(), _bn_acc(C, x.device).data_ptr(),
                       ptr(run_mean), ptr(run_var), M, C, float(eps), float(momentum), int(relu),
                       _lib.stream_ptr())
             _lib.count_launch(3)
-        ctx.save_for_backward(x2, y if relu else None, stats, gamma)
+        # for the ReLU: the signs of the output (GPU, one bit each) or the output itself (CPU)
+        ctx.save_for_backward(x2, mask if relu else None, stats, gamma)
         ctx.refs = (gamma, beta)
         ctx.relu, ctx.has_res, ctx.shape = relu, res is not None, x.shape
         return y.view(x.shape)
 
     @staticmethod
     def backward(ctx, dy):
-        x2, y, stats, gamma = ctx.saved_tensors
+        x2, mask, stats, gamma = ctx.saved_tensors
         g_ref, b_ref = ctx.refs
         M, C = x2.shape
         dy2 = dy.reshape(-1, C)
@@ -255,7 +292,7 @@ class BatchNormFn(torch.autograd.Function):
         if not on_gpu(x2):
             d = dy2.float()
             if relu:
-                d = d * (y.float() > 0)
+                d = d * (mask.float() > 0)
             mean, rstd = stats[0], stats[1]
             xhat = (x2.float() - mean) * rstd
             s0, s1 = d.sum(0), (d * xhat).sum(0)
@@ -276,9 +313,9 @@ class BatchNormFn(torch.autograd.Function):
 
         gbuf, gacc, gdirect = target(g_ref)
         bbuf, bacc, bdirect = target(b_ref)
-        _lib.call("nkb_bn_bwd", dy2.data_ptr(), x2.data_ptr(), ptr(y), stats.data_ptr(),
+        _lib.call("nkb_bn_bwd", dy2.data_ptr(), x2.data_ptr(), ptr(mask), stats.data_ptr(),
                   gamma.data_ptr(), dx.data_ptr(), ptr(dres), gbuf.data_ptr(), bbuf.data_ptr(),
-                  int(gacc), int(bacc), _bn_acc(C, x2.device).data_ptr(), M, C, int(relu),
+                  int(gacc), int(bacc), _bn_acc(C, x2.device).data_ptr(), M, C,
                   _lib.stream_ptr())
         _lib.count_launch(3)
         for p, direct in ((g_ref, gdirect), (b_ref, bdirect)):
