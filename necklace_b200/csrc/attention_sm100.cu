@@ -844,22 +844,23 @@ static int make_tmap_dq(CUtensorMap* out, float* base, int BH, int S, int D) {
   return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
 }
 
-// 1: warp-specialised kernel (head dim 64), 0: serial kernel
+// 1: warp-specialised kernel, 0: serial kernel
 static int g_attn_bwd_impl = 1;
 
+template <int D>
 static int launch_bwd_pp(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdArgs& a,
                          cudaStream_t s) {
-  constexpr int smem = AttnBwd2Smem::BYTES;
+  constexpr int smem = AttnBwd2Smem<D>::BYTES;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_pp_kernel,
+    cudaError_t e = cudaFuncSetAttribute(attn_bwd_pp_kernel<D>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
   dim3 grid(a.B * a.H, (a.S + 127) / 128);
-  attn_bwd_pp_kernel<<<grid, BWD2_THREADS, smem, s>>>(tq, tk, tv, tdo, tdq, a);
+  attn_bwd_pp_kernel<D><<<grid, BWD2_THREADS, smem, s>>>(tq, tk, tv, tdo, tdq, a);
   return (int)cudaGetLastError();
 }
 
@@ -925,10 +926,11 @@ extern "C" int nkb_attn_bwd(const void* q, const void* k, const void* v, const v
   a.scale_log2 = scale * LOG2E;
   a.causal = causal;
   a.status = status;
-  if (D == 64 && g_attn_bwd_impl >= 1) {
+  if (g_attn_bwd_impl >= 1) {
     CUtensorMap tdq;
     if ((rc = make_tmap_dq(&tdq, dq_acc, B * H, S, D))) return rc;
-    rc = launch_bwd_pp(tq, tk, tv, tdo, tdq, a, s);
+    rc = D == 64 ? launch_bwd_pp<64>(tq, tk, tv, tdo, tdq, a, s)
+                 : launch_bwd_pp<128>(tq, tk, tv, tdo, tdq, a, s);
   } else {
     rc = D == 64 ? launch_bwd<64>(tq, tk, tv, tdo, a, s) : launch_bwd<128>(tq, tk, tv, tdo, a, s);
   }
