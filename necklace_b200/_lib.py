@@ -36,6 +36,8 @@ _SIGS = {
     "nkb_ce_fwd_bwd": [vp, vp, vp, i32, i32, i64, f32, vp],
     "nkb_ce_stats": [vp, vp, vp, i32, i32, i64, i32, vp],
     "nkb_ce_grad": [vp, vp, vp, i32, i32, i64, i32, f32, vp],
+    "nkb_loss_mean": [vp, vp, i32, vp, vp, vp],
+    "nkb_loss_corr": [vp, vp, i32, vp, vp],
     "nkb_embed_fwd": [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp],
     "nkb_embed_bwd": [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp],
     "nkb_adam_flat": [vp, vp, vp, vp, i32, vp, i64, f32, f32, f32, f32, f32, f32, f32, f32, vp,

@@ -50,6 +50,45 @@ __device__ __forceinline__ void block_online_reduce(float& m, float& s, float* s
   __syncthreads();
 }
 
+__global__ void __launch_bounds__(1024)
+loss_mean_kernel(const float* __restrict__ losses, const long long* __restrict__ targets, int T,
+                 float* __restrict__ loss, float* __restrict__ n_valid) {
+  __shared__ float sh_s[32];
+  __shared__ int sh_n[32];
+  float s = 0.f;
+  int n = 0;
+  for (int t = threadIdx.x; t < T; t += 1024) {
+    s += losses[t];
+    n += targets[t] >= 0;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    n += __shfl_xor_sync(0xffffffffu, n, o);
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) { sh_s[warp] = s; sh_n[warp] = n; }
+  __syncthreads();
+  if (warp) return;
+  s = sh_s[lane];
+  n = sh_n[lane];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    n += __shfl_xor_sync(0xffffffffu, n, o);
+  }
+  if (lane == 0) {
+    const float nv = (float)(n > 1 ? n : 1);
+    *loss = __fdiv_rn(s, nv);
+    *n_valid = nv;
+  }
+}
+
+__global__ void loss_corr_kernel(const float* __restrict__ dloss, const float* __restrict__ n_valid,
+                                 float T, float* __restrict__ out) {
+  *out = *dloss * __fdiv_rn(T, *n_valid);
+}
+
 // mode 0: fused fwd+bwd (losses out, grads in place)
 // mode 1: stats only  -> stats[t] = (max, sumexp, target logit if owned else 0)
 // mode 2: grad only from stats_g[t] = (global max, global sumexp)
@@ -262,6 +301,24 @@ extern "C" int nkb_ce_grad(void* logits, const long long* targets, const float* 
   return launch_ce<2>(logits, targets, nullptr, stats_g, T, V, ld, vocab_start, grad_scale,
                       static_cast<cudaStream_t>(stream));
 }
+// loss = sum of losses / n_valid, n_valid = max(1, number of targets >= 0).  One block: the
+// mean of a few thousand rows is bound by the launch (five launches of single operations took
+// its place before).
+extern "C" int nkb_loss_mean(const float* losses, const long long* targets, int T, float* loss,
+                             float* n_valid, void* stream) {
+  if (T <= 0) return -2;
+  loss_mean_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(losses, targets, T, loss,
+                                                                     n_valid);
+  return (int)cudaGetLastError();
+}
+
+// out = dloss * T / n_valid
+extern "C" int nkb_loss_corr(const float* dloss, const float* n_valid, int T, float* out,
+                             void* stream) {
+  loss_corr_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(dloss, n_valid, (float)T, out);
+  return (int)cudaGetLastError();
+}
+
 extern "C" int nkb_embed_fwd(const long long* idx, const void* wte, const void* wpe, void* out,
                              int T, int S, int C, int vocab_start, int vocab_rows, void* stream) {
   if (C % 8) return -3;

@@ -61,6 +61,10 @@ int nkb_ce_stats(const void* logits, const long long* targets, float* stats, int
 // grads from global (max, sumexp) per row: stats_g [T,2]
 int nkb_ce_grad(void* logits, const long long* targets, const float* stats_g, int T, int V,
                 long long ld, int vocab_start, float grad_scale, void* stream);
+// loss = sum(losses) / n_valid, n_valid = max(1, targets >= 0); out = dloss * T / n_valid
+int nkb_loss_mean(const float* losses, const long long* targets, int T, float* loss,
+                  float* n_valid, void* stream);
+int nkb_loss_corr(const float* dloss, const float* n_valid, int T, float* out, void* stream);
 int nkb_embed_fwd(const long long* idx, const void* wte, const void* wpe, void* out, int T, int S,
                   int C, int vocab_start, int vocab_rows, void* stream);
 int nkb_embed_bwd(const long long* idx, const void* dout, void* dwte, void* dwpe, int T, int S,

@@ -83,6 +83,31 @@ def ce_grad(logits: torch.Tensor, targets: torch.Tensor, stats_g: torch.Tensor, 
     return logits
 
 
+def _mean_loss(losses, targets):
+    """``(sum of losses / n, n)`` with ``n`` = the number of targets that count, at least 1."""
+    if not on_gpu(losses):
+        n_valid = (targets >= 0).sum().clamp(min=1).to(torch.float32)
+        return losses.sum() / n_valid, n_valid
+    loss = torch.empty((), dtype=torch.float32, device=losses.device)
+    n_valid = torch.empty(1, dtype=torch.float32, device=losses.device)
+    _lib.call("nkb_loss_mean", losses.data_ptr(), targets.data_ptr(), losses.shape[0],
+              loss.data_ptr(), n_valid.data_ptr(), _lib.stream_ptr())
+    _lib.count_launch()
+    return loss, n_valid
+
+
+def _loss_corr(dloss, n_valid, T):
+    """``dloss * T / n_valid`` as one device float."""
+    if not on_gpu(n_valid):
+        return (dloss.float() * (T / n_valid)).reshape(1)
+    dloss = dloss.float()
+    out = torch.empty(1, dtype=torch.float32, device=n_valid.device)
+    _lib.call("nkb_loss_corr", dloss.data_ptr(), n_valid.data_ptr(), T, out.data_ptr(),
+              _lib.stream_ptr())
+    _lib.count_launch()
+    return out
+
+
 class LMHeadLossFn(torch.autograd.Function):
     """``mean CE(x @ W^T, targets)`` with the logits kept only as a bf16 scratch that
     is turned into its own gradient in place (no fp32 logits, no softmax tensor)."""
@@ -94,15 +119,15 @@ class LMHeadLossFn(torch.autograd.Function):
         tg = targets.reshape(-1).contiguous()
         logits = gemm(x2, w, bias=bias)  # [T, Vpad]
         ctx.b_ref = bias
-        n_valid = (tg >= 0).sum().clamp(min=1).to(torch.float32)
         # gradient is scaled by 1/T here (all targets valid in the benchmark configs);
         # with ignored targets the final division by n_valid/T is applied in backward
         T = x2.shape[0]
         losses = cross_entropy_fwd_bwd(logits, tg, vocab, 1.0 / T)
+        loss, n_valid = _mean_loss(losses, tg)
         ctx.save_for_backward(x2, w, logits, n_valid)
         ctx.T = T
         ctx.xshape = x.shape
-        return losses.sum() / n_valid
+        return loss
 
     @staticmethod
     def backward(ctx, dloss):
@@ -110,7 +135,7 @@ class LMHeadLossFn(torch.autograd.Function):
         x2, w, dlogits, n_valid = ctx.saved_tensors
         # dlogits holds softmax-minus-onehot times 1/T; the exact factor
         # dloss * T / n_valid stays on the device and is applied inside the GEMMs.
-        corr = (dloss.float() * (ctx.T / n_valid)).reshape(1)
+        corr = _loss_corr(dloss, n_valid, ctx.T)
         dx = gemm(dlogits, w, b_mn=True, alpha_dev=corr).view(ctx.xshape)
         dw = _deliver_grad(w, lambda out, acc: gemm(dlogits, x2, a_mn=True, b_mn=True, out=out,
                                                     accumulate=acc, alpha_dev=corr))
