@@ -36,6 +36,11 @@ int nkb_norm_bwd_dx(const void* dy, const void* x, const void* w, const float* s
 // same, plus dres [rows, C] (bf16): the gradient that reaches x along a residual connection
 int nkb_norm_bwd_dx_res(const void* dy, const void* x, const void* w, const float* stats, void* dx,
                         int rows, int C, int rms, const void* dres, void* stream);
+// dx (+ dres, may be null) and the bf16 gradients of weight and bias (db may be null) in one pass.
+// acc: fp32 [2][C], ticket: one int, both zero on entry and on exit.
+int nkb_norm_bwd_all(const void* dy, const void* x, const void* w, const float* stats, void* dx,
+                     const void* dres, int rows, int C, int rms, float* acc, int* ticket, void* dw,
+                     void* db, int accum_w, int accum_b, void* stream);
 // Column sums over rows: acc[0][c] += sum_r dy[r,c]*xhat[r,c] (if x) ; acc[1][c] += sum_r dy[r,c].
 // `acc` is fp32 [2][C] scratch that must be zero on entry.
 int nkb_colsum(const void* dy, const void* x, const float* stats, float* acc, int rows, int C,

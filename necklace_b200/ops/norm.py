@@ -106,23 +106,31 @@ class NormFn(torch.autograd.Function):
             dw = _store_f32_grad(w, dw32)
             db = _store_f32_grad(b, db32) if b is not None else None
             return dx.view(dy.shape), dw, db, None, None
-        # GPU: dx kernel, then one column-sum kernel that writes both parameter gradients as
-        # bf16 straight into their destination (flat gradient buffer or a fresh tensor)
-        dx, _, _ = norm_bwd(dy2, x2, w, stats, ctx.rms, need_wgrad=False, need_bgrad=False,
-                            dres=dres)
-        dy2 = dy2.contiguous()
+        # GPU: one kernel reads dy and x once; both parameter gradients go as bf16 straight into
+        # their destination (flat gradient buffer or a fresh tensor)
+        dy2 = _rows16(dy2)
+        if dres is not None:
+            dres = _rows16(dres)
+        dx = torch.empty_like(x2)
         rows, Cn = x2.shape
         tgt_w, acc_w, ret_w = _grad_target(w)
         tgt_b, acc_b, ret_b = _grad_target(b) if b is not None else (None, False, None)
         acc, tickets = colsum_scratch(Cn, x2.device)
-        _lib.call("nkb_colsum_fused", dy2.data_ptr(), x2.data_ptr(), stats.data_ptr(),
+        _lib.call("nkb_norm_bwd_all", dy2.data_ptr(), x2.data_ptr(), w.data_ptr(),
+                  stats.data_ptr(), dx.data_ptr(), ptr(dres), rows, Cn, int(ctx.rms),
                   acc.data_ptr(), tickets.data_ptr(), tgt_w.data_ptr(), ptr(tgt_b), int(acc_w),
-                  int(acc_b), rows, Cn, Cn, int(ctx.rms), _lib.stream_ptr())
+                  int(acc_b), _lib.stream_ptr())
         _lib.count_launch()
         _grad_done(w)
         if b is not None:
             _grad_done(b)
         return dx.view(dy.shape), ret_w, ret_b, None, None
+
+
+def _rows16(t):
+    """``t`` as rows that 16-byte accesses can read."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def _grad_target(p):
