@@ -81,6 +81,7 @@ _SIGS = {
     "nkb_conv_wgrad": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp,
                        vp],
     "nkb_bn_fwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, f32, i32, vp],
+    "nkb_bn_eval": [vp, vp, vp, f32, vp, vp, vp, vp, i64, i32, i32, vp],
     "nkb_bn_apply": [vp, vp, vp, vp, vp, vp, i64, i32, i32, vp],
     "nkb_bn_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, vp, i64, i32, vp],
     "nkb_maxpool3x3s2_fwd": [vp, vp, vp, i32, i32, i32, i32, vp],

@@ -3,6 +3,7 @@
 //
 // A convolution is a GEMM on the tcgen05 kernel of gemm_sm100.cu:
 //   1x1 stride 1      activations [N*H*W, Cin] are the A operand as they are;
+//   C, Cout % 8 == 0  conv_sm100.cu reads the image itself;
 //   everything else   `im2col` gathers the receptive fields into col [N*Ho*Wo, KH*KW*Cin]
 //                     (K index = (kh*KW + kw)*Cin + c, zero for padding), the weight is stored
 //                     [Cout, KH*KW*Cin]; the data gradient is GEMM + `col2im` (written as a
@@ -67,47 +68,56 @@ im2col_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ c
   }
 }
 
-// Channel counts that are not a multiple of 8 (the 3-channel stem): one thread builds 8
-// consecutive K entries (each with its own tap / channel, scalar 2-byte loads that hit the
-// small, heavily reused input in cache) and writes them with one 16-byte store.
+// Channel counts that are not a multiple of 8 (the 3-channel stem).  A block gathers `tw`
+// neighbouring output pixels of one row: the KH input rows that they share come into shared
+// memory once (with the padding as zeros), a table says where each of a pixel's Kpad entries
+// lies there, and a thread puts eight of them together for one 16-byte store.  (Gathering
+// from global memory, 2 bytes and two divisions per entry, took 1375 us for the 224 x 224 stem
+// of 256 images; now 484 us, the 976 MB that it writes take 150 us.)
+constexpr int IM2COL_TILE_SMEM = 40 * 1024;
 __global__ void __launch_bounds__(256)
-im2col_gather8_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col,
-                      ConvGeom g) {
-  const long long M = (long long)g.N * g.Ho * g.Wo;
-  const int kchunks = g.Kpad / 8;
-  const int Kreal = g.KH * g.KW * g.C;
-  const long long total = M * kchunks;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += stride) {
-    const long long m = idx / kchunks;
-    const int k0 = (int)(idx % kchunks) * 8;
-    const int wo = (int)(m % g.Wo);
-    const long long t = m / g.Wo;
-    const int ho = (int)(t % g.Ho);
-    const int n = (int)(t / g.Ho);
-    const int h0 = ho * g.stride - g.pad, w0 = wo * g.stride - g.pad;
-    unsigned short v[8];
-    int tap = k0 / g.C, c = k0 % g.C;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      unsigned short e = 0;
-      if (k0 + j < Kreal) {
-        const int kh = tap / g.KW, kw = tap % g.KW;
-        const int h = h0 + kh, w = w0 + kw;
-        if (h >= 0 && h < g.H && w >= 0 && w < g.W) {
-          const long long src = (((long long)n * g.H + h) * g.W + w) * g.C + c;
-          if (NKB_IN_BOUNDS(src, (long long)g.N * g.H * g.W * g.C))
-            e = reinterpret_cast<const unsigned short*>(x)[src];
-        }
-      }
-      v[j] = e;
-      if (++c == g.C) { c = 0; ++tap; }
+im2col_tile_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col, ConvGeom g,
+                   int tw, int row_elems, int tiles_w) {
+  extern __shared__ __align__(16) uint16_t ic_smem[];
+  uint16_t* table = ic_smem;                       // [Kpad]: offset of entry k, pixel 0
+  uint16_t* rows = ic_smem + g.Kpad;               // [KH][row_elems], then 8 zeros
+  const int wo0 = (blockIdx.x % tiles_w) * tw;
+  const int ho = (blockIdx.x / tiles_w) % g.Ho;
+  const int n = blockIdx.x / tiles_w / g.Ho;
+  const int kc = g.KW * g.C, Kreal = g.KH * kc;
+  const int zero = g.KH * row_elems;
+  for (int k = threadIdx.x; k < g.Kpad; k += 256)
+    table[k] = (uint16_t)(k < Kreal ? (k / kc) * row_elems + k % kc : zero);
+  const int e0 = (wo0 * g.stride - g.pad) * g.C;   // element of the input row that lies at 0
+  const int WC = g.W * g.C;
+  for (int kh = 0; kh < g.KH; ++kh) {
+    const int h = ho * g.stride - g.pad + kh;
+    const bool in = h >= 0 && h < g.H;
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(x) +
+                          ((long long)n * g.H + (in ? h : 0)) * WC;
+    for (int e = threadIdx.x; e < row_elems; e += 256) {
+      const int w = e0 + e;
+      rows[kh * row_elems + e] = in && w >= 0 && w < WC ? src[w] : (uint16_t)0;
     }
-    if (!NKB_IN_BOUNDS(m * g.Kpad + k0 + 7, M * g.Kpad)) continue;
-    *reinterpret_cast<uint4*>(col + m * g.Kpad + k0) =
-        make_uint4(v[0] | ((uint32_t)v[1] << 16), v[2] | ((uint32_t)v[3] << 16),
-                   v[4] | ((uint32_t)v[5] << 16), v[6] | ((uint32_t)v[7] << 16));
+  }
+  if (threadIdx.x == 0) rows[zero] = 0;
+  __syncthreads();
+  const int px = min(tw, g.Wo - wo0), chunks = g.Kpad >> 3, sc = g.stride * g.C;
+  uint4* out = reinterpret_cast<uint4*>(col) +
+               (((long long)n * g.Ho + ho) * g.Wo + wo0) * chunks;
+  for (int i = threadIdx.x; i < px * chunks; i += 256) {
+    const int p = i / chunks, k = (i - p * chunks) * 8;
+    const uint4 t = *reinterpret_cast<const uint4*>(table + k);
+    const uint32_t tt[4] = {t.x, t.y, t.z, t.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int a = tt[j] & 0xffff, b = tt[j] >> 16;
+      const uint32_t lo = rows[a == zero ? zero : a + p * sc];
+      const uint32_t hi = rows[b == zero ? zero : b + p * sc];
+      o[j] = lo | hi << 16;
+    }
+    out[i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -290,8 +300,8 @@ __global__ void bn_finalize_kernel(float* __restrict__ acc, float* __restrict__ 
 // y = act((x - mean) * rstd * gamma + beta (+ res)).  Thread layout as in bn_sums_kernel: a
 // thread owns 8 fixed channels (its per-channel constants stay in registers) and walks rows.
 __global__ void __launch_bounds__(256)
-bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ stats,
-                const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
+bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ mean,
+                const float* __restrict__ spread, float eps, const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
                 const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ y,
                 uint8_t* __restrict__ mask, long long M, int C, int cx, int relu) {
   const int ry = 256 / cx;
@@ -306,10 +316,12 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ s
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       float2 fg = unpack_bf16x2(ug[j]), fb = unpack_bf16x2(ub[j]);
-      sc[2 * j] = stats[C + c + 2 * j] * fg.x;
-      sc[2 * j + 1] = stats[C + c + 2 * j + 1] * fg.y;
-      sh[2 * j] = fb.x - stats[c + 2 * j] * sc[2 * j];
-      sh[2 * j + 1] = fb.y - stats[c + 2 * j + 1] * sc[2 * j + 1];
+      // spread: rstd, or the variance when eps >= 0
+      const float r0 = spread[c + 2 * j], r1 = spread[c + 2 * j + 1];
+      sc[2 * j] = (eps < 0.f ? r0 : __frsqrt_rn(r0 + eps)) * fg.x;
+      sc[2 * j + 1] = (eps < 0.f ? r1 : __frsqrt_rn(r1 + eps)) * fg.y;
+      sh[2 * j] = fb.x - mean[c + 2 * j] * sc[2 * j];
+      sh[2 * j + 1] = fb.y - mean[c + 2 * j + 1] * sc[2 * j + 1];
     }
   }
   const long long step = (long long)gridDim.y * ry;
@@ -482,52 +494,67 @@ maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
   }
 }
 
+// A thread makes the 2 x 2 input positions (2i.., 2j..) of 8 channels from the four windows that
+// touch them: each window is loaded for 4 positions instead of being looked for by each of the
+// up to 9 it covers (411 MB of dx for 256 images took 407 us, now 220 us; the traffic takes
+// 86 us).
 __global__ void __launch_bounds__(256)
 maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const uint8_t* __restrict__ idx,
                    __nv_bfloat16* __restrict__ dx, int N, int H, int W, int C, int Ho, int Wo) {
-  const int cch = C / 8;
-  const long long total = (long long)N * H * W * cch;
+  const int cch = C / 8, Hb = (H + 1) / 2, Wb = (W + 1) / 2;
+  const long long total = (long long)N * Hb * Wb * cch;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const int c = (int)(i % cch) * 8;
-    long long t = i / cch;
-    const int w = (int)(t % W);
-    t /= W;
-    const int h = (int)(t % H);
-    const int n = (int)(t / H);
-    float acc[8];
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += stride) {
+    const int c = (int)(q % cch) * 8;
+    long long t = q / cch;
+    const int j = (int)(t % Wb);
+    t /= Wb;
+    const int i = (int)(t % Hb);
+    const int n = (int)(t / Hb);
+    uint4 v[4];
+    uint2 iv[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    for (int kh = 0; kh < 3; ++kh) {
-      const int hn = h + 1 - kh;
-      if (hn < 0 || (hn & 1)) continue;
-      const int ho = hn >> 1;
-      if (ho >= Ho) continue;
-      for (int kw = 0; kw < 3; ++kw) {
-        const int wn = w + 1 - kw;
-        if (wn < 0 || (wn & 1)) continue;
-        const int wo = wn >> 1;
-        if (wo >= Wo) continue;
+    for (int k = 0; k < 4; ++k) {  // window (i + k / 2, j + k % 2)
+      const int ho = i + (k >> 1), wo = j + (k & 1);
+      v[k] = make_uint4(0, 0, 0, 0);
+      iv[k] = make_uint2(~0u, ~0u);  // no tap
+      if (ho < Ho && wo < Wo) {
         const long long src = (((long long)n * Ho + ho) * Wo + wo) * C + c;
         if (!NKB_IN_BOUNDS(src + 7, (long long)N * Ho * Wo * C)) continue;
-        uint2 iv = *reinterpret_cast<const uint2*>(idx + src);
-        uint4 v = *reinterpret_cast<const uint4*>(dy + src);
-        uint32_t u[4] = {v.x, v.y, v.z, v.w};
-        const int tap = kh * 3 + kw;
+        v[k] = *reinterpret_cast<const uint4*>(dy + src);
+        iv[k] = *reinterpret_cast<const uint2*>(idx + src);
+      }
+    }
+    float acc[4][8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float2 f = unpack_bf16x2(u[j]);
-          const uint32_t word = (2 * j < 4) ? iv.x : iv.y;
-          const int a0 = (word >> (8 * ((2 * j) & 3))) & 0xff;
-          const int a1 = (word >> (8 * ((2 * j + 1) & 3))) & 0xff;
-          if (a0 == tap) acc[2 * j] += f.x;
-          if (a1 == tap) acc[2 * j + 1] += f.y;
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[p][e] = 0.f;
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {  // (taps in ascending order for every position)
+      const uint32_t u[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float2 f = unpack_bf16x2(u[e >> 1]);
+        const float val = (e & 1) ? f.y : f.x;
+        const uint32_t tap = ((e < 4 ? iv[k].x : iv[k].y) >> (8 * (e & 3))) & 0xff;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          // row 0 is tap 1 of window row i; row 1 is tap 2 of it and tap 0 of row i + 1
+          const int dh = k >> 1, dw = k & 1, r = p >> 1, s = p & 1;
+          if (r + 1 - 2 * dh < 0 || s + 1 - 2 * dw < 0) continue;
+          if (tap == (uint32_t)((r + 1 - 2 * dh) * 3 + s + 1 - 2 * dw)) acc[p][e] += val;
         }
       }
     }
-    *reinterpret_cast<uint4*>(dx + (((long long)n * H + h) * W + w) * C + c) =
-        make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]),
-                   pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const int h = 2 * i + (p >> 1), w = 2 * j + (p & 1);
+      if (h < H && w < W)
+        *reinterpret_cast<uint4*>(dx + (((long long)n * H + h) * W + w) * C + c) =
+            make_uint4(pack_bf16x2(acc[p][0], acc[p][1]), pack_bf16x2(acc[p][2], acc[p][3]),
+                       pack_bf16x2(acc[p][4], acc[p][5]), pack_bf16x2(acc[p][6], acc[p][7]));
+    }
   }
 }
 
@@ -596,6 +623,19 @@ static ConvGeom geom(int N, int H, int W, int C, int KH, int KW, int stride, int
   return g;
 }
 
+// Output pixels per block of im2col_tile_kernel: at most 64, as many as shared memory (and the
+// table's 16-bit offsets) hold; 0 where one pixel's window does not fit or the grid would be
+// larger than a launch takes.
+static int im2col_tile(const ConvGeom& g) {
+  for (int tw = g.Wo < 64 ? g.Wo : 64; tw >= 1; tw >>= 1) {
+    const long long elems = (long long)g.KH * (((tw - 1) * g.stride + g.KW) * (long long)g.C);
+    if (2 * (g.Kpad + elems + 8) > IM2COL_TILE_SMEM || elems > 65000) continue;
+    const long long blocks = (long long)((g.Wo + tw - 1) / tw) * g.Ho * g.N;
+    return blocks < (1LL << 31) ? tw : 0;
+  }
+  return 0;
+}
+
 extern "C" int nkb_im2col_nhwc(const void* x, void* col, int N, int H, int W, int C, int KH,
                                int KW, int stride, int pad, int Kpad, void* stream) {
   if (Kpad < KH * KW * C || (Kpad & 7)) return -3;
@@ -608,9 +648,13 @@ extern "C" int nkb_im2col_nhwc(const void* x, void* col, int N, int H, int W, in
   if (vec)
     im2col_kernel<8><<<conv_grid(M * (Kpad / 8), 256), 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g);
-  else if (!(reinterpret_cast<uintptr_t>(col) & 15))
-    im2col_gather8_kernel<<<conv_grid(M * (Kpad / 8), 256), 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g);
+  else if (int tw = im2col_tile(g); tw > 0 && !(reinterpret_cast<uintptr_t>(col) & 15)) {
+    const int row_elems = ((tw - 1) * stride + KW) * C, tiles_w = (g.Wo + tw - 1) / tw;
+    im2col_tile_kernel<<<(unsigned)(tiles_w * (long long)g.Ho * N), 256,
+                         2 * (Kpad + KH * row_elems + 8), s>>>(
+        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g, tw, row_elems,
+        tiles_w);
+  }
   else
     im2col_kernel<1><<<conv_grid(M * Kpad, 256), 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g);
@@ -669,8 +713,8 @@ extern "C" int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, co
   bn_finalize_kernel<<<(C + 127) / 128, 128, 0, s>>>(acc, stats, run_mean, run_var, M, C, eps,
                                                      momentum);
   bn_apply_kernel<<<grid, 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
-      static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
+      static_cast<const __nv_bfloat16*>(x), stats, stats + C, -1.f,
+      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
       static_cast<__nv_bfloat16*>(y), static_cast<uint8_t*>(mask), M, C, cx, relu);
   return (int)cudaGetLastError();
 }
@@ -683,9 +727,26 @@ extern "C" int nkb_bn_apply(const void* x, const float* stats, const void* gamma
   dim3 grid;
   bn_sums_dims(M, C, cx, grid);
   bn_apply_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), stats, static_cast<const __nv_bfloat16*>(gamma),
-      static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
+      static_cast<const __nv_bfloat16*>(x), stats, stats + C, -1.f,
+      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
       static_cast<__nv_bfloat16*>(y), nullptr, M, C, cx, relu);
+  return (int)cudaGetLastError();
+}
+
+// The same from running statistics: rstd is taken in the kernel (three single-operation kernels
+// per layer made (mean, rstd) of them before).
+extern "C" int nkb_bn_eval(const void* x, const float* run_mean, const float* run_var, float eps,
+                           const void* gamma, const void* beta, const void* res, void* y,
+                           long long M, int C, int relu, void* stream) {
+  if (C % 8 || eps < 0.f) return -3;
+  int cx;
+  dim3 grid;
+  bn_sums_dims(M, C, cx, grid);
+  bn_apply_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(x), run_mean, run_var, eps,
+      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
+      static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(y), nullptr, M, C, cx,
+      relu);
   return (int)cudaGetLastError();
 }
 
@@ -731,7 +792,7 @@ extern "C" int nkb_maxpool3x3s2_bwd(const void* dy, const void* idx, void* dx, i
                                     int C, void* stream) {
   if (C % 8) return -3;
   const int Ho = (H + 2 - 3) / 2 + 1, Wo = (W + 2 - 3) / 2 + 1;
-  maxpool_bwd_kernel<<<conv_grid((long long)N * H * W * (C / 8), 256), 256, 0,
+  maxpool_bwd_kernel<<<conv_grid((long long)N * ((H + 1) / 2) * ((W + 1) / 2) * (C / 8), 256), 256, 0,
                        static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const uint8_t*>(idx),
       static_cast<__nv_bfloat16*>(dx), N, H, W, C, Ho, Wo);

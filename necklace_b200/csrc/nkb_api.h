@@ -102,6 +102,10 @@ int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, const void* r
                float eps, float momentum, int relu, void* stream);
 int nkb_bn_apply(const void* x, const float* stats, const void* gamma, const void* beta,
                  const void* res, void* y, long long M, int C, int relu, void* stream);
+// Evaluation with running statistics (fp32 [C] each) instead of (mean, rstd).
+int nkb_bn_eval(const void* x, const float* run_mean, const float* run_var, float eps,
+                const void* gamma, const void* beta, const void* res, void* y, long long M, int C,
+                int relu, void* stream);
 int nkb_bn_bwd(const void* dy, const void* x, const void* mask, const float* stats,
                const void* gamma, void* dx, void* dres, void* dgamma, void* dbeta, int acc_g,
                int acc_b, float* acc, long long M, int C, void* stream);

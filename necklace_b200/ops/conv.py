@@ -355,19 +355,27 @@ class BatchNorm2d(nn.Module):
         if self.training:
             return BatchNormFn.apply(x, self.weight, self.bias, residual, self.running_mean,
                                      self.running_var, self.eps, self.momentum, self.relu)
-        stats = torch.stack([self.running_mean, torch.rsqrt(self.running_var + self.eps)])
         C = self.C
         x2 = x.reshape(-1, C)
         if not on_gpu(x):
+            stats = torch.stack([self.running_mean, torch.rsqrt(self.running_var + self.eps)])
             y = (x2.float() - stats[0]) * stats[1] * self.weight.float() + self.bias.float()
             if residual is not None:
                 y = y + residual.reshape(-1, C).float()
             return (torch.relu(y) if self.relu else y).to(x.dtype).view(x.shape)
         y = torch.empty_like(x2)
         r2 = residual.reshape(-1, C) if residual is not None else None
-        _lib.call("nkb_bn_apply", x2.data_ptr(), stats.contiguous().data_ptr(),
-                  self.weight.data_ptr(), self.bias.data_ptr(), ptr(r2), y.data_ptr(),
-                  x2.shape[0], C, int(self.relu), _lib.stream_ptr())
+        mean, var = self.running_mean, self.running_var
+        if mean.dtype == var.dtype == torch.float32 and mean.is_contiguous() \
+                and var.is_contiguous() and self.eps >= 0:
+            _lib.call("nkb_bn_eval", x2.data_ptr(), mean.data_ptr(), var.data_ptr(),
+                      float(self.eps), self.weight.data_ptr(), self.bias.data_ptr(), ptr(r2),
+                      y.data_ptr(), x2.shape[0], C, int(self.relu), _lib.stream_ptr())
+        else:
+            stats = torch.stack([mean.float(), torch.rsqrt(var.float() + self.eps)])
+            _lib.call("nkb_bn_apply", x2.data_ptr(), stats.data_ptr(), self.weight.data_ptr(),
+                      self.bias.data_ptr(), ptr(r2), y.data_ptr(), x2.shape[0], C,
+                      int(self.relu), _lib.stream_ptr())
         _lib.count_launch()
         return y.view(x.shape)
 

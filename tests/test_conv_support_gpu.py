@@ -1,0 +1,52 @@
+"""The gather of layers with odd channel counts, the max pooling gradient and evaluation-mode batch
+norm against their CPU forms."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("case", [(2, 9, 11, 3, 7, 7, 2, 3), (1, 5, 200, 3, 3, 3, 1, 1),
+                                  (3, 8, 8, 5, 2, 3, 1, 0), (2, 6, 7, 12, 3, 3, 2, 1),
+                                  (1, 4, 130, 1, 1, 1, 1, 0), (1, 3, 3, 1001, 3, 3, 1, 1),
+                                  (1, 2, 2, 4099, 3, 3, 1, 1)])
+def test_gather_of_odd_channel_counts(case):
+    from necklace_b200.ops.conv import im2col
+    N, H, W, C, KH, KW, s, p = case
+    x = torch.randn(N, H, W, C, generator=torch.Generator().manual_seed(C)).bfloat16()
+    assert torch.equal(im2col(x, KH, KW, s, p), im2col(x.cuda(), KH, KW, s, p).cpu())
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 8), (2, 3, 4, 16), (3, 7, 5, 64), (1, 16, 17, 8)])
+def test_max_pool_gradient(shape):
+    from necklace_b200.ops.conv import max_pool_3x3_s2
+    n = int(torch.tensor(shape).prod())          # distinct values: one winner per window
+    x = (torch.randperm(n, generator=torch.Generator().manual_seed(3)) % 251 - 125).view(shape)
+    x = x.bfloat16()
+    a, b = x.clone().requires_grad_(True), x.cuda().requires_grad_(True)
+    ya, yb = max_pool_3x3_s2(a), max_pool_3x3_s2(b)
+    g = torch.randn(ya.shape, generator=torch.Generator().manual_seed(4)).bfloat16()
+    ya.backward(g)
+    yb.backward(g.cuda())
+    assert torch.equal(ya, yb.cpu())
+    # up to four windows are added in fp32 and rounded once on both sides
+    assert torch.allclose(a.grad.float(), b.grad.cpu().float(), rtol=2.0 ** -8, atol=1e-6)
+
+
+@pytest.mark.parametrize("C,relu,res", [(8, False, False), (72, True, True), (2048, True, False)])
+@pytest.mark.parametrize("half_stats", [False, True])
+def test_evaluation_batch_norm(C, relu, res, half_stats):
+    from necklace_b200.ops.conv import BatchNorm2d
+    g = torch.Generator().manual_seed(C)
+    x = torch.randn(3, 5, 7, C, generator=g).bfloat16()
+    r = torch.randn(3, 5, 7, C, generator=g).bfloat16() if res else None
+    bn = BatchNorm2d(C, relu=relu).eval()
+    bn.running_mean.copy_(torch.randn(C, generator=g) * 0.1)
+    bn.running_var.copy_(torch.rand(C, generator=g) + 0.5)
+    if half_stats:                        # a model converted as a whole
+        bn.running_mean, bn.running_var = bn.running_mean.bfloat16(), bn.running_var.bfloat16()
+    m, v = bn.running_mean.double(), bn.running_var.double()
+    want = (x.double() - m) * torch.rsqrt(v + bn.eps) + (r.double() if res else 0.0)
+    want = torch.relu(want) if relu else want
+    got = bn.cuda()(x.cuda(), r.cuda() if res else None).cpu().double()
+    assert bool(((got - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -19).all())
