@@ -13,6 +13,9 @@
 //   data gradient  dx[q, ci]     = sum over tap, co  dy[(q + pad - tap) / s, co]  w[co, tap, ci]
 //                  for a stride s > 1 one launch per class of positions q mod s, whose taps are those that
 //                  divide; the output is a strided view of dx
+//                  Each tap's product is rounded to bf16 before the taps are added in fp32, as when
+//                  it went through memory: every tap is an accumulator of its own, which the
+//                  epilogue adds up in registers
 //   weight grad.   dw[co, tap, ci] = sum over p  dy[p, co]  x[p * s + tap - pad, ci]
 //                  pixels are the contraction: boxes of at most 64 of them, both operands
 //                  MN-major, the range of boxes split over all SMs, fp32 partial sums
@@ -20,8 +23,9 @@
 // What bounds it: with 64 output channels the MMA (N = 64 costs as much as N = 128) and the nine
 // reads of the image from L2, with more channels the tensor cores.  ResNet-50, 256 images of
 // 224 x 224, the 19 layers that were gathered, in us: forward 2832 (gather) + about 1700 (GEMM)
-// before, 1355 now; data gradient 2777 (scatter) + about 2500, now 1456; weight gradient about
-// 5000, now 1458.  The training step went from 38.4 to 30.2 ms.
+// before, 1355 now; data gradient 2777 (scatter) + about 2500, now 1888 (1456 with one accumulator
+// for all taps, which rounds once); weight gradient about 5000, now 1458.  The training step
+// went from 38.4 to 30.2 ms.
 //
 // Warp roles and pipeline are those of the GEMM (gemm_sm100.cu): one TMA producer thread, one
 // MMA thread, eight epilogue warps, two accumulators in TMEM, one CTA per SM, tiles dealt
@@ -43,6 +47,9 @@ constexpr int CV_THREADS = 384;  // warps 0, 1: TMA and MMA; 2, 3 idle; 4..11 ep
 constexpr int CV_A_BYTES = 128 * CV_BK * 2;
 constexpr int CV_STG_BYTES = 2 * 16384;  // one 128 x 64 bf16 tile per epilogue group
 constexpr int CV_MAX_TAPS = 64;
+// setmaxnreg hand-over (data gradient); the CTA owns 384 threads x 168 registers
+constexpr int CV_CTRL_REGS = 72, CV_EPI_REGS = 216;
+static_assert(128 * CV_CTRL_REGS + 256 * CV_EPI_REGS <= CV_THREADS * 168, "register budget");
 enum { CV_FWD = 0, CV_DGRAD = 1, CV_WGRAD = 2 };
 
 struct ConvArgs {
@@ -129,7 +136,8 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
       // with 64 columns each group of four warps drains every other tile by itself
-      mbar_init(&acc_empty[a], BN == 64 ? 4 : 8);
+      // (data gradient: both groups work on every tap)
+      mbar_init(&acc_empty[a], BN == 64 && KIND != CV_DGRAD ? 4 : 8);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -150,6 +158,9 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   const int kchunks = (g.kc + CV_BK - 1) / CV_BK;
   const int ksteps = KIND == CV_WGRAD ? g.rows / 16 : CV_BK / 16;
 
+  // the data gradient's sums take up to 128 registers per epilogue thread
+  if constexpr (KIND == CV_DGRAD)
+    if (warp < 4) reg_alloc_dec<CV_CTRL_REGS>();
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0;
@@ -236,39 +247,44 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
       for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-        int nk = g.ntaps * kchunks;
+        // steps per accumulator, and accumulators: one per tap for the data gradient
+        int nk = KIND == CV_DGRAD ? kchunks : g.ntaps * kchunks;
+        const int na = KIND == CV_DGRAD ? g.ntaps : 1;
         if constexpr (KIND == CV_WGRAD) {
           const int ks = u / tiles;
           nk = (int)((long long)(ks + 1) * boxes / g.split) -
                (int)((long long)ks * boxes / g.split);
         }
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag)) {
-          cv_fail(g.status, abort_flag, NKB_ERR_ACC_FREE);
-          break;
-        }
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int i = 0; i < nk; ++i) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
-            cv_fail(g.status, abort_flag, NKB_ERR_TMA_WAIT);
+        for (int a = 0; a < na && ok; ++a) {
+          if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag)) {
+            cv_fail(g.status, abort_flag, NKB_ERR_ACC_FREE);
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint64_t dA = dA0 + (uint32_t)stage * (Cfg::STAGE >> 4);
-          const uint64_t dB = dB0 + (uint32_t)stage * (Cfg::STAGE >> 4);
+          const uint32_t d_tmem = tmem_base + acc * BN;
+          for (int i = 0; i < nk; ++i) {
+            if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
+              cv_fail(g.status, abort_flag, NKB_ERR_TMA_WAIT);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t dA = dA0 + (uint32_t)stage * (Cfg::STAGE >> 4);
+            const uint64_t dB = dB0 + (uint32_t)stage * (Cfg::STAGE >> 4);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (KIND != CV_WGRAD || k < ksteps)
-              umma_bf16_ss(d_tmem, dA + (A_MN ? k * (16 * 128 >> 4) : k * 2),
-                           dB + (B_MN ? k * (16 * 128 >> 4) : k * 2), idesc,
-                           (i > 0 || k > 0) ? 1u : 0u);
-          umma_commit(&empty_bar[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+            for (int k = 0; k < 4; ++k)
+              if (KIND != CV_WGRAD || k < ksteps)
+                umma_bf16_ss(d_tmem, dA + (A_MN ? k * (16 * 128 >> 4) : k * 2),
+                             dB + (B_MN ? k * (16 * 128 >> 4) : k * 2), idesc,
+                             (i > 0 || k > 0) ? 1u : 0u);
+            umma_commit(&empty_bar[stage]);
+            if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          }
+          if (!ok) break;
+          umma_commit(&acc_full[acc]);
+          if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
-        if (!ok) break;
-        umma_commit(&acc_full[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
   } else if (warp >= 4) {
@@ -278,6 +294,79 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     uint8_t* stg = gstg + lane_grp * 4096;
     int acc = 0;
     uint32_t acc_phase = 0;
+    if constexpr (KIND == CV_DGRAD) {
+      reg_alloc_inc<CV_EPI_REGS>();
+      // a group's columns: 32 of the 64, or every other chunk of 64
+      constexpr int NC = BN == 64 ? 32 : BN / 2;
+      int odd = 0;  // two units' tiles of 64 columns alternate between the staging buffers
+      for (int u = blockIdx.x; u < units; u += gridDim.x, odd ^= 1) {
+        float sum[NC];
+#pragma unroll
+        for (int i = 0; i < NC; ++i) sum[i] = 0.f;
+        bool ok = true;
+        for (int t = 0; t < g.ntaps; ++t) {
+          ok = ok && mbar_wait(&acc_full[acc], acc_phase, abort_flag);
+          if (ok) {
+            tc_fence_after();
+            const uint32_t t_addr = tmem_base + (uint32_t(lane_grp * 32) << 16) + acc * BN;
+#pragma unroll
+            for (int q = 0; q < NC / 32; ++q) {
+              const int c = BN == 64 ? group * 32 : ((q >> 1) * 2 + group) * 64 + (q & 1) * 32;
+              uint32_t v[32];
+              tmem_ld_32x32(t_addr + c, v);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const float2 f = unpack_bf16x2(
+                    pack_bf16x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+                sum[q * 32 + 2 * i] += f.x;
+                sum[q * 32 + 2 * i + 1] += f.y;
+              }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[acc]);
+          }
+          if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        }
+        int w0, h0, n0;
+        box_origin(g, u % g.tiles_m, w0, h0, n0);
+        const int c0 = (u / g.tiles_m) * BN;
+        const int bar = BN == 64 ? 3 : 1 + group, bar_n = BN == 64 ? 256 : 128;
+        const bool issuer = lane_grp == 0 && lane == 0 && (BN > 64 || group == 0);
+        uint8_t* tile = BN == 64 ? stg_base + odd * 16384 : gstg;
+        // the store that used the staging tile before has read it; all warps agree to go on
+        if (issuer) { if (BN == 64) tma_store_wait_read<1>(); else tma_store_wait_read<0>(); }
+        if (!named_bar_and(bar, bar_n, ok)) {
+          cv_fail(g.status, abort_flag, NKB_ERR_ACC_WAIT);
+          break;
+        }
+#pragma unroll
+        for (int ch = 0; ch < (BN == 64 ? 1 : BN / 128); ++ch) {
+          const int col = c0 + (BN == 64 ? 0 : (ch * 2 + group) * 64);
+          if (col >= g.cols) break;  // the same for all warps of the group
+          if (ch) {
+            if (issuer) tma_store_wait_read<0>();
+            named_bar_sync(bar, bar_n);
+          }
+          constexpr int Q = BN == 64 ? 4 : 8;
+#pragma unroll
+          for (int k = 0; k < Q; ++k) {
+            const float* f = sum + ch * 64 + k * 8;
+            const int q = BN == 64 ? group * 4 + k : k;
+            *reinterpret_cast<uint4*>(tile + lane_grp * 4096 + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]),
+                           pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+          }
+          fence_proxy_async_smem();
+          named_bar_sync(bar, bar_n);
+          if (issuer) {
+            tma_store_4d(&tmO, tile, col, w0, h0, n0);
+            tma_store_commit();
+          }
+        }
+      }
+    } else
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
       const bool mine = BN > 64 || acc == group;
       if (mine) {
