@@ -195,6 +195,10 @@ dp_quant_allreduce_kernel(CommCtx c, QuantArgs q) {
   const int e = begin_call(c);
   const long long nwords = (q.n + 15) >> 4;
   uint32_t* my_codes = reinterpret_cast<uint32_t*>(static_cast<char*>(c.heap[c.rank]) + q.codes_off);
+  // 16-byte accesses where the buffers allow them (element by element the kernel took 352 us on
+  // one rank for 25.6 M bf16 gradients, now 96 us; their 370 MB take 57 us)
+  const bool vec = ((reinterpret_cast<uintptr_t>(q.g) | reinterpret_cast<uintptr_t>(q.residual) |
+                     reinterpret_cast<uintptr_t>(q.out)) & 15) == 0;
 
   // phase 0: quantise my sub-slice of every shard (word granularity)
   for (int s = 0; s < c.world; ++s) {
@@ -206,6 +210,45 @@ dp_quant_allreduce_kernel(CommCtx c, QuantArgs q) {
     for (long long w = lo + threadIdx.x; w < hi; w += COMM_THREADS) {
       const long long base = w << 4;
       uint32_t word = 0;
+      if (vec && base + 16 <= q.n) {
+        float a[16];
+        if (q.g_fp32) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            *reinterpret_cast<float4*>(a + 4 * k) =
+                reinterpret_cast<const float4*>(static_cast<const float*>(q.g) + base)[k];
+        } else {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const uint4 t =
+                reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(q.g) + base)[k];
+            const uint32_t u[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = unpack_bf16x2(u[j]);
+              a[8 * k + 2 * j] = f.x;
+              a[8 * k + 2 * j + 1] = f.y;
+            }
+          }
+        }
+        float4* rp = reinterpret_cast<float4*>(q.residual + base);
+        float4 r[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r[k] = rp[k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float rr[4] = {r[k].x, r[k].y, r[k].z, r[k].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float res;
+            word |= q2_code(a[4 * k + j] + rr[j], q.thr, res) << (2 * (4 * k + j));
+            rr[j] = res;
+          }
+          rp[k] = make_float4(rr[0], rr[1], rr[2], rr[3]);
+        }
+        my_codes[w] = word;
+        continue;
+      }
 #pragma unroll 4
       for (int i = 0; i < 16; ++i) {
         const long long idx = base + i;
@@ -273,6 +316,27 @@ dp_quant_allreduce_kernel(CommCtx c, QuantArgs q) {
         uint4 pk = ld_volatile_v4(counts + w * 16);
         uint32_t pw[4] = {pk.x, pk.y, pk.z, pk.w};
         const long long base = w << 4;
+        if (vec && base + 16 <= q.n) {
+          float v[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            v[i] = (int)(signed char)((pw[i >> 2] >> (8 * (i & 3))) & 0xff) * mul;
+          if (q.out_fp32) {
+            float4* o = reinterpret_cast<float4*>(static_cast<float*>(q.out) + base);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              o[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+          } else {
+            uint4* o = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(q.out) + base);
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+              o[k] = make_uint4(pack_bf16x2(v[8 * k], v[8 * k + 1]),
+                                pack_bf16x2(v[8 * k + 2], v[8 * k + 3]),
+                                pack_bf16x2(v[8 * k + 4], v[8 * k + 5]),
+                                pack_bf16x2(v[8 * k + 6], v[8 * k + 7]));
+          }
+          continue;
+        }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const long long idx = base + i;
