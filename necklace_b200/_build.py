@@ -12,12 +12,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(os.path.dirname(HERE), "build", "nkb200")
 LIB = os.path.join(HERE, "_nkb200.so")
+# the same entry points as a Python extension (csrc/pycall.cpp), linked to LIB
+EXT = os.path.join(HERE, "_nkpy.so")
 # the bounds-checked debug variant (-DNKB_DEBUG_BOUNDS): ``--debug-bounds``
 BUILD_DBG = os.path.join(os.path.dirname(HERE), "build", "nkb200_dbg")
 LIB_DBG = os.path.join(HERE, "_nkb200_dbg.so")
@@ -79,7 +82,28 @@ def build(force: bool = False, verbose: bool = False, debug_bounds: bool = False
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError(f"link failed:\n{p.stdout}{p.stderr}")
+    if not debug_bounds:
+        _build_ext(force)
     return lib
+
+
+def _build_ext(force: bool) -> None:
+    src = os.path.join(CSRC, "pycall.cpp")
+    newest = max(os.path.getmtime(src), _headers_mtime())
+    if not force and os.path.exists(EXT) and os.path.getmtime(EXT) >= newest:
+        return
+    inc = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(inc, "Python.h")):
+        return                  # without the headers every call goes through ctypes
+    # built under another name and moved: a process may be importing it
+    tmp = EXT + f".{os.getpid()}"
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-I", inc, "-I",
+           CSRC, src, "-o", tmp, "-L", HERE, "-l:" + os.path.basename(LIB),
+           "-Wl,-rpath,$ORIGIN"]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        raise RuntimeError(f"building {EXT} failed:\n{p.stdout}{p.stderr}")
+    os.replace(tmp, EXT)
 
 
 def resource_report() -> str:

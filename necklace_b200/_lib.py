@@ -13,6 +13,8 @@ import ctypes as C
 import os
 import threading
 
+from torch import _C
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # NKB_DEBUG_BOUNDS=1 selects the bounds-checked debug build (see ``debug_bounds``)
 DEBUG_BOUNDS = os.environ.get("NKB_DEBUG_BOUNDS", "0") not in ("", "0")
@@ -123,6 +125,20 @@ def debug_bounds(raise_on_error: bool = True) -> dict:
     return bad
 
 
+# compiled entry points by name (csrc/pycall.cpp); what is not in it goes through ctypes
+_fast: dict = {}
+
+
+def _load_fast() -> dict:
+    if DEBUG_BOUNDS:
+        return {}           # the extension is linked to the normal library
+    try:
+        from . import _nkpy
+    except ImportError:
+        return {}
+    return {n: getattr(_nkpy, n) for n in dir(_nkpy) if n.startswith("nkb_")}
+
+
 def load(build_if_missing: bool = True):
     """Load (building first if needed and possible) and return the ctypes handle."""
     global _lib, _load_error
@@ -143,6 +159,7 @@ def load(build_if_missing: bool = True):
                 fn.restype = i32
             if hasattr(lib, "nkb_build_info"):
                 lib.nkb_build_info.restype = C.c_char_p
+            _fast.update(_load_fast())
             _lib = lib
         except Exception as e:  # noqa: BLE001
             _load_error = e
@@ -174,16 +191,26 @@ def check(rc: int, what: str) -> None:
 
 def call(name: str, *args) -> None:
     """Call a native entry point, raising on a non-zero return."""
-    lib = load()
-    fn = getattr(lib, name, None)
+    fn = _fast.get(name)
     if fn is None:
-        raise NativeLibraryError(f"native symbol {name} missing from {LIB_PATH}; rebuild")
-    check(fn(*args), name)
+        lib = load()
+        fn = _fast.get(name) or getattr(lib, name, None)
+        if fn is None:
+            raise NativeLibraryError(f"native symbol {name} missing from {LIB_PATH}; rebuild")
+    rc = fn(*args)
+    if rc:
+        check(rc, name)
+
+
+def value(name: str, *args) -> int:
+    """What a native function that answers a question returns."""
+    lib = load()
+    return (_fast.get(name) or getattr(lib, name))(*args)
 
 
 def stream_ptr() -> int:
-    import torch
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of the current device's current stream."""
+    return _C._cuda_getCurrentRawStream(_C._cuda_getDevice())
 
 
 # Count of native kernel launches issued through `call` wrappers that opt in

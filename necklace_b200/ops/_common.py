@@ -2,10 +2,12 @@
 from __future__ import annotations
 
 import torch
+import torch.autograd.forward_ad as _fwd_ad
 
 from .. import _lib
 
 _status: dict[int, torch.Tensor] = {}
+_status_at: dict[int, int] = {}      # their addresses: the tensors live as long as the process
 _scratch: dict[tuple, torch.Tensor] = {}
 
 STATUS_TEXT = {
@@ -30,6 +32,22 @@ def status_word(device=None) -> torch.Tensor:
         t = torch.zeros(1, dtype=torch.int32, device=f"cuda:{dev}")
         _status[dev] = t
     return t
+
+
+def status_ptr(t: torch.Tensor) -> int:
+    """Address of the status word of ``t``'s device."""
+    dev = t.get_device()
+    p = _status_at.get(dev)
+    if p is None:
+        p = _status_at[dev] = status_word(t.device).data_ptr()
+    return p
+
+
+def plain_call() -> bool:
+    """Whether an operator may run its forward pass without an autograd node: gradients are off,
+    and neither forward-mode differentiation nor a trace is looking."""
+    return not torch.is_grad_enabled() and _fwd_ad._current_level < 0 \
+        and torch._C._get_tracing_state() is None
 
 
 def check_status(reset: bool = True) -> None:

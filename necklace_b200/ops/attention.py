@@ -14,7 +14,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import _lib
-from ._common import on_gpu, status_word
+from ._common import on_gpu, plain_call, status_ptr
 
 
 def set_exp_mode(mode: int) -> None:
@@ -64,9 +64,12 @@ def _split(qkv, H):
 
 def attn_fwd(qkv: torch.Tensor, H: int, causal: bool = True):
     """Returns (out [B,S,C], lse [B,H,S] fp32)."""
-    q, k, v, B, S, C, D = _split(qkv, H)
+    B, S, C3 = qkv.shape
+    C = C3 // 3
+    D = C // H
     scale = 1.0 / math.sqrt(D)
     if not on_gpu(qkv):
+        q, k, v, B, S, C, D = _split(qkv, H)
         qf, kf, vf = q.float(), k.float(), v.float()
         s = (qf @ kf.transpose(-1, -2)) * scale
         if causal:
@@ -75,20 +78,25 @@ def attn_fwd(qkv: torch.Tensor, H: int, causal: bool = True):
         o = torch.softmax(s, -1) @ vf
         return o.permute(0, 2, 1, 3).reshape(B, S, C).to(qkv.dtype), lse
     assert qkv.dtype == torch.bfloat16 and qkv.is_contiguous() and D in (64, 128)
+    assert C3 == 3 * H * D
+    q = qkv.data_ptr()                   # q, k, v: columns [0, C), [C, 2C), [2C, 3C)
     out = torch.empty(B, S, C, dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
-    _lib.call("nkb_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-              lse.data_ptr(), B, H, S, D, S * 3 * C, D, 3 * C, S * C, D, C, float(scale),
-              int(causal), status_word(qkv.device).data_ptr(), _lib.stream_ptr())
+    _lib.call("nkb_attn_fwd", q, q + 2 * C, q + 4 * C, out.data_ptr(), lse.data_ptr(), B, H, S, D,
+              S * 3 * C, D, 3 * C, S * C, D, C, scale, int(causal), status_ptr(qkv),
+              _lib.stream_ptr())
     _lib.count_launch()
     return out, lse
 
 
 def attn_bwd(qkv, out, lse, dout, H: int, causal: bool = True):
     """Returns dqkv [B,S,3C]."""
-    q, k, v, B, S, C, D = _split(qkv, H)
+    B, S, C3 = qkv.shape
+    C = C3 // 3
+    D = C // H
     scale = 1.0 / math.sqrt(D)
     if not on_gpu(qkv):
+        q, k, v, B, S, C, D = _split(qkv, H)
         qf, kf, vf = q.float(), k.float(), v.float()
         do = dout.view(B, S, H, D).permute(0, 2, 1, 3).float()
         s = (qf @ kf.transpose(-1, -2)) * scale
@@ -107,13 +115,13 @@ def attn_bwd(qkv, out, lse, dout, H: int, causal: bool = True):
         return dqkv
     dout = dout.contiguous()
     dqkv = torch.empty_like(qkv)
-    dq, dk, dv, *_ = _split(dqkv, H)
     delta = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
     dq_acc = torch.empty(B, H, S, D, dtype=torch.float32, device=qkv.device)  # cleared by the delta kernel
-    _lib.call("nkb_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-              dout.data_ptr(), lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-              delta.data_ptr(), dq_acc.data_ptr(), B, H, S, D, S * 3 * C, D, 3 * C, S * C, D, C,
-              float(scale), int(causal), status_word(qkv.device).data_ptr(), _lib.stream_ptr())
+    q, dq = qkv.data_ptr(), dqkv.data_ptr()
+    _lib.call("nkb_attn_bwd", q, q + 2 * C, q + 4 * C, out.data_ptr(), dout.data_ptr(),
+              lse.data_ptr(), dq, dq + 2 * C, dq + 4 * C, delta.data_ptr(), dq_acc.data_ptr(), B,
+              H, S, D, S * 3 * C, D, 3 * C, S * C, D, C, scale, int(causal), status_ptr(qkv),
+              _lib.stream_ptr())
     _lib.count_launch(3)
     return dqkv
 
@@ -133,4 +141,6 @@ class AttentionQKVFn(torch.autograd.Function):
 
 
 def attention_qkv(qkv: torch.Tensor, n_head: int, causal: bool = True) -> torch.Tensor:
+    if plain_call():
+        return attn_fwd(qkv, n_head, causal)[0]
     return AttentionQKVFn.apply(qkv, n_head, causal)

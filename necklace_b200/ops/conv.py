@@ -19,7 +19,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ._common import on_gpu, ptr, scratch_zero, status_word
+from ._common import on_gpu, plain_call, ptr, scratch_zero, status_ptr
 from .gemm import _deliver_grad, gemm
 
 
@@ -86,7 +86,7 @@ def _conv_fwd(x, w, KH, KW, stride, pad):
     y = torch.empty(N, *_out_hw(H, W, KH, KW, stride, pad), w.shape[0], dtype=x.dtype,
                     device=x.device)
     _lib.call("nkb_conv_fwd", x.data_ptr(), w.data_ptr(), y.data_ptr(), N, H, W, C, w.shape[0],
-              KH, KW, stride, pad, status_word(x.device).data_ptr(), _lib.stream_ptr())
+              KH, KW, stride, pad, status_ptr(x), _lib.stream_ptr())
     _lib.count_launch()
     return y
 
@@ -95,7 +95,7 @@ def _conv_dgrad(dy, w, shape, KH, KW, stride, pad):
     N, H, W, C = shape
     dx = torch.empty(shape, dtype=dy.dtype, device=dy.device)
     _lib.call("nkb_conv_dgrad", dy.data_ptr(), w.data_ptr(), dx.data_ptr(), N, H, W, C,
-              w.shape[0], KH, KW, stride, pad, status_word(dy.device).data_ptr(),
+              w.shape[0], KH, KW, stride, pad, status_ptr(dy),
               _lib.stream_ptr())
     _lib.count_launch(min(stride, KH) * min(stride, KW))
     return dx
@@ -104,13 +104,13 @@ def _conv_dgrad(dy, w, shape, KH, KW, stride, pad):
 def _conv_wgrad(x, dy, w, KH, KW, stride, pad, out, acc):
     N, H, W, C = x.shape
     geom = (N, H, W, C, w.shape[0], KH, KW, stride, pad)
-    split = _lib.load().nkb_conv_wgrad_split(*geom)
+    split = _lib.value("nkb_conv_wgrad_split", *geom)
     ws = torch.empty(max(split, 1), w.numel(), dtype=torch.float32, device=x.device)
     direct = out is not None and out.dtype == torch.bfloat16 and out.is_contiguous() \
         and out.data_ptr() % 16 == 0
     dst = out if direct else torch.empty_like(w)
     _lib.call("nkb_conv_wgrad", x.data_ptr(), dy.data_ptr(), dst.data_ptr(), ws.data_ptr(), split,
-              *geom, int(acc and direct), status_word(x.device).data_ptr(), _lib.stream_ptr())
+              *geom, int(acc and direct), status_ptr(x), _lib.stream_ptr())
     _lib.count_launch(2)
     if out is None or direct:
         return dst
@@ -202,7 +202,19 @@ class Conv1x1SplitFn(torch.autograd.Function):
 
 
 def conv2d(x, w, KH, KW, stride=1, pad=0):
+    if plain_call():
+        return _conv2d_plain(x, w, KH, KW, stride, pad)
     return Conv2dFn.apply(x, w, KH, KW, stride, pad)
+
+
+def _conv2d_plain(x, w, KH, KW, stride, pad):
+    """The forward pass by itself."""
+    N, H, W, C = x.shape
+    direct = KH == 1 and KW == 1 and stride == 1 and pad == 0 and C % 8 == 0
+    if not direct and _image_kernels(x, w, KH, KW, stride, pad):
+        return _conv_fwd(x, w, KH, KW, stride, pad)
+    a = x.reshape(-1, C) if direct else im2col(x, KH, KW, stride, pad)
+    return gemm(a, w).view(N, *_out_hw(H, W, KH, KW, stride, pad), w.shape[0])
 
 
 class Conv2d(nn.Module):
@@ -229,7 +241,8 @@ class Conv2d(nn.Module):
         """``(x, conv(x))`` at the head of a residual block (see ``Conv1x1SplitFn``)."""
         hooked = self._forward_hooks or self._forward_pre_hooks or self._backward_hooks \
             or self._backward_pre_hooks         # they see calls of the module
-        if (self.k, self.stride, self.pad) == (1, 1, 0) and x.shape[-1] % 8 == 0 and not hooked:
+        if (self.k, self.stride, self.pad) == (1, 1, 0) and x.shape[-1] % 8 == 0 \
+                and not hooked and not plain_call():
             return Conv1x1SplitFn.apply(x, self.weight)
         return x, self(x)
 

@@ -16,7 +16,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ._common import scratch_zero, on_gpu, ptr, status_word, scratch
+from ._common import on_gpu, plain_call, ptr, scratch, scratch_zero, status_ptr
 
 EPI_NONE, EPI_GELU_FWD, EPI_GELU_BWD, EPI_RELU = 0, 1, 2, 3
 
@@ -37,14 +37,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          alpha_dev: torch.Tensor | None = None) -> torch.Tensor:
     """``a`` is stored ``[M,K]`` (or ``[K,M]`` when ``a_mn``); ``b`` is stored ``[N,K]``
     (or ``[K,N]`` when ``b_mn``).  Both must be 2-D with unit inner stride."""
-    assert a.dim() == 2 and b.dim() == 2
-    M, K = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
-    N, Kb = (b.shape[1], b.shape[0]) if b_mn else (b.shape[0], b.shape[1])
+    sa, sb = a.shape, b.shape
+    assert len(sa) == 2 and len(sb) == 2
+    M, K = (sa[1], sa[0]) if a_mn else sa
+    N, Kb = (sb[1], sb[0]) if b_mn else sb
     assert K == Kb, f"contraction mismatch {K} vs {Kb}"
     if out is None:
-        out = torch.empty(M, N, dtype=out_dtype or a.dtype, device=a.device)
         assert not accumulate
-    assert out.shape == (M, N) and out.stride(1) == 1
+        out = torch.empty((M, N), dtype=out_dtype or a.dtype, device=a.device)
+    else:
+        assert out.shape == (M, N) and out.stride(1) == 1
 
     if not on_gpu(a, b, out):
         A = a.float().t() if a_mn else a.float()
@@ -69,28 +71,34 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         return out
 
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-    assert a.stride(1) == 1 and b.stride(1) == 1
-    assert out.dtype in (torch.bfloat16, torch.float32)
+    (lda, ia), (ldb, ib) = a.stride(), b.stride()
+    assert ia == 1 and ib == 1
+    fp32 = out.dtype == torch.float32
+    assert fp32 or out.dtype == torch.bfloat16
     if bias is not None:
         assert bias.dtype == torch.bfloat16 and bias.is_contiguous() and bias.numel() == N
     if res is not None:
         assert res.dtype == torch.bfloat16 and res.shape == (M, N) and res.stride(1) == 1
-    if epi in (EPI_GELU_FWD, EPI_GELU_BWD):
+    if epi == EPI_GELU_FWD or epi == EPI_GELU_BWD:
         assert aux is not None and aux.dtype == torch.bfloat16 and aux.shape == (M, N)
         assert aux.stride(1) == 1
+    pa, pb = a.data_ptr(), b.data_ptr()
     # TMA: 16-byte aligned base and row pitch; repack the rare operand that is not
-    if a.stride(0) % 8 or a.data_ptr() % 16:
+    if lda % 8 or pa % 16:
         a = _repack(a)
-    if b.stride(0) % 8 or b.data_ptr() % 16:
+        pa, lda = a.data_ptr(), a.stride(0)
+    if ldb % 8 or pb % 16:
         b = _repack(b)
-    _ensure_workspace(a.device)
-    _lib.call("nkb_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0),
-              int(b_mn), out.data_ptr(), out.stride(0), int(out.dtype == torch.float32),
-              int(accumulate), M, N, K, float(alpha), ptr(bias), ptr(res),
-              res.stride(0) if res is not None else 0, int(epi), ptr(aux),
-              aux.stride(0) if aux is not None else 0, status_word(a.device).data_ptr(),
-              ptr(ready_flags), int(rows_per_flag), int(ready_target), int(max_ctas), int(bn),
-              ptr(alpha_dev), _lib.stream_ptr())
+        pb, ldb = b.data_ptr(), b.stride(0)
+    if a.get_device() not in _WORKSPACE:
+        _ensure_workspace(a.device)
+    _lib.call("nkb_gemm_bf16", pa, lda, a_mn, pb, ldb, b_mn, out.data_ptr(), out.stride(0), fp32,
+              accumulate, M, N, K, alpha, None if bias is None else bias.data_ptr(),
+              None if res is None else res.data_ptr(), 0 if res is None else res.stride(0), epi,
+              None if aux is None else aux.data_ptr(), 0 if aux is None else aux.stride(0),
+              status_ptr(a), None if ready_flags is None else ready_flags.data_ptr(),
+              rows_per_flag, ready_target, max_ctas, bn,
+              None if alpha_dev is None else alpha_dev.data_ptr(), _lib.stream_ptr())
     _lib.count_launch()
     return out
 
@@ -267,10 +275,23 @@ class MLPFn(torch.autograd.Function):
 
 
 def linear(x, w, b=None, residual=None):
+    if plain_call():
+        r2 = residual.reshape(-1, w.shape[0]) if residual is not None else None
+        y = gemm(x.reshape(-1, x.shape[-1]), w, bias=b, res=r2)
+        return y.view(*x.shape[:-1], w.shape[0])
     return LinearFn.apply(x, w, b, residual)
 
 
 def mlp(x, w1, b1, w2, b2, residual=None, act="gelu"):
+    if plain_call():
+        x2 = x.reshape(-1, x.shape[-1])
+        r2 = residual.reshape(-1, w2.shape[0]) if residual is not None else None
+        if act == "gelu":
+            z = torch.empty(x2.shape[0], w1.shape[0], dtype=x2.dtype, device=x2.device)
+            h = gemm(x2, w1, bias=b1, epi=EPI_GELU_FWD, aux=z)
+        else:
+            h = gemm(x2, w1, bias=b1, epi=EPI_RELU)
+        return gemm(h, w2, bias=b2, res=r2).view(*x.shape[:-1], w2.shape[0])
     return MLPFn.apply(x, w1, b1, w2, b2, residual, act)
 
 

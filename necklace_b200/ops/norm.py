@@ -5,7 +5,7 @@ import torch
 import torch.nn as nn
 
 from .. import _lib
-from ._common import on_gpu, ptr, scratch
+from ._common import on_gpu, plain_call, ptr
 from .gemm import _deliver_grad, colsum_scratch
 
 
@@ -133,6 +133,13 @@ def _rows16(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+def _norm_plain(x, w, b, eps, rms):
+    x2 = x.reshape(-1, x.shape[-1])
+    if not x2.is_contiguous():
+        x2 = x2.contiguous()
+    return norm_fwd(x2, w, b, eps, rms)[0].view(x.shape)
+
+
 def _grad_target(p):
     """(tensor the kernel writes, accumulate?, what autograd gets) for parameter ``p``."""
     buf = getattr(p, "_nkb_grad", None)
@@ -177,10 +184,14 @@ class LayerNorm(nn.Module):
         self.bias = nn.Parameter(torch.zeros(dim, dtype=dtype, device=device)) if bias else None
 
     def forward(self, x):
+        if plain_call():
+            return _norm_plain(x, self.weight, self.bias, self.eps, False)
         return NormFn.apply(x, self.weight, self.bias, self.eps, False)
 
     def split(self, x):
         """``(x, norm(x))`` for a pre-norm residual block (see ``NormSplitFn``)."""
+        if plain_call():
+            return x, _norm_plain(x, self.weight, self.bias, self.eps, False)
         return NormSplitFn.apply(x, self.weight, self.bias, self.eps, False)
 
 
@@ -191,8 +202,12 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim, dtype=dtype, device=device))
 
     def forward(self, x):
+        if plain_call():
+            return _norm_plain(x, self.weight, None, self.eps, True)
         return NormFn.apply(x, self.weight, None, self.eps, True)
 
     def split(self, x):
         """``(x, norm(x))`` for a pre-norm residual block (see ``NormSplitFn``)."""
+        if plain_call():
+            return x, _norm_plain(x, self.weight, None, self.eps, True)
         return NormSplitFn.apply(x, self.weight, None, self.eps, True)

@@ -4,7 +4,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ._common import on_gpu
+from ._common import on_gpu, plain_call
 
 
 def _rope_ref(qkv, H, base, sign, pos_offset=0):
@@ -93,6 +93,10 @@ def rope(qkv, n_head, base=10000.0, pos_offset=0):
 
 def linear_rope(x, w, n_head, base=10000.0, pos_offset=0):
     """Packed QKV projection (``w`` = ``[q; k; v]`` rows, no bias) with rotary q / k."""
+    if plain_call():
+        from .gemm import gemm
+        qkv = gemm(x.reshape(-1, x.shape[-1]), w).view(*x.shape[:-1], w.shape[0])
+        return _apply(qkv, n_head, base, False, pos_offset)
     return LinearRopeFn.apply(x, w, n_head, base, pos_offset)
 
 
