@@ -1582,53 +1582,64 @@ static int gemm_run(GemmArgs g, const void* A, long long lda, int a_mn, const vo
                     long long ldb, int b_mn, int max_ctas, int bn_hint, void* stream) {
   const int M = g.M, N = g.N, K = g.K;
   // Tile choice.  bn_hint: 0 = automatic, 128 / 256 = single-CTA tile of that width,
-  // 512 = CTA-pair 256 x 256 tile.
+  // 512 = CTA-pair 256 x 256 tile; and split-K when the output has too few tiles to occupy the
+  // machine and K is long.
+  //
+  // Time in us: launch, prologue and last epilogue; the K steps of 64 of every round (0.27 for all
+  // three kinds: the tensor pipe bounds the 256-wide tiles, the operand traffic of 64 B/clk
+  // per SM the 128 x 128 one); the part of a further round's epilogue that its main loop does not
+  // hide.  With more than about 110 SMs at work the 48 KB that a 128 x 256 tile loads per step meet
+  // the rate of L2, more so when both operands are MN-major (4096 x 1024 x 8192 weight gradient:
+  // 56.2 us against 51.3 with pairs, which load a third less).  A split adds the reduction's launch
+  // and its fp32 partial sums, written and read at about 8 TB/s as most of them stay in L2.
+  // Fitted to graphs of equal GEMMs, M = 333 .. 4096, N = 768 .. 5504, K = 768 .. 8192:
+  // 2313 x 768 x 768 takes 8.6 / 9.9 / 11.4 us, 4096 x 4096 x 1024 42 / 30.6 / 29.6 us (128 x 128,
+  // 128 x 256, pair).  Weighing rounds alone (0.68 : 0.88 : 1) took 26.8 us for 2313 x 1024 x 4096
+  // (pair; 25.2 with 128 x 256) and 30.7 us for 1024 x 1024 x 8192 (128 x 128 in 2 slices; 24.3 with
+  // pairs in 4).  With at most 8 slices a 64 x 64 weight gradient over 802816 pixels ran on
+  // 8 SMs: the 49 split GEMMs of a ResNet-50 step took 9.0 ms (its 1x1 layers 2.0 ms now).
   int BN = 256;
   bool pair = false;
-  if (bn_hint == 128 || bn_hint == 256) {
-    BN = bn_hint;
-  } else if (bn_hint == 512) {
-    pair = true;
-  } else {
-    // cost = rounds of the persistent loop x work per round / measured relative
-    // throughput of the tile kind (pair 1.0, single-CTA 128x256 0.88, 128x128 0.68)
-    int sms = num_sms();
-    long long mblk = (M + BM - 1) / BM;
-    long long t256 = mblk * ((N + 255) / 256);
-    long long t128 = mblk * ((N + 127) / 128);
-    double c256 = (double)((t256 + sms - 1) / sms) * 2.0 / 0.88;
-    double c128 = (double)((t128 + sms - 1) / sms) * 1.0 / 0.68;
-    double best = c256;
-    if (N <= 128 || c128 < c256) { BN = 128; best = c128; }
-    long long tp = ((M + 255) / 256) * (long long)((N + 255) / 256);
-    int npair = sms / 2;
-    double cp = (double)((tp + npair - 1) / npair) * 2.0;
-    if (g_pair_enabled && M > 128 && N > 128 && cp <= best) pair = true;
-    if (g.ag_ctas && (g.ag_rows_per_rank % 256)) pair = false;
-  }
-  // split-K when the output has too few tiles to occupy the machine and K is long
   g.split_k = 1;
   g.splitk_ws = nullptr;
-  if (g_splitk_enabled && g_splitk_ws && !g.ag_ctas && !g.rs_on && g.epi == NKB_EPI_NONE &&
-      !g.bias && !g.res && (N % 4) == 0 && (g.ldc % 4) == 0 && K >= 2048) {
-    long long slots = pair ? num_sms() / 2 : num_sms();
-    long long tl = pair ? ((M + 255) / 256) * (long long)((N + 255) / 256)
-                        : ((M + BM - 1) / BM) * (long long)((N + BN - 1) / BN);
-    // With at most 8 slices a 64 x 64 weight gradient over 802816 pixels ran on 8 SMs: the 49
-    // split GEMMs of a ResNet-50 step took 9.0 ms (its 1x1 layers 2.0 ms now).
-    // A slice of K costs about 0.27 us per 64 (a pair's 256 x 256 x 64 step); every slice is
-    // written and read once more as fp32, about 8 TB/s as most of it stays in L2.
-    int S = 1;
+  {
+    const int sms = num_sms();
+    const long long mblk = (M + BM - 1) / BM;
+    const int kb = (K + BK - 1) / BK;
+    const bool can_split = g_splitk_enabled && g_splitk_ws && !g.ag_ctas && !g.rs_on &&
+                           g.epi == NKB_EPI_NONE && !g.bias && !g.res && (N % 4) == 0 &&
+                           (g.ldc % 4) == 0 && K >= 2048;
     double best = 1e30;
-    for (int c = 1; c <= 64 && c <= slots / tl; ++c) {
-      if (c > 1 && ((K / BK) / c < 8 || (long long)c * M * N > g_splitk_ws_floats)) break;
-      const double cost = 0.27 * (K / BK) / c + (c > 1 ? (double)c * M * N * 1e-6 : 0.0);
-      if (cost < best) { best = cost; S = c; }
-    }
-    if (S > 1 && tl * 10 <= slots * 7) {
-      g.split_k = S;
-      g.splitk_ws = g_splitk_ws;
-    }
+    const double mn = a_mn && b_mn ? 1.2 : 1.0;
+    auto consider = [&](int kind_bn, bool kind_pair, long long tiles, int slots, double fixed,
+                        double extra) {
+      const int most = can_split && tiles * 10 <= slots * 7 ? 64 : 1;
+      for (int S = 1; S <= most && (S == 1 || S <= slots / tiles); ++S) {
+        if (S > 1 && ((K / BK) / S < 8 || (long long)S * M * N > g_splitk_ws_floats)) break;
+        const long long r = (tiles * S + slots - 1) / slots;
+        double step = 0.27;
+        if (kind_bn == 256 && !kind_pair) {
+          const double busy = (double)(tiles * S) / r;
+          step *= mn * (busy > 110.0 ? busy / 110.0 : 1.0);
+        }
+        const double c = fixed + r * (step * ((kb + S - 1) / S)) + (r - 1) * extra +
+                         (S > 1 ? 2.5 + (double)S * M * N * 1e-6 : 0.0);
+        if (c < best) {
+          best = c;
+          BN = kind_bn;
+          pair = kind_pair;
+          g.split_k = S;
+        }
+      }
+    };
+    const bool any = bn_hint != 128 && bn_hint != 256 && bn_hint != 512;
+    if (bn_hint == 128 || any) consider(128, false, mblk * ((N + 127) / 128), sms, 4.6, 1.0);
+    if (bn_hint == 256 || (any && N > 128))
+      consider(256, false, mblk * ((N + 255) / 256), sms, 6.1, 1.8);
+    if (bn_hint == 512 || (any && g_pair_enabled && M > 128 && N > 128 &&
+                           !(g.ag_ctas && (g.ag_rows_per_rank % 256))))
+      consider(256, true, ((M + 255) / 256) * (long long)((N + 255) / 256), sms / 2, 7.8, 1.2);
+    if (g.split_k > 1) g.splitk_ws = g_splitk_ws;
   }
   CUtensorMap tmA, tmB;
   int rc;

@@ -25,3 +25,17 @@ def test_long_contractions_in_many_slices(M, N, K):
     _close(out, want, mag, K)
     acc = gemm(a, b, a_mn=True, b_mn=True, out=out.clone(), accumulate=True)
     assert bool(((acc.double() - 2 * want).abs() <= want.abs() * 2.0 ** -6 + mag * K * 2.0 ** -23).all())
+
+
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn", [
+    (333, 776, 768, 0, 0), (333, 1024, 4104, 0, 1),          # 128 x 128, whole and split
+    (771, 3080, 768, 0, 1), (2313, 1032, 2752, 0, 0),        # 128 x 256
+    (4097, 3072, 1032, 0, 0), (1032, 1024, 8200, 1, 1),      # pairs, whole and split
+    (129, 129, 64, 0, 0), (128, 264, 2048, 0, 0)])
+def test_every_kind_of_tile_that_the_sizes_choose(M, N, K, a_mn, b_mn):
+    from necklace_b200.ops.gemm import gemm
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn(*((K, M) if a_mn else (M, K)), generator=g, device="cuda").bfloat16()
+    b = torch.randn(*((K, N) if b_mn else (N, K)), generator=g, device="cuda").bfloat16()
+    A, B = (a.t() if a_mn else a).double(), (b.t() if b_mn else b).double()
+    _close(gemm(a, b, a_mn=bool(a_mn), b_mn=bool(b_mn)), A @ B.t(), A.abs() @ B.abs().t(), K)
