@@ -194,7 +194,8 @@ class Conv1x1SplitFn(torch.autograd.Function):
             dy2 = dy2.contiguous()
         dx = None
         if ctx.needs_input_grad[0]:
-            r2 = dres.reshape(a.shape) if dres is not None else None
+            # (the gradient of a sum arrives as an expanded scalar)
+            r2 = dres.reshape(a.shape).contiguous() if dres is not None else None
             dx = gemm(dy2, w, b_mn=True, res=r2).view(x.shape)
         dw = _deliver_grad(w, lambda out, acc: gemm(dy2, a, a_mn=True, b_mn=True, out=out,
                                                     accumulate=acc))

@@ -27,6 +27,11 @@ def test_residual_head_adds_the_other_gradient(shape):
     w = conv.weight.detach().double()
     want = dy.double() @ w + dr.double()
     _close(x.grad, want, dy.double().abs() @ w.abs() + dr.double().abs(), 40)
+    x.grad = None
+    alias, y = conv.split(x)
+    (alias.sum() + y.sum()).backward()            # expanded gradients
+    want = w.sum(0).expand(shape) + 1.0
+    _close(x.grad, want, w.abs().sum(0).expand(shape) + 1.0, 40)
     calls = []
     conv.register_forward_hook(lambda *a: calls.append(1))
     alias, y = conv.split(x)                      # a hooked module is called
