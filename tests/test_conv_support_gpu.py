@@ -50,3 +50,23 @@ def test_evaluation_batch_norm(C, relu, res, half_stats):
     want = torch.relu(want) if relu else want
     got = bn.cuda()(x.cuda(), r.cuda() if res else None).cpu().double()
     assert bool(((got - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -19).all())
+
+
+@pytest.mark.parametrize("eps", [1e-5, 0.0, 1e-3])
+def test_evaluation_batch_norm_bits(eps):
+    """Variance and eps in the kernel give the bits of (mean, torch.rsqrt(variance + eps)): the
+    same layer with statistics of another kind of memory takes that way."""
+    from necklace_b200.ops.conv import BatchNorm2d
+    g = torch.Generator(device="cuda").manual_seed(1)
+    C = 4096
+    bn = BatchNorm2d(C, eps=eps, device="cuda").eval()
+    with torch.no_grad():
+        bn.weight.copy_(torch.randn(C, generator=g, device="cuda"))
+        bn.bias.copy_(torch.randn(C, generator=g, device="cuda"))
+    bn.running_mean.normal_(generator=g)
+    bn.running_var.copy_(torch.rand(C, generator=g, device="cuda").add(1e-4) * 4)
+    x = torch.randn(64, 1, 1, C, generator=g, device="cuda").bfloat16()
+    one = bn(x)
+    bn.running_mean = torch.stack([bn.running_mean, bn.running_mean], 1)[:, 0]   # strided
+    assert not bn.running_mean.is_contiguous()
+    assert torch.equal(one, bn(x))
