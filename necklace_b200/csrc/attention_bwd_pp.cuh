@@ -404,6 +404,12 @@ attn_bwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int e = 0; e < 64; ++e)
           if (r > w * 64 + e) p[e] = 0.f;
       }
+      // Keys behind the last one: their scores are 0, so a query whose scores are all far below
+      // 0 would give them P = exp2(-lse) = inf, and inf * 0 in dQ = dS K
+      if (j * 128 + r >= a.S) {
+#pragma unroll
+        for (int e = 0; e < 64; ++e) p[e] = 0.f;
+      }
       if (!mbar_wait(s_read, it & 1, abort_flag)) {
         att_error(a.status, abort_flag, NKB_ERR_ACC_WAIT);
         ok = false;
