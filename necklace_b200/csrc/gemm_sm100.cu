@@ -1458,8 +1458,8 @@ int make_tmap_bf16_nd(CUtensorMap* out, const void* base, int rank, const long l
 static int g_num_sms = 0;
 static int g_pair_enabled = 1;
 static int g_splitk_enabled = 1;
-static float* g_splitk_ws = nullptr;      // caller-provided workspace (see nkb_gemm_set_workspace)
-static long long g_splitk_ws_floats = 0;  // CTA-pair tiles in the automatic choice
+// fp32 values of all slices of a split GEMM, at most (128 MB)
+constexpr long long SPLITK_MAX_FLOATS = 32LL << 20;
 int num_sms() {
   if (!g_num_sms) {
     int dev = 0;
@@ -1544,13 +1544,6 @@ using namespace nkb;
 
 extern "C" void nkb_gemm_set_pair(int enabled) { nkb::g_pair_enabled = enabled; }
 extern "C" void nkb_gemm_set_splitk(int enabled) { nkb::g_splitk_enabled = enabled; }
-// Caller-owned fp32 workspace for split-K partial tiles (the library never allocates);
-// without one, split-K is not used.
-extern "C" void nkb_gemm_set_workspace(float* ws, long long n_floats) {
-  nkb::g_splitk_ws = ws;
-  nkb::g_splitk_ws_floats = n_floats;
-}
-
 static int gemm_run_splitk(GemmArgs g, const CUtensorMap& tmA, const CUtensorMap& tmB, int a_mn,
                            int b_mn, bool pair, int BN, int max_ctas, cudaStream_t s) {
   int rc;
@@ -1578,69 +1571,94 @@ static int gemm_run_splitk(GemmArgs g, const CUtensorMap& tmA, const CUtensorMap
   return (int)cudaGetLastError();
 }
 
-static int gemm_run(GemmArgs g, const void* A, long long lda, int a_mn, const void* B,
-                    long long ldb, int b_mn, int max_ctas, int bn_hint, void* stream) {
-  const int M = g.M, N = g.N, K = g.K;
-  // Tile choice.  bn_hint: 0 = automatic, 128 / 256 = single-CTA tile of that width,
-  // 512 = CTA-pair 256 x 256 tile; and split-K when the output has too few tiles to occupy the
-  // machine and K is long.
-  //
-  // Time in us: launch, prologue and last epilogue; the K steps of 64 of every round (0.27 for all
-  // three kinds: the tensor pipe bounds the 256-wide tiles, the operand traffic of 64 B/clk
-  // per SM the 128 x 128 one); the part of a further round's epilogue that its main loop does not
-  // hide.  With more than about 110 SMs at work the 48 KB that a 128 x 256 tile loads per step meet
-  // the rate of L2, more so when both operands are MN-major (4096 x 1024 x 8192 weight gradient:
-  // 56.2 us against 51.3 with pairs, which load a third less).  A split adds the reduction's launch
-  // and its fp32 partial sums, written and read at about 8 TB/s as most of them stay in L2.
-  // Fitted to graphs of equal GEMMs, M = 333 .. 4096, N = 768 .. 5504, K = 768 .. 8192:
-  // 2313 x 768 x 768 takes 8.6 / 9.9 / 11.4 us, 4096 x 4096 x 1024 42 / 30.6 / 29.6 us (128 x 128,
-  // 128 x 256, pair).  Weighing rounds alone (0.68 : 0.88 : 1) took 26.8 us for 2313 x 1024 x 4096
-  // (pair; 25.2 with 128 x 256) and 30.7 us for 1024 x 1024 x 8192 (128 x 128 in 2 slices; 24.3 with
-  // pairs in 4).  With at most 8 slices a 64 x 64 weight gradient over 802816 pixels ran on
-  // 8 SMs: the 49 split GEMMs of a ResNet-50 step took 9.0 ms (its 1x1 layers 2.0 ms now).
+struct TilePlan {
   int BN = 256;
   bool pair = false;
-  g.split_k = 1;
-  g.splitk_ws = nullptr;
-  {
-    const int sms = num_sms();
-    const long long mblk = (M + BM - 1) / BM;
-    const int kb = (K + BK - 1) / BK;
-    const bool can_split = g_splitk_enabled && g_splitk_ws && !g.ag_ctas && !g.rs_on &&
-                           g.epi == NKB_EPI_NONE && !g.bias && !g.res && (N % 4) == 0 &&
-                           (g.ldc % 4) == 0 && K >= 2048;
-    double best = 1e30;
-    const double mn = a_mn && b_mn ? 1.2 : 1.0;
-    auto consider = [&](int kind_bn, bool kind_pair, long long tiles, int slots, double fixed,
-                        double extra) {
-      const int most = can_split && tiles * 10 <= slots * 7 ? 64 : 1;
-      for (int S = 1; S <= most && (S == 1 || S <= slots / tiles); ++S) {
-        if (S > 1 && ((K / BK) / S < 8 || (long long)S * M * N > g_splitk_ws_floats)) break;
-        const long long r = (tiles * S + slots - 1) / slots;
-        double step = 0.27;
-        if (kind_bn == 256 && !kind_pair) {
-          const double busy = (double)(tiles * S) / r;
-          step *= mn * (busy > 110.0 ? busy / 110.0 : 1.0);
-        }
-        const double c = fixed + r * (step * ((kb + S - 1) / S)) + (r - 1) * extra +
-                         (S > 1 ? 2.5 + (double)S * M * N * 1e-6 : 0.0);
-        if (c < best) {
-          best = c;
-          BN = kind_bn;
-          pair = kind_pair;
-          g.split_k = S;
-        }
+  int slices = 1;
+};
+
+// Tile choice.  bn_hint: 0 = automatic, 128 / 256 = single-CTA tile of that width,
+// 512 = CTA-pair 256 x 256 tile; and split-K when the output has too few tiles to occupy the
+// machine and K is long.
+//
+// Time in us: launch, prologue and last epilogue; the K steps of 64 of every round (0.27 for all
+// three kinds: the tensor pipe bounds the 256-wide tiles, the operand traffic of 64 B/clk
+// per SM the 128 x 128 one); the part of a further round's epilogue that its main loop does not
+// hide.  With more than about 110 SMs at work the 48 KB that a 128 x 256 tile loads per step meet
+// the rate of L2, more so when both operands are MN-major (4096 x 1024 x 8192 weight gradient:
+// 56.2 us against 51.3 with pairs, which load a third less).  A split adds the reduction's launch
+// and its fp32 partial sums, written and read at about 8 TB/s as most of them stay in L2.
+// Fitted to graphs of equal GEMMs, M = 333 .. 4096, N = 768 .. 5504, K = 768 .. 8192:
+// 2313 x 768 x 768 takes 8.6 / 9.9 / 11.4 us, 4096 x 4096 x 1024 42 / 30.6 / 29.6 us (128 x 128,
+// 128 x 256, pair).  Weighing rounds alone (0.68 : 0.88 : 1) took 26.8 us for 2313 x 1024 x 4096
+// (pair; 25.2 with 128 x 256) and 30.7 us for 1024 x 1024 x 8192 (128 x 128 in 2 slices; 24.3 with
+// pairs in 4).  With at most 8 slices a 64 x 64 weight gradient over 802816 pixels ran on
+// 8 SMs: the 49 split GEMMs of a ResNet-50 step took 9.0 ms (its 1x1 layers 2.0 ms now).
+static TilePlan gemm_plan(int M, int N, int K, bool both_mn, int bn_hint, bool can_split,
+                          bool pairs) {
+  TilePlan best_plan;
+  const int sms = num_sms();
+  const long long mblk = (M + BM - 1) / BM;
+  const int kb = (K + BK - 1) / BK;
+  double best = 1e30;
+  const double mn = both_mn ? 1.2 : 1.0;
+  auto consider = [&](int kind_bn, bool kind_pair, long long tiles, int slots, double fixed,
+                      double extra) {
+    const int most = can_split && tiles * 10 <= slots * 7 ? 64 : 1;
+    for (int S = 1; S <= most && (S == 1 || S <= slots / tiles); ++S) {
+      if (S > 1 && ((K / BK) / S < 8 || (long long)S * M * N > SPLITK_MAX_FLOATS)) break;
+      const long long r = (tiles * S + slots - 1) / slots;
+      double step = 0.27;
+      if (kind_bn == 256 && !kind_pair) {
+        const double busy = (double)(tiles * S) / r;
+        step *= mn * (busy > 110.0 ? busy / 110.0 : 1.0);
       }
-    };
-    const bool any = bn_hint != 128 && bn_hint != 256 && bn_hint != 512;
-    if (bn_hint == 128 || any) consider(128, false, mblk * ((N + 127) / 128), sms, 4.6, 1.0);
-    if (bn_hint == 256 || (any && N > 128))
-      consider(256, false, mblk * ((N + 255) / 256), sms, 6.1, 1.8);
-    if (bn_hint == 512 || (any && g_pair_enabled && M > 128 && N > 128 &&
-                           !(g.ag_ctas && (g.ag_rows_per_rank % 256))))
-      consider(256, true, ((M + 255) / 256) * (long long)((N + 255) / 256), sms / 2, 7.8, 1.2);
-    if (g.split_k > 1) g.splitk_ws = g_splitk_ws;
+      const double c = fixed + r * (step * ((kb + S - 1) / S)) + (r - 1) * extra +
+                       (S > 1 ? 2.5 + (double)S * M * N * 1e-6 : 0.0);
+      if (c < best) {
+        best = c;
+        best_plan.BN = kind_bn;
+        best_plan.pair = kind_pair;
+        best_plan.slices = S;
+      }
+    }
+  };
+  const bool any = bn_hint != 128 && bn_hint != 256 && bn_hint != 512;
+  if (bn_hint == 128 || any) consider(128, false, mblk * ((N + 127) / 128), sms, 4.6, 1.0);
+  if (bn_hint == 256 || (any && N > 128))
+    consider(256, false, mblk * ((N + 255) / 256), sms, 6.1, 1.8);
+  if (bn_hint == 512 || (any && pairs && M > 128 && N > 128))
+    consider(256, true, ((M + 255) / 256) * (long long)((N + 255) / 256), sms / 2, 7.8, 1.2);
+  return best_plan;
+}
+
+// K can be cut into slices when nothing but a sum and a factor follows: the slices' fp32 sums
+// go through a workspace and a second kernel adds them up, four columns at a time.
+static bool splittable(int N, int K, long long ldc) {
+  return g_splitk_enabled && N % 4 == 0 && ldc % 4 == 0 && K >= 2048;
+}
+
+// slices > 1: the number that nkb_gemm_slices gave for these sizes, ws holds that many fp32
+// matrices [M, N].
+static int gemm_run(GemmArgs g, const void* A, long long lda, int a_mn, const void* B,
+                    long long ldb, int b_mn, int max_ctas, int bn_hint, float* ws, int slices,
+                    void* stream) {
+  const int M = g.M, N = g.N, K = g.K;
+  const bool split = slices > 1;
+  if (split) {
+    const uintptr_t align = g.c_fp32 ? 15 : 7;  // the reduction writes four values at a time
+    if (!ws || g.ag_ctas || g.rs_on || g.epi != NKB_EPI_NONE || g.bias || g.res ||
+        !splittable(N, K, g.ldc) || (reinterpret_cast<uintptr_t>(g.C) & align) ||
+        (reinterpret_cast<uintptr_t>(ws) & 15))
+      return -3;
   }
+  const TilePlan plan = gemm_plan(M, N, K, a_mn && b_mn, bn_hint, split,
+                                  g_pair_enabled && !(g.ag_ctas && (g.ag_rows_per_rank % 256)));
+  if (split && plan.slices != slices) return -3;
+  const int BN = plan.BN;
+  const bool pair = plan.pair;
+  g.split_k = plan.slices;
+  g.splitk_ws = split ? ws : nullptr;
   CUtensorMap tmA, tmB;
   int rc;
   g.tma_c = g.tma_aux = 0;
@@ -1682,6 +1700,24 @@ extern "C" int nkb_gemm_bf16(const void* A, long long lda, int a_mn, const void*
                              long long ldres, int epi, void* aux, long long ldaux, int* status,
                              const int* ready_flags, int rows_per_flag, int ready_target,
                              int max_ctas, int bn_hint, const float* alpha_dev, void* stream) {
+  return nkb_gemm_bf16_ws(A, lda, a_mn, B, ldb, b_mn, C, ldc, c_fp32, accumulate, M, N, K, alpha,
+                          bias, res, ldres, epi, aux, ldaux, status, ready_flags, rows_per_flag,
+                          ready_target, max_ctas, bn_hint, alpha_dev, nullptr, 1, stream);
+}
+
+extern "C" int nkb_gemm_slices(int M, int N, int K, int a_mn, int b_mn, long long ldc,
+                               int bn_hint) {
+  if (M <= 0 || N <= 0 || !splittable(N, K, ldc)) return 1;
+  return gemm_plan(M, N, K, a_mn && b_mn, bn_hint, true, g_pair_enabled).slices;
+}
+
+extern "C" int nkb_gemm_bf16_ws(const void* A, long long lda, int a_mn, const void* B,
+                                long long ldb, int b_mn, void* C, long long ldc, int c_fp32,
+                                int accumulate, int M, int N, int K, float alpha,
+                                const void* bias, const void* res, long long ldres, int epi,
+                                void* aux, long long ldaux, int* status, const int* ready_flags,
+                                int rows_per_flag, int ready_target, int max_ctas, int bn_hint,
+                                const float* alpha_dev, float* ws, int slices, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return -2;
   // TMA needs 16-byte aligned bases and row pitches
   if ((lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(A) & 15) ||
@@ -1703,7 +1739,7 @@ extern "C" int nkb_gemm_bf16(const void* A, long long lda, int a_mn, const void*
   g.ready_target = ready_target;
   g.ag_ctas = 0;
   g.rs_on = 0;
-  return gemm_run(g, A, lda, a_mn, B, ldb, b_mn, max_ctas, bn_hint, stream);
+  return gemm_run(g, A, lda, a_mn, B, ldb, b_mn, max_ctas, bn_hint, ws, slices, stream);
 }
 
 
@@ -1751,7 +1787,7 @@ extern "C" int nkb_ag_gemm_bf16(void** heap, long long flag_off, long long data_
   g.ag_rows_per_rank = rows_per_rank;
   g.ag_row_bytes = (long long)K * 2;
   g.ag_pitch = lda * 2;
-  int rc = gemm_run(g, A_local, lda, 0, B, ldb, b_mn, 0, bn_hint, stream);
+  int rc = gemm_run(g, A_local, lda, 0, B, ldb, b_mn, 0, bn_hint, nullptr, 1, stream);
   if (rc) return rc;
   if (world > 1) {
     epoch_bump_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(epoch);
@@ -1797,7 +1833,7 @@ extern "C" int nkb_gemm_rs_bf16(void** heap, long long flag_off, long long stage
   // the tile-flag layout depends on the tile width: fix it (pair tiles when shards are
   // multiples of 256 rows, else single-CTA 128 x 256)
   if (bn_hint == 0) bn_hint = (rows_per_rank % 256 == 0 && g_pair_enabled) ? 512 : 256;
-  int rc = gemm_run(g, A, lda, 0, B, ldb, b_mn, 0, bn_hint, stream);
+  int rc = gemm_run(g, A, lda, 0, B, ldb, b_mn, 0, bn_hint, nullptr, 1, stream);
   if (rc) return rc;
   epoch_bump_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(epoch);
   return (int)cudaGetLastError();

@@ -26,6 +26,17 @@ int nkb_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long lo
                   void* aux, long long ldaux, int* status, const int* ready_flags,
                   int rows_per_flag, int ready_target, int max_ctas, int bn_hint,
                   const float* alpha_dev, void* stream);
+// The number of slices (>= 1) into which a GEMM of these sizes without bias, residual and
+// activation cuts K, and the same GEMM with that number and the fp32 [slices][M][N] workspace of
+// its partial sums.  The workspace is the call's own: no other work may use it before both of
+// the call's kernels have run.
+int nkb_gemm_slices(int M, int N, int K, int a_mn, int b_mn, long long ldc, int bn_hint);
+int nkb_gemm_bf16_ws(const void* A, long long lda, int a_mn, const void* B, long long ldb,
+                     int b_mn, void* C, long long ldc, int c_fp32, int accumulate, int M, int N,
+                     int K, float alpha, const void* bias, const void* res, long long ldres,
+                     int epi, void* aux, long long ldaux, int* status, const int* ready_flags,
+                     int rows_per_flag, int ready_target, int max_ctas, int bn_hint,
+                     const float* alpha_dev, float* ws, int slices, void* stream);
 
 // ---- norm.cu ---------------------------------------------------------------
 // rms = 1: RMSNorm (no mean, no bias).  stats: [rows,2] fp32 (mean, rstd).

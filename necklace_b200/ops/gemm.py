@@ -90,36 +90,24 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if ldb % 8 or pb % 16:
         b = _repack(b)
         pb, ldb = b.data_ptr(), b.stride(0)
-    if a.get_device() not in _WORKSPACE:
-        _ensure_workspace(a.device)
-    _lib.call("nkb_gemm_bf16", pa, lda, a_mn, pb, ldb, b_mn, out.data_ptr(), out.stride(0), fp32,
-              accumulate, M, N, K, alpha, None if bias is None else bias.data_ptr(),
+    slices, ws = 1, None
+    if K >= 2048 and epi == EPI_NONE and bias is None and res is None \
+            and out.data_ptr() % (16 if fp32 else 8) == 0:
+        slices = _lib.value("nkb_gemm_slices", M, N, K, a_mn, b_mn, out.stride(0), bn)
+        if slices > 1:
+            # the partial sums' memory belongs to this call: the allocator orders its reuse on
+            # the stream (also while a graph is captured), and no other thread gets it meanwhile
+            ws = torch.empty(slices * M * N, dtype=torch.float32, device=a.device)
+    _lib.call("nkb_gemm_bf16_ws", pa, lda, a_mn, pb, ldb, b_mn, out.data_ptr(), out.stride(0),
+              fp32, accumulate, M, N, K, alpha, None if bias is None else bias.data_ptr(),
               None if res is None else res.data_ptr(), 0 if res is None else res.stride(0), epi,
               None if aux is None else aux.data_ptr(), 0 if aux is None else aux.stride(0),
               status_ptr(a), None if ready_flags is None else ready_flags.data_ptr(),
               rows_per_flag, ready_target, max_ctas, bn,
-              None if alpha_dev is None else alpha_dev.data_ptr(), _lib.stream_ptr())
+              None if alpha_dev is None else alpha_dev.data_ptr(),
+              None if ws is None else ws.data_ptr(), slices, _lib.stream_ptr())
     _lib.count_launch()
     return out
-
-
-_WORKSPACE: dict = {}
-SPLITK_WORKSPACE_FLOATS = 32 * 1024 * 1024  # 128 MB: 8 slices of a 1024 x 4096 fp32 tile set
-
-
-def _ensure_workspace(device) -> None:
-    """Hand the library its split-K workspace (the library itself never allocates).  One
-    buffer per device, owned here for the life of the process; weight-gradient GEMMs with
-    few output tiles and a long K use it to spread their K range over all SMs."""
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    if idx in _WORKSPACE:
-        return
-    ws = torch.empty(SPLITK_WORKSPACE_FLOATS, dtype=torch.float32, device=device)
-    _WORKSPACE[idx] = ws
-    lib = _lib.load()
-    lib.nkb_gemm_set_workspace.argtypes = [_lib.vp, _lib.i64]
-    lib.nkb_gemm_set_workspace.restype = None
-    lib.nkb_gemm_set_workspace(ws.data_ptr(), ws.numel())
 
 
 def set_splitk(enabled: bool) -> None:
