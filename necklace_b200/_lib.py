@@ -32,6 +32,7 @@ _SIGS = {
     "nkb_gemm_slices": [i32, i32, i32, i32, i32, i64, i32],
     "nkb_gemm_bf16_ws": [vp, i64, i32, vp, i64, i32, vp, i64, i32, i32, i32, i32, i32, f32, vp,
                          vp, i64, i32, vp, i64, vp, vp, i32, i32, i32, i32, vp, vp, i32, vp],
+    "nkb_capture_id": [vp],
     "nkb_norm_fwd": [vp, vp, vp, vp, vp, i32, i32, f32, i32, vp],
     "nkb_norm_bwd_dx": [vp, vp, vp, vp, vp, i32, i32, i32, vp],
     "nkb_norm_bwd_dx_res": [vp, vp, vp, vp, vp, i32, i32, i32, vp, vp],

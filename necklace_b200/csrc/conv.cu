@@ -12,6 +12,8 @@
 // The reference trains CNNs through torch's cuDNN convolutions
 // (examples/dp/mnist/pytorch/main.py); these kernels take their place for the ResNet-50
 // configuration.
+#include <mutex>
+
 #include "ptx.cuh"
 #include "nkb_api.h"
 
@@ -698,6 +700,10 @@ static void bn_sums_dims(long long M, int C, int& cx, dim3& grid) {
 // Forward: batch statistics of x [M, C], then y = act(bn(x) (+ res)).  acc: fp32 [2][C], zero on
 // entry, left zero.  stats out: fp32 [2][C] (mean, rstd).  mask (optional): one bit per element,
 // y > 0, in [M * C / 8] bytes, bit j of byte i for element 8 i + j.
+//
+// The kernels of a call hand their sums on through `acc`, which calls on one stream share: no other
+// thread's call on that stream may come between them.
+static std::mutex g_bn_order;
 extern "C" int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, const void* res,
                           void* y, void* mask, float* stats, float* acc, float* run_mean, float* run_var,
                           long long M, int C, float eps, float momentum, int relu, void* stream) {
@@ -710,6 +716,7 @@ extern "C" int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, co
   int cx;
   dim3 grid;
   bn_sums_dims(M, C, cx, grid);
+  std::lock_guard<std::mutex> order(g_bn_order);
   bn_sums_kernel<0><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), nullptr, nullptr,
                                          nullptr, acc, M, C, cx);
   bn_finalize_kernel<<<(C + 127) / 128, 128, 0, s>>>(acc, stats, run_mean, run_var, M, C, eps,
@@ -765,6 +772,7 @@ extern "C" int nkb_bn_bwd(const void* dy, const void* x, const void* mask, const
   int cx;
   dim3 grid;
   bn_sums_dims(M, C, cx, grid);
+  std::lock_guard<std::mutex> order(g_bn_order);
   bn_sums_kernel<1><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(dy),
                                          static_cast<const __nv_bfloat16*>(x),
                                          static_cast<const uint8_t*>(mask), stats, acc, M, C,

@@ -136,3 +136,14 @@ extern "C" int nkb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long lo
       static_cast<__nv_bfloat16*>(dgu), T, F);
   return (int)cudaGetLastError();
 }
+
+// A number (> 0) for the graph capture that `stream` takes part in, 0 outside of one.
+extern "C" int nkb_capture_id(void* stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &st, &id) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream while another thread captures: not part of it
+    return 0;
+  }
+  return st == cudaStreamCaptureStatusActive ? (int)(id % 0x7fffffff) + 1 : 0;
+}

@@ -38,6 +38,10 @@ int nkb_gemm_bf16_ws(const void* A, long long lda, int a_mn, const void* B, long
                      int rows_per_flag, int ready_target, int max_ctas, int bn_hint,
                      const float* alpha_dev, float* ws, int slices, void* stream);
 
+// ---- elementwise.cu ----------------------------------------------------------
+// A number (> 0) for the graph capture that `stream` takes part in, 0 outside of one.
+int nkb_capture_id(void* stream);
+
 // ---- norm.cu ---------------------------------------------------------------
 // rms = 1: RMSNorm (no mean, no bias).  stats: [rows,2] fp32 (mean, rstd).
 int nkb_norm_fwd(const void* x, const void* w, const void* b, void* y, float* stats, int rows,

@@ -1,6 +1,8 @@
 """Shared helpers for the operator wrappers."""
 from __future__ import annotations
 
+import threading
+
 import torch
 import torch.autograd.forward_ad as _fwd_ad
 
@@ -8,7 +10,9 @@ from .. import _lib
 
 _status: dict[int, torch.Tensor] = {}
 _status_at: dict[int, int] = {}      # their addresses: the tensors live as long as the process
-_scratch: dict[tuple, torch.Tensor] = {}
+_scratch: dict[tuple, object] = {}   # (tag, device, stream, capture) -> what `make` gave
+_scratch_lock = threading.Lock()
+_SCRATCH_KEPT = 48                   # of 1/2 MB at most
 
 STATUS_TEXT = {
     0: "ok", 1: "MMA warp timed out waiting for a TMA stage",
@@ -61,24 +65,22 @@ def check_status(reset: bool = True) -> None:
                 f"device-side error {code} on cuda:{dev}: {STATUS_TEXT.get(code, 'unknown')}")
 
 
-def scratch(key: str, numel: int, dtype: torch.dtype, device) -> torch.Tensor:
-    """A cached scratch tensor per (key, device); grown, never shrunk."""
-    k = (key, str(device), dtype)
+def stream_scratch(tag: str, device: torch.device, make):
+    """Scratch that kernels find at zero and leave at zero (accumulators, ticket counters), made by
+    ``make()`` once per device and stream: what runs on another stream may run at the same time.
+    A graph being captured gets scratch of its own, cleared by the graph itself, because replays
+    of two graphs may overlap wherever they were captured."""
+    s = _lib.stream_ptr()
+    capture = _lib.value("nkb_capture_id", s)
+    k = (tag, device.index, s, capture)
     t = _scratch.get(k)
-    if t is None or t.numel() < numel:
-        t = torch.empty(max(numel, 1), dtype=dtype, device=device)
-        _scratch[k] = t
-    return t[:numel]
-
-
-def scratch_zero(key: str, numel: int, dtype: torch.dtype, device) -> torch.Tensor:
-    """Like ``scratch`` but zero-filled when (re)allocated; for kernels that leave their
-    scratch at zero on exit (accumulators, ticket counters)."""
-    k = (key, str(device), dtype, "z")
-    t = _scratch.get(k)
-    if t is None or t.numel() < numel:
-        t = torch.zeros(max(numel, 1), dtype=dtype, device=device)
-        _scratch[k] = t
+    if t is None:
+        t = make()
+        with _scratch_lock:
+            # what is dropped goes back to the allocator, which orders its reuse on its stream
+            for old in [o for o in _scratch if not capture or o[3] != capture][:-_SCRATCH_KEPT]:
+                del _scratch[old]
+            _scratch[k] = t
     return t
 
 

@@ -19,7 +19,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ._common import on_gpu, plain_call, ptr, scratch_zero, status_ptr
+from ._common import on_gpu, plain_call, ptr, status_ptr, stream_scratch
 from .gemm import _deliver_grad, gemm
 
 
@@ -250,7 +250,8 @@ class Conv2d(nn.Module):
 
 # ------------------------------------------------------------------------ batch norm
 def _bn_acc(C, device):
-    return scratch_zero("bn_acc", 2 * 8192, torch.float32, device)
+    return stream_scratch("batch_norm", device, lambda: torch.zeros(
+        2 * 8192, dtype=torch.float32, device=device))
 
 
 class BatchNormFn(torch.autograd.Function):

@@ -16,7 +16,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _lib
-from ._common import on_gpu, plain_call, ptr, scratch, scratch_zero, status_ptr
+from ._common import on_gpu, plain_call, status_ptr, stream_scratch
 
 EPI_NONE, EPI_GELU_FWD, EPI_GELU_BWD, EPI_RELU = 0, 1, 2, 3
 
@@ -147,12 +147,12 @@ def colsum(dy: torch.Tensor, out: torch.Tensor | None = None, accumulate: bool =
 
 
 def colsum_scratch(Cn: int, device):
-    """fp32 accumulator [2][C] and ticket counters of the fused column-sum kernel; shared by
-    all calls on the device's compute stream (the kernel leaves both at zero)."""
-    acc = scratch_zero("colsum_acc", 2 * 65536, torch.float32, device)
-    tickets = scratch_zero("colsum_tickets", 256, torch.int32, device)
+    """fp32 accumulator [2][C] and ticket counters of the kernels that sum columns (each leaves
+    both at zero), shared by the calls on one stream."""
     assert Cn <= 65536
-    return acc, tickets
+    return stream_scratch("colsum", device, lambda: (
+        torch.zeros(2 * 65536, dtype=torch.float32, device=device),
+        torch.zeros(256, dtype=torch.int32, device=device)))
 
 
 # ---------------------------------------------------------------- autograd

@@ -36,7 +36,7 @@ def _gemms(seed):
     return run, [o for _, _, o in ops]
 
 
-def _same_side_by_side(make, how):
+def _same_side_by_side(make, how, same=torch.equal):
     from necklace_b200.ops._common import check_status
     runs, outs = zip(*(make(s) for s in range(2)))
     for r in runs:
@@ -72,7 +72,7 @@ def _same_side_by_side(make, how):
     check_status()
     for out, w in zip(outs, want):
         for o, v in zip(out, w):
-            assert torch.equal(o, v)
+            assert same(o, v)
 
 
 @pytest.mark.gpu
@@ -94,3 +94,56 @@ def test_output_that_a_split_cannot_write():
         want, mag = a.double().t() @ b.double(), a.double().abs().t() @ b.double().abs()
         bound = want.abs() * rel + mag * 4112 * 2.0 ** -24
         assert bool(((out.double() - want).abs() <= bound).all())
+
+
+def _sums(seed):
+    """Norms and column sums there and back; inputs of the two sets are far apart, so that a sum
+    that gets a share of the other's shows."""
+    from necklace_b200.ops import LayerNorm
+    from necklace_b200.ops.conv import BatchNorm2d
+    from necklace_b200.ops.gemm import colsum
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    ln, bn = LayerNorm(512, device="cuda"), BatchNorm2d(512, relu=True, device="cuda")
+    x = (r(3000, 512) * (1 + 3 * seed) + 4 * seed).bfloat16()
+    dy = (r(3000, 512) + 2 - 4 * seed).bfloat16()
+    xs = [x.clone().requires_grad_(True) for _ in range(2)]
+    outs = [torch.empty_like(t) for t in (ln.weight, ln.bias, xs[0], bn.weight, bn.bias, xs[1],
+                                          ln.bias)]
+
+    def run():
+        got = torch.autograd.grad(ln(xs[0]), [ln.weight, ln.bias, xs[0]], dy)
+        got += torch.autograd.grad(bn(xs[1].view(50, 60, 1, 512)).view(3000, 512),
+                                   [bn.weight, bn.bias, xs[1]], dy)
+        for o, v in zip(outs, got + (colsum(dy),)):
+            o.copy_(v)
+    return run, outs
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["streams", "threads", "graphs"])
+def test_sums_side_by_side(how):
+    # the sums are added in any order (fp32, rounded to bf16 once)
+    _same_side_by_side(_sums, how, lambda o, v: bool(
+        ((o.double() - v.double()).abs() <= v.double().abs() * 2.0 ** -6
+         + v.double().square().mean().sqrt() * 2.0 ** -6).all()))
+
+
+@pytest.mark.gpu
+def test_first_use_inside_a_capture():
+    """Scratch made while a graph is captured is cleared by the graph, not by the capture."""
+    from necklace_b200.ops.gemm import colsum
+    dy = torch.randn(700, 264, device="cuda").bfloat16()
+    want = colsum(dy)
+    s = torch.cuda.Stream()                           # nothing has run on it yet
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        out = colsum(dy)
+    for _ in range(3):
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.allclose(out.float(), want.float(), rtol=2.0 ** -7, atol=1e-2)
+    with torch.cuda.stream(s):                        # the stream's own scratch afterwards
+        again = colsum(dy)
+    torch.cuda.synchronize()
+    assert torch.allclose(again.float(), want.float(), rtol=2.0 ** -7, atol=1e-2)
