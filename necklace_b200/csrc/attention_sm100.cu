@@ -769,13 +769,8 @@ template <int D, int EXPM>
 static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                       const AttnFwdArgs& a, cudaStream_t s) {
   constexpr int smem = 4 * (128 * D * 2) + 32768 + 4096 + 1024 + 128;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<D, EXPM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static bool done[64];
+  if (int e = allow_smem(attn_fwd_kernel<D, EXPM>, smem, done)) return e;
   dim3 grid(a.B * a.H, (a.S + 127) / 128);
   attn_fwd_kernel<D, EXPM><<<grid, ATT_THREADS, smem, s>>>(tq, tk, tv, a);
   return (int)cudaGetLastError();
@@ -788,13 +783,8 @@ template <int D, int EXPM>
 static int launch_fwd_pp(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const AttnFwdArgs& a, cudaStream_t s) {
   constexpr int smem = 6 * (128 * D * 2) + 1024 + 256;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_pp_kernel<D, EXPM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static bool done[64];
+  if (int e = allow_smem(attn_fwd_pp_kernel<D, EXPM>, smem, done)) return e;
   dim3 grid(a.B * a.H, (a.S + 255) / 256);
   attn_fwd_pp_kernel<D, EXPM><<<grid, ATT2_THREADS, smem, s>>>(tq, tk, tv, a);
   return (int)cudaGetLastError();
@@ -817,13 +807,8 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
                       const CUtensorMap& tdo, const AttnBwdArgs& a, cudaStream_t s) {
   constexpr int STAGES = (D == 64) ? 2 : 1;
   constexpr int smem = (2 + 2 * STAGES) * (128 * D * 2) + 65536 + 1024 + 128;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<D>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static bool done[64];
+  if (int e = allow_smem(attn_bwd_kernel<D>, smem, done)) return e;
   dim3 grid(a.B * a.H, (a.S + 127) / 128);
   attn_bwd_kernel<D><<<grid, ATT_THREADS, smem, s>>>(tq, tk, tv, tdo, a);
   return (int)cudaGetLastError();
@@ -852,13 +837,8 @@ static int launch_bwd_pp(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
                          const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdArgs& a,
                          cudaStream_t s) {
   constexpr int smem = AttnBwd2Smem<D>::BYTES;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_pp_kernel<D>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static bool done[64];
+  if (int e = allow_smem(attn_bwd_pp_kernel<D>, smem, done)) return e;
   dim3 grid(a.B * a.H, (a.S + 127) / 128);
   attn_bwd_pp_kernel<D><<<grid, BWD2_THREADS, smem, s>>>(tq, tk, tv, tdo, tdq, a);
   return (int)cudaGetLastError();

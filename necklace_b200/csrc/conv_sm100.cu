@@ -564,13 +564,8 @@ template <int KIND, int BN>
 static int launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& o,
                   const ConvArgs& g, int units, cudaStream_t s) {
   auto kern = conv_kernel<KIND, BN>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         ConvCfg<KIND, BN>::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static bool done[64];
+  if (int e = allow_smem(kern, ConvCfg<KIND, BN>::SMEM, done)) return e;
   const int sms = num_sms();
   kern<<<units < sms ? units : sms, CV_THREADS, ConvCfg<KIND, BN>::SMEM, s>>>(a, b, o, g);
   return (int)cudaGetLastError();

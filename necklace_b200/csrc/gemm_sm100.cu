@@ -1476,14 +1476,9 @@ static int launch_gemm_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm
   constexpr int STAGES = (BN == 256) ? 4 : 6;
   constexpr int smem_bytes =
       STAGES * (A_STAGE_BYTES + BN * BK * 2) + EPI_WARPS * EPI_STAGE_BYTES + 1024 + 256;
-  static bool configured = false;
+  static bool done[64];
   auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, MODE>;
-  if (!configured) {
-    cudaError_t e =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (int e = allow_smem(kern, smem_bytes, done)) return e;
   g.num_m_blocks = (g.M + BM - 1) / BM;
   g.num_n_blocks = (g.N + BN - 1) / BN;
   int tiles = g.num_m_blocks * g.num_n_blocks * g.split_k;
@@ -1509,14 +1504,9 @@ template <bool A_MN, bool B_MN, int MODE>
 static int launch_gemm_pair_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmArgs& g,
                                  int max_ctas, cudaStream_t stream) {
   constexpr int smem_bytes = PAIR_STAGES * PAIR_STAGE_BYTES + EPI_WARPS * EPI_STAGE_BYTES + 1024 + 256;
-  static bool configured = false;
+  static bool done[64];
   auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, MODE>;
-  if (!configured) {
-    cudaError_t e =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (int e = allow_smem(kern, smem_bytes, done)) return e;
   g.num_m_blocks = (g.M + 255) / 256;
   g.num_n_blocks = (g.N + 255) / 256;
   int tiles = g.num_m_blocks * g.num_n_blocks * g.split_k;

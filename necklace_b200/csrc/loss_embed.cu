@@ -267,14 +267,9 @@ static int launch_ce(void* logits, const long long* targets, float* out, const f
     if (need <= 200 * 1024) {
       smem = need;
       use_smem = 1;
-      static size_t configured = 0;
-      if (need > 48 * 1024 && need > configured) {
-        cudaError_t e = cudaFuncSetAttribute(ce_kernel<MODE>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             200 * 1024);
-        if (e != cudaSuccess) return (int)e;
-        configured = 200 * 1024;
-      }
+      static bool done[64];
+      if (need > 48 * 1024)
+        if (int e = allow_smem(ce_kernel<MODE>, 200 * 1024, done)) return e;
     }
   }
   ce_kernel<MODE><<<T, CE_THREADS, smem, s>>>(static_cast<__nv_bfloat16*>(logits), targets, out,

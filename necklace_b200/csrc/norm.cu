@@ -591,18 +591,10 @@ extern "C" int nkb_norm_bwd_all(const void* dy, const void* x, const void* w, co
                                 accum_w, accum_b, s);
 }
 
-// the ring needs more than the 48 KB a kernel gets without opting in (once per device)
+// the ring needs more than the 48 KB a kernel gets without opting in
 static int colsum_configure() {
-  static bool done[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-  if (!done[dev]) {
-    if (cudaFuncSetAttribute(nkb::colsum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             nkb::COLSUM_SMEM_BYTES) != cudaSuccess)
-      return -1;
-    done[dev] = true;
-  }
-  return 0;
+  static bool done[64];
+  return nkb::allow_smem(nkb::colsum_kernel, nkb::COLSUM_SMEM_BYTES, done);
 }
 
 // row splits: about three CTAs per SM (64 KB of ring each), and at least COLSUM_UNROLL rows per

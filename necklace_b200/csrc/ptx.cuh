@@ -37,6 +37,20 @@ enum : int {
   NKB_ERR_BOUNDS = 6,      // an index check failed (debug builds)
 };
 
+// Lets `kern` have `bytes` of dynamic shared memory.  The attribute belongs to the kernel on one
+// device, so it is set before the first launch on each; `done` is the caller's, one per kernel.
+template <typename K>
+inline int allow_smem(K kern, int bytes, bool (&done)[64]) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const bool known = e == cudaSuccess && dev >= 0 && dev < 64;
+  if (known && done[dev]) return 0;
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (known && e == cudaSuccess) done[dev] = true;
+  return (int)e;
+}
+
 // ---------------------------------------------------------------- debug bounds checks
 // With -DNKB_DEBUG_BOUNDS every kernel that computes global-memory indices by hand checks
 // them against the extents it was told (NKB_IN_BOUNDS).  A failing check records how many

@@ -4,6 +4,7 @@ a variable from another scope would only surface there."""
 import ast
 import builtins
 import os
+import re
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -92,3 +93,14 @@ def test_the_scan_sees_an_unbound_name(tmp_path):
     p.write_text("class A:\n    def __init__(self, x):\n        self.x = x\n"
                  "        if which == 4:\n            pass\n")
     assert check(str(p)) == [("__init__", 4, "which")]
+
+
+def test_kernel_attributes_are_set_on_every_device():
+    """A kernel's shared-memory limit holds on one device only.  One helper sets it, per device;
+    a `static bool` next to a launch would set it on the first device and fail on the next."""
+    csrc = os.path.join(ROOT, "necklace_b200", "csrc")
+    for f in sorted(os.listdir(csrc)):
+        src = open(os.path.join(csrc, f)).read()
+        assert src.count("cudaFuncSetAttribute(") == (f == "ptx.cuh"), f
+        for line in src.splitlines():
+            assert not re.match(r"\s*static bool \w+( =|;)", line), (f, line)
