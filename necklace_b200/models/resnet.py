@@ -35,7 +35,8 @@ class Bottleneck(nn.Module):
             self.down_bn = BatchNorm2d(width * 4, device=device)
 
     def forward(self, x):
-        x, out = self.conv1.split(x)     # the residual path's gradient is added in conv1's
+        # the residual path's gradient is added in conv1's (a module put in its place is called)
+        x, out = self.conv1.split(x) if isinstance(self.conv1, Conv2d) else (x, self.conv1(x))
         idt = x if self.down_conv is None else self.down_bn(self.down_conv(x))
         out = self.bn1(out)
         out = self.bn2(self.conv2(out))

@@ -17,6 +17,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import _lib
 from ._common import on_gpu, plain_call, ptr, status_ptr, stream_scratch
@@ -240,12 +241,19 @@ class Conv2d(nn.Module):
 
     def split(self, x):
         """``(x, conv(x))`` at the head of a residual block (see ``Conv1x1SplitFn``)."""
-        hooked = self._forward_hooks or self._forward_pre_hooks or self._backward_hooks \
-            or self._backward_pre_hooks         # they see calls of the module
         if (self.k, self.stride, self.pad) == (1, 1, 0) and x.shape[-1] % 8 == 0 \
-                and not hooked and not plain_call():
+                and x.requires_grad and not plain_call() and not self._observed():
             return Conv1x1SplitFn.apply(x, self.weight)
         return x, self(x)
+
+    def _observed(self) -> bool:
+        """Whether something would notice that the module is not called: hooks of its own or
+        global ones, or a forward of a subclass or of this instance."""
+        cls = type(self)
+        return bool(self._forward_hooks or self._forward_pre_hooks or self._backward_hooks
+                    or self._backward_pre_hooks or _has_any_global_hook()
+                    or cls.forward is not Conv2d.forward or cls.__call__ is not nn.Module.__call__
+                    or "forward" in self.__dict__)
 
 
 # ------------------------------------------------------------------------ batch norm
