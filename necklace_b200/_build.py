@@ -13,14 +13,16 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(os.path.dirname(HERE), "build", "nkb200")
 LIB = os.path.join(HERE, "_nkb200.so")
-# the same entry points as a Python extension (csrc/pycall.cpp), linked to LIB
-EXT = os.path.join(HERE, "_nkpy.so")
+# the same entry points as a Python extension (csrc/pycall.cpp), linked to LIB; the suffix names
+# the interpreter, so another Python version in the same checkout does not load it
+EXT = os.path.join(HERE, "_nkpy" + sysconfig.get_config_var("EXT_SUFFIX"))
 # the bounds-checked debug variant (-DNKB_DEBUG_BOUNDS): ``--debug-bounds``
 BUILD_DBG = os.path.join(os.path.dirname(HERE), "build", "nkb200_dbg")
 LIB_DBG = os.path.join(HERE, "_nkb200_dbg.so")
@@ -83,27 +85,40 @@ def build(force: bool = False, verbose: bool = False, debug_bounds: bool = False
         if p.returncode != 0:
             raise RuntimeError(f"link failed:\n{p.stdout}{p.stderr}")
     if not debug_bounds:
-        _build_ext(force)
+        build_ext(force)
     return lib
 
 
-def _build_ext(force: bool) -> None:
+def build_ext(force: bool = False) -> bool:
+    """Compile the Python extension; whether there is one.  Every call also works through ctypes,
+    more slowly, so a failure is a warning."""
+    untagged = os.path.join(os.path.dirname(EXT), "_nkpy.so")
+    if os.path.exists(untagged):           # as it was named before, for any interpreter
+        os.remove(untagged)
     src = os.path.join(CSRC, "pycall.cpp")
     newest = max(os.path.getmtime(src), _headers_mtime())
     if not force and os.path.exists(EXT) and os.path.getmtime(EXT) >= newest:
-        return
+        return True
     inc = sysconfig.get_paths()["include"]
-    if not os.path.exists(os.path.join(inc, "Python.h")):
-        return                  # without the headers every call goes through ctypes
     # built under another name and moved: a process may be importing it
     tmp = EXT + f".{os.getpid()}"
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-I", inc, "-I",
            CSRC, src, "-o", tmp, "-L", HERE, "-l:" + os.path.basename(LIB),
            "-Wl,-rpath,$ORIGIN"]
-    p = subprocess.run(cmd, capture_output=True, text=True)
-    if p.returncode != 0:
-        raise RuntimeError(f"building {EXT} failed:\n{p.stdout}{p.stderr}")
-    os.replace(tmp, EXT)
+    try:
+        p = subprocess.run(cmd, capture_output=True, text=True)
+        log = f"exit code {p.returncode}\n{p.stdout}{p.stderr}" if p.returncode else ""
+    except OSError as e:
+        log = str(e)
+    if not log:
+        os.replace(tmp, EXT)
+        return True
+    # one that was built for other signatures must not stay
+    for old in (tmp, EXT):
+        if os.path.exists(old):
+            os.remove(old)
+    warnings.warn(f"building {EXT} failed, calls go through ctypes:\n{log[-2000:]}", stacklevel=2)
+    return False
 
 
 def resource_report() -> str:

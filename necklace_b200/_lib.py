@@ -10,6 +10,7 @@ reference implementation for CPU tensors.
 from __future__ import annotations
 
 import ctypes as C
+import importlib
 import os
 import threading
 
@@ -133,12 +134,17 @@ def debug_bounds(raise_on_error: bool = True) -> dict:
 _fast: dict = {}
 
 
-def _load_fast() -> dict:
+def _load_fast(build_if_missing: bool) -> dict:
     if DEBUG_BOUNDS:
         return {}           # the extension is linked to the normal library
     try:
         from . import _nkpy
     except ImportError:
+        if build_if_missing:
+            from . import _build
+            if _build.build_ext():
+                importlib.invalidate_caches()
+                return _load_fast(False)
         return {}
     return {n: getattr(_nkpy, n) for n in dir(_nkpy) if n.startswith("nkb_")}
 
@@ -163,7 +169,7 @@ def load(build_if_missing: bool = True):
                 fn.restype = i32
             if hasattr(lib, "nkb_build_info"):
                 lib.nkb_build_info.restype = C.c_char_p
-            _fast.update(_load_fast())
+            _fast.update(_load_fast(build_if_missing))
             _lib = lib
         except Exception as e:  # noqa: BLE001
             _load_error = e
