@@ -49,9 +49,11 @@ def status_ptr(t: torch.Tensor) -> int:
 
 def plain_call() -> bool:
     """Whether an operator may run its forward pass without an autograd node: gradients are off,
-    and neither forward-mode differentiation nor a trace is looking."""
+    and neither forward-mode differentiation, a trace nor a function transform is looking (the
+    last refuse these operators, with a message of their own)."""
     return not torch.is_grad_enabled() and _fwd_ad._current_level < 0 \
-        and torch._C._get_tracing_state() is None
+        and torch._C._get_tracing_state() is None \
+        and torch._C._functorch.peek_interpreter_stack() is None
 
 
 def check_status(reset: bool = True) -> None:
