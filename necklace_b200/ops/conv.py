@@ -77,7 +77,7 @@ def _image_kernels(x, w, KH, KW, stride, pad) -> bool:
     bases; the data gradient is written for strides 1 and 2; 64 taps fit the argument block."""
     C, Cout = x.shape[-1], w.shape[0]
     return (x.is_cuda and C % 8 == 0 and Cout % 8 == 0 and stride <= 2 and KH * KW <= 64
-            and pad < 64 and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+            and 0 <= pad < 64 and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
             and x.is_contiguous() and w.is_contiguous() and w.shape[1] == KH * KW * C
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and x.numel() > 0)
 

@@ -1,0 +1,40 @@
+"""Calls that the convolution kernels on the image must leave to the gathered form, or answer as it
+does."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*s, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(*s, generator=g, device="cuda").bfloat16()
+
+
+def _close(got, want, mag, terms):
+    # bf16 rounding of the result and fp32 sums of `terms` products (each a few roundings)
+    bound = want.abs() * 2.0 ** -8 + mag * (terms + 16) * 2.0 ** -24 + 1e-30
+    err = (got.double() - want).abs()
+    assert bool((err <= bound).all()), float((err / bound).max())
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+def test_negative_padding_cuts_the_border_off(stride):
+    from necklace_b200.ops.conv import conv2d
+    x, w = _rand(2, 9, 10, 16).requires_grad_(True), _rand(24, 9 * 16, seed=1).requires_grad_(True)
+    y = conv2d(x, w, 3, 3, stride, -1)
+    inner = x.detach()[:, 1:-1, 1:-1].contiguous().requires_grad_(True)
+    w2 = w.detach().clone().requires_grad_(True)
+    ref = conv2d(inner, w2, 3, 3, stride, 0)
+    assert torch.allclose(y.float(), ref.float(), rtol=2.0 ** -7, atol=1e-2)
+    dy = _rand(*y.shape, seed=2)
+    y.backward(dy)
+    ref.backward(dy)
+    assert torch.allclose(w.grad.float(), w2.grad.float(), rtol=2.0 ** -7, atol=1e-2)
+    # taps are rounded to bf16 each
+    assert torch.allclose(x.grad[:, 1:-1, 1:-1].float(), inner.grad.float(), rtol=2.0 ** -6,
+                          atol=0.1)
+    border = x.grad.clone()
+    border[:, 1:-1, 1:-1] = 0
+    assert not border.any()
