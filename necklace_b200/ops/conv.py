@@ -159,11 +159,15 @@ class Conv2dFn(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        if ctx.image and x.is_contiguous() and \
-                not (x.data_ptr() | w.data_ptr() | dy2.data_ptr()) % 16:
-            dx = _conv_dgrad(dy2, w, ctx.xshape, *ctx.geom) if ctx.needs_input_grad[0] else None
-            dw = _deliver_grad(w, lambda out, acc: _conv_wgrad(x, dy2, w, *ctx.geom, out, acc))
-            return dx, dw, None, None, None, None
+        if ctx.image:
+            # (saved-tensor hooks may give back another layout)
+            xc, wc = x.contiguous(), w.contiguous()
+            if not (xc.data_ptr() | wc.data_ptr() | dy2.data_ptr()) % 16:
+                dx = _conv_dgrad(dy2, wc, ctx.xshape, *ctx.geom) if ctx.needs_input_grad[0] \
+                    else None
+                dw = _deliver_grad(w, lambda out, acc: _conv_wgrad(xc, dy2, wc, *ctx.geom, out,
+                                                                   acc))
+                return dx, dw, None, None, None, None
         dx = None
         if ctx.needs_input_grad[0]:
             d = gemm(dy2, w, b_mn=True)                       # [M, Kpad]

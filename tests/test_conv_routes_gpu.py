@@ -38,3 +38,18 @@ def test_negative_padding_cuts_the_border_off(stride):
     border = x.grad.clone()
     border[:, 1:-1, 1:-1] = 0
     assert not border.any()
+
+
+def test_saved_tensors_that_come_back_strided():
+    """Saved-tensor hooks may give back the same values in another layout."""
+    from necklace_b200.ops.conv import conv2d
+    grads = []
+    dy = _rand(2, 9, 10, 24, seed=2)
+    for unpack in (lambda t: t, lambda t: t.transpose(0, -1).contiguous().transpose(0, -1)):
+        x, w = _rand(2, 9, 10, 16).requires_grad_(True), _rand(24, 144, seed=1).requires_grad_(True)
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            y = conv2d(x, w, 3, 3, 1, 1)
+        y.backward(dy)
+        grads.append((x.grad, w.grad))
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
