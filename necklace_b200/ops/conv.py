@@ -115,7 +115,8 @@ def _conv_wgrad(x, dy, w, KH, KW, stride, pad, out, acc):
     _lib.count_launch(2)
     if out is None or direct:
         return dst
-    return out.add_(dst) if acc else out.copy_(dst)
+    dw = ws.sum(0).view_as(w)            # in fp32, as long as the destination holds that
+    return out.copy_(out.float() + dw if acc else dw)
 
 
 class Conv2dFn(torch.autograd.Function):

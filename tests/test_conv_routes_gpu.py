@@ -53,3 +53,27 @@ def test_saved_tensors_that_come_back_strided():
         grads.append((x.grad, w.grad))
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_weight_gradient_into_a_buffer_of_another_kind(dtype):
+    """A gradient buffer in fp32 gets the fp32 sums; one that is not aligned is rounded once."""
+    from necklace_b200.ops.conv import conv2d
+    x, w, dy = _rand(3, 9, 10, 16), _rand(24, 144, seed=1), _rand(3, 9, 10, 24, seed=2)
+    w = torch.nn.Parameter(w)
+    flat = torch.zeros(24 * 144 + 1, dtype=dtype, device="cuda")
+    w._nkb_grad, w._nkb_grad_has = flat[1:].view(24, 144), False
+    ref = []
+    for d in (dy, _rand(3, 9, 10, 24, seed=3)):
+        conv2d(x, w, 3, 3, 1, 1).backward(d)
+        for v in (x.double(), x.double().abs()):
+            wr = torch.zeros(24, 16, 3, 3, dtype=torch.float64, device="cuda", requires_grad=True)
+            y = F.conv2d(v.permute(0, 3, 1, 2), wr, padding=1)
+            y.backward((d.double() if v.min() < 0 else d.double().abs()).permute(0, 3, 1, 2))
+            ref.append(wr.grad.permute(0, 2, 3, 1).reshape(24, 144))
+    want, mag = ref[0] + ref[2], ref[1] + ref[3]
+    # fp32 sums of 270 products twice; bf16: the first sum is rounded too
+    bound = mag * 300 * 2.0 ** -24 * 4
+    if dtype == torch.bfloat16:
+        bound = bound + (ref[0].abs() + want.abs()) * 2.0 ** -8
+    assert bool(((w._nkb_grad.double() - want).abs() <= bound).all())
