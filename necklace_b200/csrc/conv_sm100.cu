@@ -761,9 +761,14 @@ extern "C" int nkb_conv_wgrad(const void* x, const void* dy, void* dw, float* ws
   CUtensorMap a, b;
   int rc = tmap_pixels(&a, dy, Cout, g.W, g.H, N, Cout, (long long)g.W * Cout,
                        (long long)g.H * g.W * Cout, g.bw, g.bh, g.bn, 1);
+  // Positions outside the output read dy as zero, but x at their taps may lie inside the image.
+  // Pixels behind the last window (a remainder of the stride) are cut off the map: no window has
+  // them, so an Inf or NaN there must not meet those zeros.  (Where a window has such a pixel,
+  // its channel's gradient holds an Inf or NaN in any case.)
+  const int Wu = (g.W - 1) * stride + KW - pad, Hu = (g.H - 1) * stride + KH - pad;
   if (!rc)
-    rc = tmap_pixels(&b, x, C, W, H, N, C, (long long)W * C, (long long)H * W * C, g.bw, g.bh,
-                     g.bn, stride);
+    rc = tmap_pixels(&b, x, C, Wu < 1 ? 1 : Wu < W ? Wu : W, Hu < 1 ? 1 : Hu < H ? Hu : H, N, C,
+                     (long long)W * C, (long long)H * W * C, g.bw, g.bh, g.bn, stride);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int units = g.tiles_m * g.tiles_n * g.split;

@@ -77,3 +77,20 @@ def test_weight_gradient_into_a_buffer_of_another_kind(dtype):
     if dtype == torch.bfloat16:
         bound = bound + (ref[0].abs() + want.abs()) * 2.0 ** -8
     assert bool(((w._nkb_grad.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("k,pad", [(1, 0), (3, 0), (2, 0)])
+def test_pixels_that_no_window_has(k, pad):
+    """The last row and column of an image that the stride does not divide."""
+    from necklace_b200.ops.conv import _conv_wgrad
+    N, H, W, ci, co = 3, 8, 10, 16, 24
+    if k == 2:
+        H, W = 9, 11
+    x, w = _rand(N, H, W, ci), _rand(co, k * k * ci, seed=1)
+    Ho, Wo = (H - k) // 2 + 1, (W - k) // 2 + 1
+    dy = _rand(N, Ho, Wo, co, seed=2)
+    clean = _conv_wgrad(x, dy.reshape(-1, co), w, k, k, 2, pad, None, False)
+    x[:, (Ho - 1) * 2 + k:] = float("inf")
+    x[:, :, (Wo - 1) * 2 + k:] = float("nan")
+    assert not x.isfinite().all()
+    assert torch.equal(clean, _conv_wgrad(x, dy.reshape(-1, co), w, k, k, 2, pad, None, False))
