@@ -21,7 +21,7 @@ from torch.nn.modules.module import _has_any_global_hook
 
 from .. import _lib
 from ._common import on_gpu, plain_call, ptr, status_ptr, stream_scratch
-from .gemm import _deliver_grad, gemm
+from .gemm import _deliver_grad, _deliver_nothing, gemm
 
 
 def _out_hw(H, W, KH, KW, stride, pad):
@@ -188,13 +188,14 @@ class Conv1x1SplitFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w):
         ctx.save_for_backward(x, w)
+        ctx.set_materialize_grads(False)
         return x.view_as(x), gemm(x.reshape(-1, x.shape[-1]), w).view(*x.shape[:-1], w.shape[0])
 
     @staticmethod
     def backward(ctx, dres, dy):
         x, w = ctx.saved_tensors
         if dy is None:      # only the residual path was used
-            return dres, None
+            return dres, _deliver_nothing(w)
         a, dy2 = x.reshape(-1, x.shape[-1]), dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()

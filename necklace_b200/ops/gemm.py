@@ -177,6 +177,12 @@ def _deliver_grad(p: torch.Tensor, compute):
     return None
 
 
+def _deliver_nothing(p: torch.Tensor):
+    """The gradient of a parameter whose output nobody used: zeros, delivered like any other."""
+    return _deliver_grad(p, lambda out, acc: torch.zeros_like(p) if out is None
+                         else (out if acc else out.zero_()))
+
+
 class LinearFn(torch.autograd.Function):
     """``y = x @ w^T + b (+ residual)`` with ``w`` stored ``[out, in]``."""
 

@@ -6,7 +6,7 @@ import torch.nn as nn
 
 from .. import _lib
 from ._common import on_gpu, plain_call, ptr
-from .gemm import _deliver_grad, colsum_scratch
+from .gemm import _deliver_grad, _deliver_nothing, colsum_scratch
 
 
 def norm_fwd(x2: torch.Tensor, w: torch.Tensor, b: torch.Tensor | None, eps: float, rms: bool):
@@ -166,12 +166,15 @@ class NormSplitFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b, eps, rms):
         y = NormFn.forward(ctx, x, w, b, eps, rms)
+        ctx.set_materialize_grads(False)
         return x.view_as(x), y
 
     @staticmethod
     def backward(ctx, dres, dy):
         if dy is None:  # only the residual branch was used
-            return dres, None, None, None, None
+            w, b = ctx.saved_tensors[1], ctx.b_ref
+            db = _deliver_nothing(b) if b is not None else None
+            return dres, _deliver_nothing(w), db, None, None
         return NormFn.backward(ctx, dy, dres)
 
 

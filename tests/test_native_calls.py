@@ -91,3 +91,17 @@ def test_the_node_stays_where_something_looks():
     with torch.inference_mode():
         assert plain_call()
         assert linear(torch.ones(2, 8), torch.ones(4, 8)).shape == (2, 4)
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_forward_by_itself_adds_the_residual(device):
+    from necklace_b200.ops import linear
+    g = torch.Generator().manual_seed(5)
+    x, w, res = (torch.randn(*s, generator=g).bfloat16().to(device)
+                 for s in ((2, 9, 128), (256, 128), (2, 9, 256)))
+    with torch.no_grad():
+        y = linear(x, w, None, res)
+        bare = linear(x, w)
+    assert torch.equal(y, linear(x, w, None, res).detach())
+    assert float((y.float() - bare.float() - res.float()).abs().max()) < 0.3
+    assert float(res.float().abs().max()) > 2
