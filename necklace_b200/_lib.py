@@ -108,6 +108,26 @@ def _try_build() -> None:
     _build.build(debug_bounds=DEBUG_BOUNDS)
 
 
+_BOUNDS_TUS = ("conv", "convimg", "loss", "optim", "comm")
+
+
+def debug_bounds_seen() -> set:
+    """Debug build only: the translation units in which an index check has been evaluated since the
+    last call."""
+    lib = load()
+    import torch
+    torch.cuda.synchronize()
+    seen = set()
+    for tu in _BOUNDS_TUS:
+        fn = getattr(lib, f"nkb_debug_bounds_seen_{tu}")
+        flag = C.c_int()
+        fn.argtypes, fn.restype = [C.c_void_p], i32
+        check(fn(C.addressof(flag)), f"nkb_debug_bounds_seen_{tu}")
+        if flag.value:
+            seen.add(tu)
+    return seen
+
+
 def debug_bounds(raise_on_error: bool = True) -> dict:
     """Debug build only: read and clear the index-check records of every translation unit.
     Returns ``{tu: (count, source line, first bad index)}`` for units with failures and raises
@@ -116,7 +136,7 @@ def debug_bounds(raise_on_error: bool = True) -> dict:
     import torch
     torch.cuda.synchronize()
     bad = {}
-    for tu in ("conv", "loss", "optim", "comm"):
+    for tu in _BOUNDS_TUS:
         fn = getattr(lib, f"nkb_debug_bounds_{tu}", None)
         if fn is None:
             continue

@@ -99,14 +99,16 @@ im2col_tile_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
                           ((long long)n * g.H + (in ? h : 0)) * WC;
     for (int e = threadIdx.x; e < row_elems; e += 256) {
       const int w = e0 + e;
-      rows[kh * row_elems + e] = in && w >= 0 && w < WC ? src[w] : (uint16_t)0;
+      const bool ok = in && w >= 0 && w < WC &&
+                      NKB_IN_BOUNDS(((long long)n * g.H + h) * WC + w, (long long)g.N * g.H * WC);
+      rows[kh * row_elems + e] = ok ? src[w] : (uint16_t)0;
     }
   }
   if (threadIdx.x == 0) rows[zero] = 0;
   __syncthreads();
   const int px = min(tw, g.Wo - wo0), chunks = g.Kpad >> 3, sc = g.stride * g.C;
-  uint4* out = reinterpret_cast<uint4*>(col) +
-               (((long long)n * g.Ho + ho) * g.Wo + wo0) * chunks;
+  const long long out0 = (((long long)n * g.Ho + ho) * g.Wo + wo0) * chunks;
+  uint4* out = reinterpret_cast<uint4*>(col) + out0;
   for (int i = threadIdx.x; i < px * chunks; i += 256) {
     const int p = i / chunks, k = (i - p * chunks) * 8;
     const uint4 t = *reinterpret_cast<const uint4*>(table + k);
@@ -119,7 +121,8 @@ im2col_tile_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
       const uint32_t hi = rows[b == zero ? zero : b + p * sc];
       o[j] = lo | hi << 16;
     }
-    out[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    if (NKB_IN_BOUNDS(out0 + i, (long long)g.N * g.Ho * g.Wo * chunks))
+      out[i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 

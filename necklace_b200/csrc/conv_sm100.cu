@@ -403,7 +403,8 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int row = i * 4 + (lane >> 3);
-              if (row < rows_valid && c + ch * 4 < g.cin)
+              if (row < rows_valid && c + ch * 4 < g.cin &&
+                  NKB_IN_BOUNDS(dst - g.ws + row * ld + ch * 4 + 3, g.split * g.cout * ld))
                 *reinterpret_cast<uint4*>(dst + row * ld + ch * 4) =
                     *reinterpret_cast<const uint4*>(stg + row * 128 + ((ch ^ (row & 7)) << 4));
             }
@@ -782,3 +783,4 @@ extern "C" int nkb_conv_wgrad(const void* x, const void* dy, void* dw, float* ws
 }
 
 NKB_DEFINE_WAIT_SETTER(conv)
+NKB_DEFINE_BOUNDS_GETTER(convimg)

@@ -62,7 +62,9 @@ inline int allow_smem(K kern, int bytes, bool (&done)[64]) {
 // compiles away.
 #ifdef NKB_DEBUG_BOUNDS
 static __device__ int g_nkb_bounds_rec[4];  // count, line, index low word, index high word
+static __device__ int g_nkb_bounds_seen;    // whether any check was evaluated
 __device__ __forceinline__ bool nkb_in_bounds(long long i, long long n, int line) {
+  g_nkb_bounds_seen = 1;
   if (i >= 0 && i < n) return true;
   if (atomicAdd(&g_nkb_bounds_rec[0], 1) == 0) {
     g_nkb_bounds_rec[1] = line;
@@ -77,6 +79,12 @@ __device__ __forceinline__ bool nkb_in_bounds(long long i, long long n, int line
     int z[4] = {0, 0, 0, 0};                                                               \
     cudaError_t e = cudaMemcpyFromSymbol(out4, nkb::g_nkb_bounds_rec, sizeof(z));          \
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(nkb::g_nkb_bounds_rec, z, sizeof(z));     \
+    return (int)e;                                                                         \
+  }                                                                                        \
+  extern "C" int nkb_debug_bounds_seen_##tu(int* out) {                                    \
+    int z = 0;                                                                             \
+    cudaError_t e = cudaMemcpyFromSymbol(out, nkb::g_nkb_bounds_seen, sizeof(z));          \
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(nkb::g_nkb_bounds_seen, &z, sizeof(z));   \
     return (int)e;                                                                         \
   }
 #else
