@@ -30,7 +30,7 @@ vp, i32, i64, f32 = C.c_void_p, C.c_int, C.c_longlong, C.c_float
 _SIGS = {
     "nkb_gemm_bf16": [vp, i64, i32, vp, i64, i32, vp, i64, i32, i32, i32, i32, i32, f32, vp, vp,
                       i64, i32, vp, i64, vp, vp, i32, i32, i32, i32, vp, vp],
-    "nkb_gemm_slices": [i32, i32, i32, i32, i32, i64, i32],
+    "nkb_gemm_slices": [i32, i32, i32, i64, i32],
     "nkb_gemm_bf16_ws": [vp, i64, i32, vp, i64, i32, vp, i64, i32, i32, i32, i32, i32, f32, vp,
                          vp, i64, i32, vp, i64, vp, vp, i32, i32, i32, i32, vp, vp, i32, vp],
     "nkb_capture_id": [vp],

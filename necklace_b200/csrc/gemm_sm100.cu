@@ -1565,61 +1565,58 @@ struct TilePlan {
   int BN = 256;
   bool pair = false;
   int slices = 1;
+  double us = 1e30;  // estimated
 };
 
 // Tile choice.  bn_hint: 0 = automatic, 128 / 256 = single-CTA tile of that width,
 // 512 = CTA-pair 256 x 256 tile; and split-K when the output has too few tiles to occupy the
 // machine and K is long.
 //
-// Time in us: launch, prologue and last epilogue; the K steps of 64 of every round (0.27 for all
-// three kinds: the tensor pipe bounds the 256-wide tiles, the operand traffic of 64 B/clk
-// per SM the 128 x 128 one); the part of a further round's epilogue that its main loop does not
-// hide.  With more than about 110 SMs at work the 48 KB that a 128 x 256 tile loads per step meet
-// the rate of L2, more so when both operands are MN-major (4096 x 1024 x 8192 weight gradient:
-// 56.2 us against 51.3 with pairs, which load a third less).  A split adds the reduction's launch
-// and its fp32 partial sums, written and read at about 8 TB/s as most of them stay in L2.
-// Fitted to graphs of equal GEMMs, M = 333 .. 4096, N = 768 .. 5504, K = 768 .. 8192:
-// 2313 x 768 x 768 takes 8.6 / 9.9 / 11.4 us, 4096 x 4096 x 1024 42 / 30.6 / 29.6 us (128 x 128,
-// 128 x 256, pair).  Weighing rounds alone (0.68 : 0.88 : 1) took 26.8 us for 2313 x 1024 x 4096
-// (pair; 25.2 with 128 x 256) and 30.7 us for 1024 x 1024 x 8192 (128 x 128 in 2 slices; 24.3 with
-// pairs in 4).  With at most 8 slices a 64 x 64 weight gradient over 802816 pixels ran on
-// 8 SMs: the 49 split GEMMs of a ResNet-50 step took 9.0 ms (its 1x1 layers 2.0 ms now).
-static TilePlan gemm_plan(int M, int N, int K, bool both_mn, int bn_hint, bool can_split,
-                          bool pairs) {
-  TilePlan best_plan;
+// Time in us: launch, prologue and last epilogue (`fixed`); the K steps of 64 of every round; the
+// part of a further round's epilogue that its main loop does not hide (`extra`).  A step takes the
+// MMA's time while few SMs are at work (`step`), and with all of them what the operands' way from
+// L2 allows (`full`, in proportion to the SMs at work): 32, 48 and 64 KB per tile, so the pair,
+// with half of the tiles, is the one that large operands want.  A split adds the reduction's
+// launch and its fp32 partial sums, written and read at about 8 TB/s as most of them stay in L2.
+// Fitted to 2000 times of GEMMs of all three kinds of tile (M 16 .. 16384, N 64 .. 8192, K 64 ..
+// 20480, each operand order); the choice is 0.6 % above the best kind on average, 5 % at the 95th
+// percentile.  One step time for all kinds (0.27 us, and a penalty of the 128 x 256 tile above 110
+// SMs) was 2.0 and 16 %: 2943 x 952 x 9208 took 86.4 us on 128 x 256 tiles (62.4 with pairs),
+// 896 x 6744 x 6640 114 (83).  Weighing rounds alone (0.68 : 0.88 : 1) was 2.8 and 27 %:
+// 2313 x 1024 x 4096 took 26.8 us (pair; 25.2 with 128 x 256).  With at most 8 slices a 64 x 64
+// weight gradient over 802816 pixels ran on 8 SMs: the 49 split GEMMs of a ResNet-50 step took
+// 9.0 ms (its 1x1 layers 2.0 ms now).
+static TilePlan gemm_plan(int M, int N, int K, int bn_hint, bool can_split, bool pairs) {
+  TilePlan best;
   const int sms = num_sms();
   const long long mblk = (M + BM - 1) / BM;
   const int kb = (K + BK - 1) / BK;
-  double best = 1e30;
-  const double mn = both_mn ? 1.2 : 1.0;
   auto consider = [&](int kind_bn, bool kind_pair, long long tiles, int slots, double fixed,
-                      double extra) {
+                      double step, double full, double extra) {
     const int most = can_split && tiles * 10 <= slots * 7 ? 64 : 1;
     for (int S = 1; S <= most && (S == 1 || S <= slots / tiles); ++S) {
       if (S > 1 && ((K / BK) / S < 8 || (long long)S * M * N > SPLITK_MAX_FLOATS)) break;
       const long long r = (tiles * S + slots - 1) / slots;
-      double step = 0.27;
-      if (kind_bn == 256 && !kind_pair) {
-        const double busy = (double)(tiles * S) / r;
-        step *= mn * (busy > 110.0 ? busy / 110.0 : 1.0);
-      }
-      const double c = fixed + r * (step * ((kb + S - 1) / S)) + (r - 1) * extra +
-                       (S > 1 ? 2.5 + (double)S * M * N * 1e-6 : 0.0);
-      if (c < best) {
-        best = c;
-        best_plan.BN = kind_bn;
-        best_plan.pair = kind_pair;
-        best_plan.slices = S;
+      const double loaded = full * (double)(tiles * S) / (double)(r * slots);
+      const double us = fixed + r * ((step > loaded ? step : loaded) * ((kb + S - 1) / S)) +
+                        (r - 1) * extra + (S > 1 ? 1.5 + (double)S * M * N * 1.15e-6 : 0.0);
+      if (us < best.us) {
+        best.BN = kind_bn;
+        best.pair = kind_pair;
+        best.slices = S;
+        best.us = us;
       }
     }
   };
   const bool any = bn_hint != 128 && bn_hint != 256 && bn_hint != 512;
-  if (bn_hint == 128 || any) consider(128, false, mblk * ((N + 127) / 128), sms, 4.6, 1.0);
+  if (bn_hint == 128 || any)
+    consider(128, false, mblk * ((N + 127) / 128), sms, 4.7, 0.29, 0.32, 0.6);
   if (bn_hint == 256 || (any && N > 128))
-    consider(256, false, mblk * ((N + 255) / 256), sms, 6.1, 1.8);
+    consider(256, false, mblk * ((N + 255) / 256), sms, 6.0, 0.38, 0.45, 1.4);
   if (bn_hint == 512 || (any && pairs && M > 128 && N > 128))
-    consider(256, true, ((M + 255) / 256) * (long long)((N + 255) / 256), sms / 2, 7.8, 1.2);
-  return best_plan;
+    consider(256, true, ((M + 255) / 256) * (long long)((N + 255) / 256), sms / 2, 7.8, 0.31, 0.38,
+             2.0);
+  return best;
 }
 
 // K can be cut into slices when nothing but a sum and a factor follows: the slices' fp32 sums
@@ -1642,7 +1639,7 @@ static int gemm_run(GemmArgs g, const void* A, long long lda, int a_mn, const vo
         (reinterpret_cast<uintptr_t>(ws) & 15))
       return -3;
   }
-  const TilePlan plan = gemm_plan(M, N, K, a_mn && b_mn, bn_hint, split,
+  const TilePlan plan = gemm_plan(M, N, K, bn_hint, split,
                                   g_pair_enabled && !(g.ag_ctas && (g.ag_rows_per_rank % 256)));
   if (split && plan.slices != slices) return -3;
   const int BN = plan.BN;
@@ -1695,10 +1692,9 @@ extern "C" int nkb_gemm_bf16(const void* A, long long lda, int a_mn, const void*
                           ready_target, max_ctas, bn_hint, alpha_dev, nullptr, 1, stream);
 }
 
-extern "C" int nkb_gemm_slices(int M, int N, int K, int a_mn, int b_mn, long long ldc,
-                               int bn_hint) {
+extern "C" int nkb_gemm_slices(int M, int N, int K, long long ldc, int bn_hint) {
   if (M <= 0 || N <= 0 || !splittable(N, K, ldc)) return 1;
-  return gemm_plan(M, N, K, a_mn && b_mn, bn_hint, true, g_pair_enabled).slices;
+  return gemm_plan(M, N, K, bn_hint, true, g_pair_enabled).slices;
 }
 
 extern "C" int nkb_gemm_bf16_ws(const void* A, long long lda, int a_mn, const void* B,

@@ -30,7 +30,7 @@ int nkb_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long lo
 // activation cuts K, and the same GEMM with that number and the fp32 [slices][M][N] workspace of
 // its partial sums.  The workspace is the call's own: no other work may use it before both of
 // the call's kernels have run.
-int nkb_gemm_slices(int M, int N, int K, int a_mn, int b_mn, long long ldc, int bn_hint);
+int nkb_gemm_slices(int M, int N, int K, long long ldc, int bn_hint);
 int nkb_gemm_bf16_ws(const void* A, long long lda, int a_mn, const void* B, long long ldb,
                      int b_mn, void* C, long long ldc, int c_fp32, int accumulate, int M, int N,
                      int K, float alpha, const void* bias, const void* res, long long ldres,

@@ -93,7 +93,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     slices, ws = 1, None
     if K >= 2048 and epi == EPI_NONE and bias is None and res is None \
             and out.data_ptr() % (16 if fp32 else 8) == 0:
-        slices = _lib.value("nkb_gemm_slices", M, N, K, a_mn, b_mn, out.stride(0), bn)
+        slices = _lib.value("nkb_gemm_slices", M, N, K, out.stride(0), bn)
         if slices > 1:
             # the partial sums' memory belongs to this call: the allocator orders its reuse on
             # the stream (also while a graph is captured), and no other thread gets it meanwhile

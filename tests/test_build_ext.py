@@ -45,7 +45,7 @@ def test_built_when_missing(tmp_path):
             if not f.startswith("_nkpy") and not f.endswith(("_dbg.so", ".pyc")):
                 os.symlink(os.path.join(d, f), os.path.join(out, f))
     code = ("from necklace_b200 import _lib; _lib.load(); assert _lib._fast; "
-            "assert _lib.value('nkb_gemm_slices', 64, 64, 64, 0, 0, 64, 0) == 1")
+            "assert _lib.value('nkb_gemm_slices', 64, 64, 64, 64, 0) == 1")
     r = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True,
                        env=dict(os.environ, PYTHONPATH=str(tmp_path)), timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]

@@ -11,13 +11,13 @@ def test_slices_of_a_gemm():
     if not _lib.available():
         pytest.skip("native library not built")
     n = lambda *a: _lib.value("nkb_gemm_slices", *a)  # noqa: E731
-    assert n(64, 64, 50000, 1, 1, 64, 0) > 8
-    assert n(64, 64, 2047, 1, 1, 64, 0) == 1          # K too short
-    assert n(64, 66, 50000, 1, 1, 68, 0) == 1         # columns not in fours
-    assert n(64, 64, 50000, 1, 1, 66, 0) == 1
-    assert n(8192, 4096, 4096, 0, 0, 4096, 0) == 1    # fills the machine
-    assert n(0, 64, 4096, 0, 0, 64, 0) == 1
-    assert n(4096, 4096, 1 << 20, 0, 0, 4096, 0) * 4096 * 4096 <= 32 << 20
+    assert n(64, 64, 50000, 64, 0) > 8
+    assert n(64, 64, 2047, 64, 0) == 1          # K too short
+    assert n(64, 66, 50000, 68, 0) == 1         # columns not in fours
+    assert n(64, 64, 50000, 66, 0) == 1
+    assert n(8192, 4096, 4096, 4096, 0) == 1    # fills the machine
+    assert n(0, 64, 4096, 64, 0) == 1
+    assert n(4096, 4096, 1 << 20, 4096, 0) * 4096 * 4096 <= 32 << 20
 
 
 def _gemms(seed):
