@@ -84,6 +84,7 @@ _SIGS = {
     "nkb_col2im_nhwc": [vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp],
     "nkb_conv_fwd": [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp],
     "nkb_conv_dgrad": [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp],
+    "nkb_conv_route": [i32, i32, i32, i32, i32, i32, i32, i32, i32],
     "nkb_conv_wgrad_split": [i32, i32, i32, i32, i32, i32, i32, i32, i32],
     "nkb_conv_wgrad": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp,
                        vp],

@@ -39,6 +39,7 @@
 namespace nkb {
 
 int num_sms();
+double gemm_time_us(int M, int N, int K);
 int make_tmap_bf16_nd(CUtensorMap* out, const void* base, int rank, const long long* dims,
                       const long long* strides, const int* box, const int* estr);
 
@@ -780,6 +781,74 @@ extern "C" int nkb_conv_wgrad(const void* x, const void* dy, void* dw, float* ws
   conv_dw_reduce_kernel<<<(unsigned)((n4 + 63) / 64), 256, 0, s>>>(
       ws, g.split, n4, static_cast<__nv_bfloat16*>(dw), accumulate);
   return (int)cudaGetLastError();
+}
+
+// Which of a layer's three products are quicker on the image: bit 0 forward and weight gradient
+// (which use one gathered matrix otherwise), bit 1 data gradient; -3 as above.
+//
+// The image kernels read no gathered matrix, but a tile runs through all taps and channels one
+// after the other and K is not split, so a layer with few positions and a long contraction leaves
+// most SMs idle, where the GEMM of the gathered form has slices: 512 -> 512, 3x3, stride 2, 8 images
+// of 14 x 14 take 23 + 15 + 39 us on the image (forward, weight and data gradient; the last in
+// four launches, one per class of positions), 11 + 9 + 12 us gathered.  With few channels a step
+// of 64 is mostly empty and a box has rows of 16 bytes: 8 -> 64, 3x3, 128 images of 56 x 56 take
+// 231 + 125 + 206 us on the image, 95 + 35 + 78 gathered.  With 64 channels and more and pixels enough the
+// image wins: 64 -> 64, 3x3, 64 images of 28 x 28, 13 + 18 + 19 against 44 + 15 + 49 us.
+// Times in us fitted to 502 layers (C, Cout 8 .. 1024, windows 1 .. 7, strides 1 and 2, 1 .. 256
+// images): choosing by them is 0.3 % (forward and weight gradient) and 2 % (data gradient) above
+// the quicker form on average; the image for all was 23 and 28 %.  The gathered form has another
+// kernel to launch, which costs the host about 4 us: it must win by more.
+extern "C" int nkb_conv_route(int N, int H, int W, int C, int Cout, int KH, int KW, int stride,
+                              int pad) {
+  if (!conv_ok(N, H, W, C, Cout, KH, KW, stride, pad) || stride > 2) return -3;
+  const int Ho = (H + 2 * pad - KH) / stride + 1, Wo = (W + 2 * pad - KW) / stride + 1;
+  const int sms = num_sms(), T = KH * KW;
+  const long long P = (long long)N * Ho * Wo, K = (long long)T * C;
+  if (P > (1 << 30) || K > (1 << 30)) return 3;
+  auto boxes = [&](int w, int h, int s) {
+    int bw, bh, bn;
+    pick_box(w, h, N, s, bw, bh, bn);
+    return ((w + bw - 1) / bw) * ((h + bh - 1) / bh) * ((N + bn - 1) / bn);
+  };
+  auto rounds = [&](int tiles_m, int cols, int& BN) {
+    BN = pick_bn(tiles_m, cols);
+    return (int)(((long long)tiles_m * ((cols + BN - 1) / BN) + sms - 1) / sms);
+  };
+  // what a box of rows narrower than 128 bytes costs more, when there are many of them
+  auto narrow = [](int channels, double us) { return channels < 64 ? us / channels : 0.0; };
+  int BN;
+  int r = rounds(boxes(Wo, Ho, stride), Cout, BN);
+  double step = (0.284 + (r > 1 ? narrow(C, 3.5) : 0.0)) * (BN == 256 ? 1.25 : 1.0);
+  double image = 3.1 + r * (T * ((C + 63) / 64) * step + 0.9);
+  ConvArgs g{};
+  const int split = wgrad_plan(g, N, H, W, C, Cout, KH, KW, stride, pad, BN);
+  const int units = g.tiles_m * g.tiles_n * split;
+  const int per_unit = (g.nbw * g.nbh * g.nbn + split - 1) / split;
+  step = 0.56 * g.rows / 64 * (BN == 256 ? 1.0 : 0.37) + narrow(C, 1.6);
+  image += 5.6 + (units + sms - 1) / sms * (per_unit * step + 1.65) +
+           (double)split * Cout * K * 1.4e-6;
+  const double mb = P * K * 2e-6;  // the gathered matrix, MB
+  const double gather = 1.2 + mb / 1.95;
+  const double gathered = gather * (mb > 2147.0 ? 2 : 1) +  // (it is not kept then)
+                          gemm_time_us((int)P, Cout, (int)K) +
+                          0.93 * gemm_time_us(Cout, (int)K, (int)P);
+  double image_dx = 0.0;
+  for (int ph = 0; ph < stride; ++ph)
+    for (int pw = 0; pw < stride; ++pw) {
+      const int Hc = (H - ph + stride - 1) / stride, Wc = (W - pw + stride - 1) / stride;
+      int taps = 0;
+      for (int t = 0; t < T; ++t)
+        taps += (ph + pad - t / KW) % stride == 0 && (pw + pad - t % KW) % stride == 0;
+      if (Hc <= 0 || Wc <= 0 || !taps) continue;
+      r = rounds(boxes(Wc, Hc, 1), C, BN);
+      // a tap's MMAs, or its way out of the accumulator
+      const double mma = (Cout + 63) / 64 *
+                         (0.385 * (BN == 256 ? 1.1 : 1.0) + (r > 1 ? narrow(Cout, 2.0) : 0.0));
+      const double drain = 0.6 * BN / 128;
+      image_dx += 3.2 + r * (taps * (mma > drain ? mma : drain) + 1.6);
+    }
+  const double gathered_dx = 4.9 + mb / 1.5 + gemm_time_us((int)P, (int)K, Cout);
+  return (image <= gathered + 4.0 ? 1 : 0) | (image_dx <= gathered_dx + 3.0 ? 2 : 0);
 }
 
 NKB_DEFINE_WAIT_SETTER(conv)

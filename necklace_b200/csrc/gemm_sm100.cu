@@ -1625,6 +1625,13 @@ static bool splittable(int N, int K, long long ldc) {
   return g_splitk_enabled && N % 4 == 0 && ldc % 4 == 0 && K >= 2048;
 }
 
+namespace nkb {
+// Estimated time of a plain GEMM with contiguous rows.
+double gemm_time_us(int M, int N, int K) {
+  return gemm_plan(M, N, K, 0, splittable(N, K, N), g_pair_enabled).us;
+}
+}  // namespace nkb
+
 // slices > 1: the number that nkb_gemm_slices gave for these sizes, ws holds that many fp32
 // matrices [M, N].
 static int gemm_run(GemmArgs g, const void* A, long long lda, int a_mn, const void* B,

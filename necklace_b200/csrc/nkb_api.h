@@ -98,12 +98,15 @@ int nkb_col2im_nhwc(const void* dcol, void* dx, int N, int H, int W, int C, int 
                     int stride, int pad, int Kpad, void* stream);
 // Convolutions on the image itself (conv_sm100.cu): w / dw [Cout, KH*KW*C], C and Cout multiples
 // of 8, 16-byte aligned bases, stride <= 8 (data gradient: 1 or 2); -3 for anything else.
+// nkb_conv_route: which products are quicker there than gathered (bit 0 forward and weight gradient,
+// bit 1 data gradient).
 // nkb_conv_wgrad: ws holds nkb_conv_wgrad_split() fp32 matrices of dw's shape; dw is written or
 // added to.
 int nkb_conv_fwd(const void* x, const void* w, void* y, int N, int H, int W, int C, int Cout,
                  int KH, int KW, int stride, int pad, int* status, void* stream);
 int nkb_conv_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int C, int Cout,
                    int KH, int KW, int stride, int pad, int* status, void* stream);
+int nkb_conv_route(int N, int H, int W, int C, int Cout, int KH, int KW, int stride, int pad);
 int nkb_conv_wgrad_split(int N, int H, int W, int C, int Cout, int KH, int KW, int stride,
                          int pad);
 int nkb_conv_wgrad(const void* x, const void* dy, void* dw, float* ws, int split, int N, int H,

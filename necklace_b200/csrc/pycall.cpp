@@ -102,7 +102,8 @@ PyMethodDef methods[] = {
     ENTRY(nkb_bn_fwd),           ENTRY(nkb_bn_apply),         ENTRY(nkb_bn_bwd),
     ENTRY(nkb_bn_eval),          ENTRY(nkb_maxpool3x3s2_fwd), ENTRY(nkb_maxpool3x3s2_bwd),
     ENTRY(nkb_avgpool_fwd),      ENTRY(nkb_avgpool_bwd),      ENTRY(nkb_gemm_slices),
-    ENTRY(nkb_gemm_bf16_ws),     ENTRY(nkb_capture_id),       {nullptr, nullptr, 0, nullptr}};
+    ENTRY(nkb_gemm_bf16_ws),     ENTRY(nkb_capture_id),       ENTRY(nkb_conv_route),
+    {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_nkpy", nullptr, -1, methods,
                       nullptr, nullptr, nullptr, nullptr};

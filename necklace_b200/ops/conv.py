@@ -14,6 +14,8 @@ data-parallel configuration.
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
@@ -72,7 +74,7 @@ def col2im(dcol: torch.Tensor, shape, KH: int, KW: int, stride: int, pad: int) -
 
 
 def _image_kernels(x, w, KH, KW, stride, pad) -> bool:
-    """Whether the kernels that read the image itself take this layer (else: gather).  The
+    """Whether the kernels that read the image itself can take this layer (else: gather).  The
     tensor maps want channel counts that are multiples of 8 (16-byte strides) and aligned
     bases; the data gradient is written for strides 1 and 2; 64 taps fit the argument block."""
     C, Cout = x.shape[-1], w.shape[0]
@@ -80,6 +82,18 @@ def _image_kernels(x, w, KH, KW, stride, pad) -> bool:
             and 0 <= pad < 64 and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
             and x.is_contiguous() and w.is_contiguous() and w.shape[1] == KH * KW * C
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and x.numel() > 0)
+
+
+@functools.lru_cache(maxsize=4096)
+def _route(N, H, W, C, Cout, KH, KW, stride, pad) -> int:
+    """Which of a layer's products are quicker on the image than gathered (a matter of its sizes
+    alone): bit 0 forward and weight gradient, bit 1 data gradient."""
+    return max(_lib.value("nkb_conv_route", N, H, W, C, Cout, KH, KW, stride, pad), 0)
+
+
+def _image_route(x, w, KH, KW, stride, pad) -> int:
+    return _route(*x.shape, w.shape[0], KH, KW, stride, pad) \
+        if _image_kernels(x, w, KH, KW, stride, pad) else 0
 
 
 def _conv_fwd(x, w, KH, KW, stride, pad):
@@ -130,8 +144,8 @@ class Conv2dFn(torch.autograd.Function):
         ctx.xshape = tuple(x.shape)
         direct = KH == 1 and KW == 1 and stride == 1 and pad == 0 and C % 8 == 0
         ctx.direct = direct
-        ctx.image = not direct and _image_kernels(x, w, KH, KW, stride, pad)
-        if ctx.image:
+        ctx.route = 0 if direct else _image_route(x, w, KH, KW, stride, pad)
+        if ctx.route & 1:
             ctx.keep_col = False
             ctx.save_for_backward(x, w)
             return _conv_fwd(x, w, KH, KW, stride, pad)
@@ -160,19 +174,21 @@ class Conv2dFn(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        if ctx.image:
-            # (saved-tensor hooks may give back another layout)
-            xc, wc = x.contiguous(), w.contiguous()
-            if not (xc.data_ptr() | wc.data_ptr() | dy2.data_ptr()) % 16:
-                dx = _conv_dgrad(dy2, wc, ctx.xshape, *ctx.geom) if ctx.needs_input_grad[0] \
-                    else None
-                dw = _deliver_grad(w, lambda out, acc: _conv_wgrad(xc, dy2, wc, *ctx.geom, out,
-                                                                   acc))
-                return dx, dw, None, None, None, None
+        # (saved-tensor hooks may give back another layout)
+        xc, wc = (x, w) if ctx.direct else (x.contiguous(), w.contiguous())
+        route = 0 if (xc.data_ptr() | wc.data_ptr() | dy2.data_ptr()) % 16 else ctx.route
         dx = None
         if ctx.needs_input_grad[0]:
-            d = gemm(dy2, w, b_mn=True)                       # [M, Kpad]
-            dx = d.view(N, H, W, C) if ctx.direct else col2im(d, ctx.xshape, KH, KW, stride, pad)
+            if route & 2:
+                dx = _conv_dgrad(dy2, wc, ctx.xshape, *ctx.geom)
+            else:
+                d = gemm(dy2, wc, b_mn=True)                  # [M, Kpad]
+                dx = d.view(N, H, W, C) if ctx.direct else \
+                    col2im(d, ctx.xshape, KH, KW, stride, pad)
+        if route & 1:
+            dw = _deliver_grad(w, lambda out, acc: _conv_wgrad(xc, dy2, wc, *ctx.geom, out, acc))
+            return dx, dw, None, None, None, None
+        x, col = xc, None if col is None else col.contiguous()
         a = x.reshape(-1, C) if ctx.direct else \
             (col if col is not None else im2col(x, KH, KW, stride, pad))
         dw = _deliver_grad(w, lambda out, acc: gemm(dy2, a, a_mn=True, b_mn=True, out=out,
@@ -219,7 +235,7 @@ def _conv2d_plain(x, w, KH, KW, stride, pad):
     """The forward pass by itself."""
     N, H, W, C = x.shape
     direct = KH == 1 and KW == 1 and stride == 1 and pad == 0 and C % 8 == 0
-    if not direct and _image_kernels(x, w, KH, KW, stride, pad):
+    if not direct and _image_route(x, w, KH, KW, stride, pad) & 1:
         return _conv_fwd(x, w, KH, KW, stride, pad)
     a = x.reshape(-1, C) if direct else im2col(x, KH, KW, stride, pad)
     return gemm(a, w).view(N, *_out_hw(H, W, KH, KW, stride, pad), w.shape[0])

@@ -1,8 +1,12 @@
 """Calls that the convolution kernels on the image must leave to the gathered form, or answer as it
 does."""
+import importlib
+
 import pytest
 import torch
 import torch.nn.functional as F
+
+from test_conv_image_gpu import SHAPES, test_image_kernels_match_torch
 
 pytestmark = pytest.mark.gpu
 
@@ -17,6 +21,14 @@ def _close(got, want, mag, terms):
     bound = want.abs() * 2.0 ** -8 + mag * (terms + 16) * 2.0 ** -24 + 1e-30
     err = (got.double() - want).abs()
     assert bool((err <= bound).all()), float((err / bound).max())
+
+
+@pytest.mark.parametrize("route", [0, 1, 2, 3])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_every_route_at_every_shape(shape, route, monkeypatch):
+    monkeypatch.setattr(importlib.import_module("necklace_b200.ops.conv"), "_route",
+                        lambda *a: route)
+    test_image_kernels_match_torch(shape)
 
 
 @pytest.mark.parametrize("stride", [1, 2])
