@@ -312,7 +312,7 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ m
   const int ry = 256 / cx;
   const int tx = threadIdx.x % cx, ty = threadIdx.x / cx;
   const int c = (blockIdx.x * cx + tx) * 8;
-  if (c >= C) return;
+  if (c >= C || ty >= ry) return;
   float sc[8], sh[8];
   {
     uint4 vg = *reinterpret_cast<const uint4*>(gamma + c);
@@ -379,7 +379,7 @@ bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
   const int ry = 256 / cx;
   const int tx = threadIdx.x % cx, ty = threadIdx.x / cx;
   const int c = (blockIdx.x * cx + tx) * 8;
-  if (c >= C) return;
+  if (c >= C || ty >= ry) return;
   const float invM = 1.f / (float)M;
   // dx = k1 * dy' + k2 * x + k3 with k1 = gamma rstd, k2 = -k1 rstd s1/M,
   // k3 = -k1 (s0/M - mean rstd s1/M)
@@ -688,7 +688,8 @@ extern "C" int nkb_col2im_nhwc(const void* dcol, void* dx, int N, int H, int W, 
 static void bn_sums_dims(long long M, int C, int& cx, dim3& grid) {
   // strips of at most 32 chunks of 8 channels, all of the same width: with widths in powers of two
   // the 17 chunks of 136 channels were a strip of 16 and one of a single chunk, whose blocks held
-  // their place on the SM with one lane in 16 (evaluation, 802816 rows: 138 us)
+  // their place on the SM with one lane in 16 (802816 rows: evaluation 138 -> 81 us, there and back
+  // 456 -> 313 us).  The threads behind cx * ry (at most cx - 1) have no row.
   const int chunks = C / 8;
   const int gx = (chunks + 31) / 32;
   cx = (chunks + gx - 1) / gx;

@@ -70,3 +70,44 @@ def test_evaluation_batch_norm_bits(eps):
     bn.running_mean = torch.stack([bn.running_mean, bn.running_mean], 1)[:, 0]   # strided
     assert not bn.running_mean.is_contiguous()
     assert torch.equal(one, bn(x))
+
+
+@pytest.mark.parametrize("C", [24, 72, 136, 264, 520, 8192])
+@pytest.mark.parametrize("M", [1, 13, 5003])
+def test_batch_norm_strips(C, M):
+    """Channel counts whose chunks of 8 do not fill a power of two, there and back against fp64."""
+    from necklace_b200.ops.conv import BatchNorm2d
+    g = torch.Generator(device="cuda").manual_seed(C + M)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    bn = BatchNorm2d(C, relu=True, device="cuda")
+    with torch.no_grad():
+        bn.weight.copy_(r(C) * 0.3 + 1), bn.bias.copy_(r(C))
+    x = (r(M, 1, 1, C) + r(C)).bfloat16().requires_grad_(True)
+    res = r(M, 1, 1, C).bfloat16().requires_grad_(True)
+    dy = r(M, 1, 1, C).bfloat16()
+    y = bn(x, res)
+    y.backward(dy)
+    xd = x.detach().double().view(M, C).requires_grad_(True)
+    wd, bd = (t.detach().double().requires_grad_(True) for t in (bn.weight, bn.bias))
+    var, mean = torch.var_mean(xd, 0, unbiased=False)
+    rstd = torch.rsqrt(var + bn.eps)
+    xhat = (xd - mean) * rstd
+    out = xhat * wd + bd + res.detach().double().view(M, C)
+    # fp32 statistics: a rounding of the mean or of a square moves xhat by about 2^-22 of the
+    # channel's (largest value / spread)^2; one row has no spread but eps
+    move = 2.0 ** -22 * (1 + (xd.detach().abs().amax(0) * rstd.detach()).square())
+    err = (y.detach().double().view(M, C) - torch.relu(out)).abs()
+    assert bool((err <= out.abs() * 2.0 ** -8 + move * wd.abs() * 4 + 1e-6).all())
+    on = (y.detach().view(M, C) > 0).double()            # the signs of the stored output
+    d = dy.double().view(M, C) * on
+    assert torch.equal(res.grad.double().view(M, C), d)
+    out.backward(d)
+    h = xhat.detach().abs() + move
+    for got, want, mag in ((bn.bias.grad, bd.grad, d.abs().sum(0)),
+                           (bn.weight.grad, wd.grad, (d.abs() * h).sum(0))):
+        slack = mag * ((M + 16) * 2.0 ** -24 + move * 4)
+        assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-6).all())
+    k = (wd.abs() * rstd).detach()
+    mag = k * (d.abs() + d.abs().mean(0) + h * (d.abs() * h).mean(0))
+    bound = xd.grad.abs() * 2.0 ** -8 + mag * ((M + 16) * 2.0 ** -24 + move * 8) + 1e-6
+    assert bool(((x.grad.double().view(M, C) - xd.grad).abs() <= bound).all())
