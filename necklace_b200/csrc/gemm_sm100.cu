@@ -243,34 +243,40 @@ __device__ __noinline__ static void ag_copy_role(const GemmArgs& g) {
 __global__ void epoch_bump_kernel(int* epoch) { epoch[0] += 1; }
 
 // out = (accumulate ? out : 0) + alpha * sum_s ws[s]; 4 elements per thread (N % 4 == 0 and
-// 16-byte aligned rows are guaranteed by the caller).  Four threads share the slices of a
-// group of four elements: an output with few elements has up to 64 slices, and one thread
-// per group would run through them in a serial chain of loads on a few SMs.
+// 16-byte aligned rows are guaranteed by the caller).  With more than eight slices four threads
+// share those of a group of four elements: such an output has few elements, and one thread per
+// group would run through up to 64 slices in a serial chain of loads on a few SMs.  With fewer
+// that costs more than it brings (half of the threads have nothing to load with two slices).
+template <int LANES>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, int S, long long MN, int N, void* out,
                      long long ldc, int c_fp32, int accumulate, float alpha,
                      const float* __restrict__ alpha_dev) {
-  __shared__ float4 sh[3][64];
+  constexpr int GROUPS = 256 / LANES;
+  __shared__ float4 sh[LANES > 1 ? LANES - 1 : 1][GROUPS];
   if (alpha_dev) alpha *= *alpha_dev;
-  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+  const int tx = threadIdx.x % GROUPS, ty = threadIdx.x / GROUPS;
   const long long n4 = MN >> 2;
-  const long long i = (long long)blockIdx.x * 64 + tx;
+  const long long i = (long long)blockIdx.x * GROUPS + tx;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   if (i < n4) {
 #pragma unroll 4
-    for (int s = ty; s < S; s += 4) {
+    for (int s = ty; s < S; s += LANES) {
       const float4 v = reinterpret_cast<const float4*>(ws + (long long)s * MN)[i];
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
   }
-  if (ty) sh[ty - 1][tx] = acc;
-  __syncthreads();
-  if (ty || i >= n4) return;
+  if constexpr (LANES > 1) {
+    if (ty) sh[ty - 1][tx] = acc;
+    __syncthreads();
+    if (ty) return;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float4 v = sh[k][tx];
-    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    for (int k = 0; k < LANES - 1; ++k) {
+      const float4 v = sh[k][tx];
+      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    }
   }
+  if (i >= n4) return;
   const long long e = i << 2, row = e / N, col = e % N;
   acc.x *= alpha; acc.y *= alpha; acc.z *= alpha; acc.w *= alpha;
   if (c_fp32) {
@@ -1555,9 +1561,10 @@ static int gemm_run_splitk(GemmArgs g, const CUtensorMap& tmA, const CUtensorMap
   }
   if (rc) return rc;
   const long long MN = (long long)g.M * g.N;
-  const unsigned blocks = (unsigned)((MN / 4 + 63) / 64);
-  splitk_reduce_kernel<<<blocks, 256, 0, s>>>(g.splitk_ws, g.split_k, MN, g.N, g.C, g.ldc, g.c_fp32,
-                                              g.accumulate, g.alpha, g.alpha_dev);
+  auto reduce = g.split_k > 8 ? splitk_reduce_kernel<4> : splitk_reduce_kernel<1>;
+  const int per_block = 4 * 256 / (g.split_k > 8 ? 4 : 1);  // elements
+  reduce<<<(unsigned)((MN + per_block - 1) / per_block), 256, 0, s>>>(
+      g.splitk_ws, g.split_k, MN, g.N, g.C, g.ldc, g.c_fp32, g.accumulate, g.alpha, g.alpha_dev);
   return (int)cudaGetLastError();
 }
 

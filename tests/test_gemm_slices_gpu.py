@@ -39,3 +39,27 @@ def test_every_kind_of_tile_that_the_sizes_choose(M, N, K, a_mn, b_mn):
     b = torch.randn(*((K, N) if b_mn else (N, K)), generator=g, device="cuda").bfloat16()
     A, B = (a.t() if a_mn else a).double(), (b.t() if b_mn else b).double()
     _close(gemm(a, b, a_mn=bool(a_mn), b_mn=bool(b_mn)), A @ B.t(), A.abs() @ B.abs().t(), K)
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 64, 2048), (64, 64, 4096), (64, 64, 4608), (132, 260, 4160),
+                                   (1032, 1024, 8200)])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_reduction_of_few_and_many_slices(M, N, K, fp32):
+    """Up to eight slices are added by one thread per group of columns, more by four: both, at the
+    line between them, written and added to, with rows apart."""
+    from necklace_b200 import _lib
+    from necklace_b200.ops.gemm import gemm
+    assert _lib.value("nkb_gemm_slices", M, N, K, N + 8, 0) > 1
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    b = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    want, mag = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    wide = torch.full((M, N + 8), 3.0, dtype=torch.float32 if fp32 else torch.bfloat16,
+                      device="cuda")
+    out, rel = wide[:, :N], 0.0 if fp32 else 2.0 ** -8
+    gemm(a, b, out=out, alpha=0.5)
+    assert bool(((out.double() - want / 2).abs() <= want.abs() * rel + mag * (K + 16) * 2.0 ** -24).all())
+    gemm(a, b, out=out, accumulate=True, alpha_dev=torch.full((1,), 2.0, device="cuda"))
+    bound = want.abs() * 4 * rel + mag * (K + 16) * 2.0 ** -21
+    assert bool(((out.double() - 2.5 * want).abs() <= bound).all())
+    assert bool((wide[:, N:] == 3).all())
