@@ -39,7 +39,7 @@ _SIGS = {
     "nkb_norm_bwd_dx_res": [vp, vp, vp, vp, vp, i32, i32, i32, vp, vp],
     "nkb_norm_bwd_all": [vp, vp, vp, vp, vp, vp, i32, i32, i32, vp, vp, vp, vp, i32, i32, vp],
     "nkb_colsum": [vp, vp, vp, vp, i32, i32, i64, i32, vp],
-    "nkb_colsum_fused": [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i64, i32, vp],
+    "nkb_colsum_fused": [vp, vp, vp, vp, i32, i32, i32, i64, vp],
     "nkb_f32_to_bf16": [vp, vp, i64, i32, vp],
     "nkb_ce_fwd_bwd": [vp, vp, vp, i32, i32, i64, f32, vp],
     "nkb_ce_stats": [vp, vp, vp, i32, i32, i64, i32, vp],

@@ -388,8 +388,8 @@ __device__ __forceinline__ void colsum_cp16(void* smem_dst, const void* gsrc) {
 __global__ void __launch_bounds__(256)
 colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
               const float* __restrict__ stats, float* __restrict__ acc, int rows, int C,
-              long long ld, int rms, int* __restrict__ tickets, __nv_bfloat16* __restrict__ out_a,
-              __nv_bfloat16* __restrict__ out_b, int accum_a, int accum_b) {
+              long long ld, int rms, int* __restrict__ tickets, __nv_bfloat16* __restrict__ out,
+              int accumulate) {
   // ring slots [which: dy | x][slot][thread] (16 bytes each); the reduction buffer reuses it
   extern __shared__ __align__(16) uint8_t colsum_smem[];  // COLSUM_SMEM_BYTES, dynamic
   uint4 (*ring)[COLSUM_RING][256] = reinterpret_cast<uint4 (*)[COLSUM_RING][256]>(colsum_smem);
@@ -488,14 +488,9 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restr
   __threadfence();
   const int gc = blockIdx.x * 256 + threadIdx.x;
   if (gc < C) {
-    for (int which = x ? 0 : 1; which < 2; ++which) {
-      float v = atomicExch(&acc[(long long)which * C + gc], 0.f);
-      __nv_bfloat16* out = which == 0 ? out_a : out_b;
-      if (out) {
-        if (which == 0 ? accum_a : accum_b) v += __bfloat162float(out[gc]);
-        out[gc] = __float2bfloat16(v);
-      }
-    }
+    float v = atomicExch(&acc[(long long)C + gc], 0.f);
+    if (accumulate) v += __bfloat162float(out[gc]);
+    out[gc] = __float2bfloat16(v);
   }
   if (threadIdx.x == 0) tickets[blockIdx.x] = 0;
 }
@@ -615,25 +610,22 @@ extern "C" int nkb_colsum(const void* dy, const void* x, const float* stats, flo
   if (colsum_configure()) return -6;
   colsum_kernel<<<dim3(gx, gy), 256, nkb::COLSUM_SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, acc, rows,
-      C, ld, rms, nullptr, nullptr, nullptr, 0, 0);
+      C, ld, rms, nullptr, nullptr, 0);
   return (int)cudaGetLastError();
 }
 
-// Column sums straight to bf16 outputs in one launch.  acc: fp32 [2][C] and tickets: int
-// [ceil(C/256)], both owned by the caller, zero before the first call and left zero by every
-// call (calls that share them must be ordered on one stream).  With x / stats: out_a = sum of
-// dy * xhat (norm weight gradient), out_b = sum of dy; without: only out_b.
-extern "C" int nkb_colsum_fused(const void* dy, const void* x, const float* stats, float* acc,
-                                int* tickets, void* out_a, void* out_b, int accum_a, int accum_b,
-                                int rows, int C, long long ld, int rms, void* stream) {
-  if ((C & 1) || (ld & 1) || !acc || !tickets) return -3;
+// Column sums of dy straight to a bf16 output in one launch.  acc: fp32 [2][C] (the second half
+// is used) and tickets: int [ceil(C/256)], both owned by the caller, zero before the first call
+// and left zero by every call (calls that share them must be ordered on one stream).
+extern "C" int nkb_colsum_fused(const void* dy, float* acc, int* tickets, void* out,
+                                int accumulate, int rows, int C, long long ld, void* stream) {
+  if ((C & 1) || (ld & 1) || !acc || !tickets || !out) return -3;
   int gx = (C + 255) / 256;
   int gy = colsum_row_splits(gx, rows);
   if (colsum_configure()) return -6;
   colsum_kernel<<<dim3(gx, gy), 256, nkb::COLSUM_SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, acc, rows,
-      C, ld, rms, tickets, static_cast<__nv_bfloat16*>(out_a), static_cast<__nv_bfloat16*>(out_b),
-      accum_a, accum_b);
+      static_cast<const __nv_bfloat16*>(dy), nullptr, nullptr, acc, rows, C, ld, 0, tickets,
+      static_cast<__nv_bfloat16*>(out), accumulate);
   return (int)cudaGetLastError();
 }
 

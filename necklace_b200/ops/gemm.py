@@ -139,9 +139,8 @@ def colsum(dy: torch.Tensor, out: torch.Tensor | None = None, accumulate: bool =
         return out
     assert dy.dtype == torch.bfloat16 and dy.stride(1) == 1
     acc, tickets = colsum_scratch(Cn, dy.device)
-    _lib.call("nkb_colsum_fused", dy.data_ptr(), None, None, acc.data_ptr(), tickets.data_ptr(),
-              None, out.data_ptr(), 0, int(accumulate), rows, Cn, dy.stride(0), 0,
-              _lib.stream_ptr())
+    _lib.call("nkb_colsum_fused", dy.data_ptr(), acc.data_ptr(), tickets.data_ptr(),
+              out.data_ptr(), int(accumulate), rows, Cn, dy.stride(0), _lib.stream_ptr())
     _lib.count_launch()
     return out
 
