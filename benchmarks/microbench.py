@@ -65,15 +65,22 @@ def bench_gemm(flush):
     return rows
 
 
+def _layer_norm_backward(x):
+    """The backward of the layer as a training step runs it (one kernel)."""
+    from necklace_b200.ops.norm import LayerNorm
+    ln, leaf = LayerNorm(x.shape[1], device="cuda"), x.clone().requires_grad_(True)
+    y, wanted = ln(leaf), [leaf, ln.weight, ln.bias]
+    return lambda: torch.autograd.grad(y, wanted, x, retain_graph=True)
+
+
 def bench_norm(flush):
-    from necklace_b200.ops.norm import norm_fwd, norm_bwd
+    from necklace_b200.ops.norm import norm_fwd
     rows, C = 65536, 1024
     x = torch.randn(rows, C, device="cuda").bfloat16()
     w = torch.ones(C, device="cuda").bfloat16()
     b = torch.zeros(C, device="cuda").bfloat16()
     ms = _time(lambda: norm_fwd(x, w, b, 1e-5, False), flush=flush)
-    y, st = norm_fwd(x, w, b, 1e-5, False)
-    ms_b = _time(lambda: norm_bwd(x, x, w, st, False), flush=flush)
+    ms_b = _time(_layer_norm_backward(x), flush=flush)
     byts = rows * C * 2
     print(json.dumps({"op": "layernorm_fwd", "ms": round(ms, 4), "GBps": round(2 * byts / ms / 1e6)}))
     print(json.dumps({"op": "layernorm_bwd(dx+dw+db)", "ms": round(ms_b, 4),
@@ -156,14 +163,13 @@ def bench_small(flush):
     size: larger than L2, small enough for a counter capture of single launches."""
     from necklace_b200.ops import adam_step, cross_entropy_fwd_bwd
     from necklace_b200.ops.conv import Conv2d
-    from necklace_b200.ops.norm import norm_bwd, norm_fwd
+    from necklace_b200.ops.norm import norm_fwd
     rows, C = 65536, 1024
     x = torch.randn(rows, C, device="cuda").bfloat16()
     w = torch.ones(C, device="cuda").bfloat16()
     b = torch.zeros(C, device="cuda").bfloat16()
-    y, st = norm_fwd(x, w, b, 1e-5, False)
     ms = _time(lambda: norm_fwd(x, w, b, 1e-5, False), iters=2, warmup=1, flush=flush)
-    ms_b = _time(lambda: norm_bwd(x, x, w, st, False), iters=2, warmup=1, flush=flush)
+    ms_b = _time(_layer_norm_backward(x), iters=2, warmup=1, flush=flush)
     byts = rows * C * 2
     print(json.dumps({"op": "layernorm_fwd", "rows": rows, "C": C, "ms": round(ms, 4),
                       "GBps": round(2 * byts / ms / 1e6)}))

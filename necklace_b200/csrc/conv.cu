@@ -3,7 +3,7 @@
 //
 // A convolution is a GEMM on the tcgen05 kernel of gemm_sm100.cu:
 //   1x1 stride 1      activations [N*H*W, Cin] are the A operand as they are;
-//   C, Cout % 8 == 0  conv_sm100.cu reads the image itself;
+//   C, Cout % 8 == 0  conv_sm100.cu reads the image itself where nkb_conv_route finds that quicker;
 //   everything else   `im2col` gathers the receptive fields into col [N*Ho*Wo, KH*KW*Cin]
 //                     (K index = (kh*KW + kw)*Cin + c, zero for padding), the weight is stored
 //                     [Cout, KH*KW*Cin]; the data gradient is GEMM + `col2im` (written as a
@@ -306,7 +306,8 @@ __global__ void bn_finalize_kernel(float* __restrict__ acc, float* __restrict__ 
 // thread owns 8 fixed channels (its per-channel constants stay in registers) and walks rows.
 __global__ void __launch_bounds__(256)
 bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ mean,
-                const float* __restrict__ spread, float eps, const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
+                const float* __restrict__ spread, float eps,
+                const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
                 const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ y,
                 uint8_t* __restrict__ mask, long long M, int C, int cx, int relu) {
   const int ry = 256 / cx;
@@ -652,19 +653,19 @@ extern "C" int nkb_im2col_nhwc(const void* x, void* col, int N, int H, int W, in
   const long long M = (long long)N * g.Ho * g.Wo;
   const bool vec = (C % 8 == 0) && !(reinterpret_cast<uintptr_t>(x) & 15) &&
                    !(reinterpret_cast<uintptr_t>(col) & 15);
-  if (vec)
+  if (vec) {
     im2col_kernel<8><<<conv_grid(M * (Kpad / 8), 256), 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g);
-  else if (int tw = im2col_tile(g); tw > 0 && !(reinterpret_cast<uintptr_t>(col) & 15)) {
+  } else if (int tw = im2col_tile(g); tw > 0 && !(reinterpret_cast<uintptr_t>(col) & 15)) {
     const int row_elems = ((tw - 1) * stride + KW) * C, tiles_w = (g.Wo + tw - 1) / tw;
     im2col_tile_kernel<<<(unsigned)(tiles_w * (long long)g.Ho * N), 256,
                          2 * (Kpad + KH * row_elems + 8), s>>>(
         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g, tw, row_elems,
         tiles_w);
-  }
-  else
+  } else {
     im2col_kernel<1><<<conv_grid(M * Kpad, 256), 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g);
+  }
   return (int)cudaGetLastError();
 }
 
@@ -711,8 +712,9 @@ static void bn_sums_dims(long long M, int C, int& cx, dim3& grid) {
 // thread's call on that stream may come between them.
 static std::mutex g_bn_order;
 extern "C" int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, const void* res,
-                          void* y, void* mask, float* stats, float* acc, float* run_mean, float* run_var,
-                          long long M, int C, float eps, float momentum, int relu, void* stream) {
+                          void* y, void* mask, float* stats, float* acc, float* run_mean,
+                          float* run_var, long long M, int C, float eps, float momentum, int relu,
+                          void* stream) {
   if (C % 8) return -3;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) |
        reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) & 15)
@@ -729,7 +731,8 @@ extern "C" int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, co
                                                      momentum);
   bn_apply_kernel<<<grid, 256, 0, s>>>(
       static_cast<const __nv_bfloat16*>(x), stats, stats + C, -1.f,
-      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
+      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
+      static_cast<const __nv_bfloat16*>(res),
       static_cast<__nv_bfloat16*>(y), static_cast<uint8_t*>(mask), M, C, cx, relu);
   return (int)cudaGetLastError();
 }
@@ -743,7 +746,8 @@ extern "C" int nkb_bn_apply(const void* x, const float* stats, const void* gamma
   bn_sums_dims(M, C, cx, grid);
   bn_apply_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), stats, stats + C, -1.f,
-      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
+      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
+      static_cast<const __nv_bfloat16*>(res),
       static_cast<__nv_bfloat16*>(y), nullptr, M, C, cx, relu);
   return (int)cudaGetLastError();
 }
@@ -808,8 +812,8 @@ extern "C" int nkb_maxpool3x3s2_bwd(const void* dy, const void* idx, void* dx, i
                                     int C, void* stream) {
   if (C % 8) return -3;
   const int Ho = (H + 2 - 3) / 2 + 1, Wo = (W + 2 - 3) / 2 + 1;
-  maxpool_bwd_kernel<<<conv_grid((long long)N * ((H + 1) / 2) * ((W + 1) / 2) * (C / 8), 256), 256, 0,
-                       static_cast<cudaStream_t>(stream)>>>(
+  const long long quads = (long long)N * ((H + 1) / 2) * ((W + 1) / 2) * (C / 8);
+  maxpool_bwd_kernel<<<conv_grid(quads, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const uint8_t*>(idx),
       static_cast<__nv_bfloat16*>(dx), N, H, W, C, Ho, Wo);
   return (int)cudaGetLastError();

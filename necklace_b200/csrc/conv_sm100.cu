@@ -11,11 +11,14 @@
 //
 //   forward        y[p, co]      = sum over tap, ci  x[p * s + tap - pad, ci]  w[co, tap, ci]
 //   data gradient  dx[q, ci]     = sum over tap, co  dy[(q + pad - tap) / s, co]  w[co, tap, ci]
-//                  for a stride s > 1 one launch per class of positions q mod s, whose taps are those that
-//                  divide; the output is a strided view of dx
-//                  Each tap's product is rounded to bf16 before the taps are added in fp32, as when
-//                  it went through memory: every tap is an accumulator of its own, which the
-//                  epilogue adds up in registers
+//                  for a stride s > 1 one launch per class of positions q mod s, whose taps are
+//                  those that divide; the output is a strided view of dx.
+//                  Each tap's product is rounded to bf16 before the taps are added in fp32: every
+//                  tap is an accumulator of its own, which the epilogue adds up in registers.
+//                  The gathered form rounds there because the products go through memory; here
+//                  the only reason is that both forms of a layer then give the same results (one
+//                  accumulator for all taps is quicker and rounds once: it moved results by
+//                  0.26 % of their norm)
 //   weight grad.   dw[co, tap, ci] = sum over p  dy[p, co]  x[p * s + tap - pad, ci]
 //                  pixels are the contraction: boxes of at most 64 of them, both operands
 //                  MN-major, the range of boxes split over all SMs, fp32 partial sums
@@ -24,8 +27,8 @@
 // reads of the image from L2, with more channels the tensor cores.  ResNet-50, 256 images of
 // 224 x 224, the 19 layers that were gathered, in us: forward 2832 (gather) + about 1700 (GEMM)
 // before, 1355 now; data gradient 2777 (scatter) + about 2500, now 1888 (1456 with one accumulator
-// for all taps, which rounds once); weight gradient about 5000, now 1458.  The training step
-// went from 38.4 to 30.2 ms.
+// for all taps, which rounds once); weight gradient about 5000, now 1458.  Layers with few
+// positions or few channels are quicker gathered: nkb_conv_route decides.
 //
 // Warp roles and pipeline are those of the GEMM (gemm_sm100.cu): one TMA producer thread, one
 // MMA thread, eight epilogue warps, two accumulators in TMEM, one CTA per SM, tiles dealt
@@ -355,7 +358,8 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           for (int k = 0; k < Q; ++k) {
             const float* f = sum + ch * 64 + k * 8;
             const int q = BN == 64 ? group * 4 + k : k;
-            *reinterpret_cast<uint4*>(tile + lane_grp * 4096 + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+            uint8_t* row = tile + lane_grp * 4096 + lane * 128;
+            *reinterpret_cast<uint4*>(row + ((q ^ (lane & 7)) << 4)) =
                 make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]),
                            pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
           }
@@ -367,8 +371,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
       }
-    } else
-    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+    } else for (int u = blockIdx.x; u < units; u += gridDim.x) {
       const bool mine = BN > 64 || acc == group;
       if (mine) {
         const bool ok = mbar_wait(&acc_full[acc], acc_phase, abort_flag);
@@ -522,7 +525,8 @@ static void pick_box(int W, int H, int N, int stride, int& bw, int& bh, int& bn)
         if (h <= lim) {
           int n = 128 / (w * h);
           if (n > N) n = N;
-          const long long cost = (long long)((W + w - 1) / w) * ((H + h - 1) / h) * ((N + n - 1) / n);
+          const long long cost =
+              (long long)((W + w - 1) / w) * ((H + h - 1) / h) * ((N + n - 1) / n);
           if (best < 0 || cost < best) { best = cost; bw = w; bh = h; bn = n; }
         }
         const int k = (H + h - 1) / h + 1, nx = (H + k - 1) / k;
@@ -574,8 +578,9 @@ static int launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap&
 }
 
 // Column tile: as wide as the columns allow; between 128 and 256 what the last round of tiles
-// leaves idle decides, with the rates of the two widths that the GEMM's tiles were measured at
-// (0.68 : 0.88 of a CTA pair's).
+// leaves idle decides, a round of 256 columns counted as 1.55 rounds of 128.  The weight is a
+// GEMM's, not these kernels' own: fitted over 502 layers (see nkb_conv_route) a step of 256
+// columns takes 1.25 times one of 128.
 static int pick_bn(int tiles_m, int cols) {
   if (cols <= 64) return 64;
   if (cols <= 128) return 128;
@@ -788,16 +793,17 @@ extern "C" int nkb_conv_wgrad(const void* x, const void* dy, void* dw, float* ws
 //
 // The image kernels read no gathered matrix, but a tile runs through all taps and channels one
 // after the other and K is not split, so a layer with few positions and a long contraction leaves
-// most SMs idle, where the GEMM of the gathered form has slices: 512 -> 512, 3x3, stride 2, 8 images
-// of 14 x 14 take 23 + 15 + 39 us on the image (forward, weight and data gradient; the last in
-// four launches, one per class of positions), 11 + 9 + 12 us gathered.  With few channels a step
-// of 64 is mostly empty and a box has rows of 16 bytes: 8 -> 64, 3x3, 128 images of 56 x 56 take
-// 231 + 125 + 206 us on the image, 95 + 35 + 78 gathered.  With 64 channels and more and pixels enough the
-// image wins: 64 -> 64, 3x3, 64 images of 28 x 28, 13 + 18 + 19 against 44 + 15 + 49 us.
+// most SMs idle, where the GEMM of the gathered form has slices: 512 -> 512, 3x3, stride 2, 8
+// images of 14 x 14 take 23 + 15 + 39 us on the image (forward, weight and data gradient; the last
+// in four launches, one per class of positions), 11 + 9 + 12 us gathered.  With few channels a
+// step of 64 is mostly empty and a box has rows of 16 bytes: 8 -> 64, 3x3, 128 images of 56 x 56
+// take 231 + 125 + 206 us on the image, 95 + 35 + 78 gathered.  With 64 channels and more and
+// pixels enough the image wins: 64 -> 64, 3x3, 64 images of 28 x 28, 13 + 18 + 19 against
+// 44 + 15 + 49 us.
 // Times in us fitted to 502 layers (C, Cout 8 .. 1024, windows 1 .. 7, strides 1 and 2, 1 .. 256
 // images): choosing by them is 0.3 % (forward and weight gradient) and 2 % (data gradient) above
 // the quicker form on average; the image for all was 23 and 28 %.  The gathered form has another
-// kernel to launch, which costs the host about 4 us: it must win by more.
+// kernel to launch, which costs the host about 4 us: it must win by more (3 % with that).
 extern "C" int nkb_conv_route(int N, int H, int W, int C, int Cout, int KH, int KW, int stride,
                               int pad) {
   if (!conv_ok(N, H, W, C, Cout, KH, KW, stride, pad) || stride > 2) return -3;

@@ -1,11 +1,12 @@
 """ResNet-50 (bottleneck blocks [3, 4, 6, 3], 1000 classes) for the data-parallel
 benchmark configuration, entirely on this library's kernels.
 
-Activations are channels-last (``[N, H, W, C]``) bf16.  Every convolution is a GEMM on the
-tcgen05 kernel: the 1x1 ones on the activation matrix as it is, the 3x3 / 7x7 / strided
-ones on a gathered ``col`` matrix (``ops.conv``); batch norm, the residual add and ReLU
-are one fused kernel after the statistics pass; max / average pooling, the classifier and
-its cross-entropy are native kernels as well, so the step contains no cuDNN call.  The
+Activations are channels-last (``[N, H, W, C]``) bf16.  The 1x1 convolutions are GEMMs on the
+activation matrix as it is; the 3x3 and strided ones run on the image itself, or gathered where
+their sizes make that quicker, the 7x7 stem on a gathered ``col`` matrix (``ops.conv``); batch
+norm, the residual add and ReLU are one fused kernel after the statistics pass; max / average
+pooling, the classifier and its cross-entropy are native kernels as well, so the step contains
+no cuDNN call.  The
 reference itself only ships MNIST-sized CNNs (examples/dp/mnist/pytorch/main.py); ResNet-50
 comes from the benchmark configurations.
 """

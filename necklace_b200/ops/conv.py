@@ -1,11 +1,12 @@
 """Convolution, batch norm (+ residual + ReLU) and pooling on channels-last bf16 tensors.
 
 Tensors are ``[N, H, W, C]`` (NHWC) everywhere, so a 1x1 convolution is a GEMM on the
-activation matrix as it is (``ops.gemm``).  Every other convolution whose channel counts are
-multiples of 8 runs on the tcgen05 convolution kernels, which read shifted boxes of the image
-through 4-D tensor maps; the rest (a 3-channel stem) is a GEMM on a gathered ``col`` matrix.  Weights are stored
-``[C_out, KH*KW*C_in]`` with the input channel innermost, which is what that GEMM wants as
-its K-major B operand.  CPU tensors take PyTorch reference paths (``F.conv2d`` and friends
+activation matrix as it is (``ops.gemm``).  Other convolutions whose channel counts are multiples
+of 8 run on the tcgen05 convolution kernels, which read shifted boxes of the image through 4-D
+tensor maps, where that is the quicker form for their sizes (``_route``); the rest (a 3-channel
+stem, a handful of pixels) is a GEMM on a gathered ``col`` matrix.  Weights are stored
+``[C_out, KH*KW*C_in]`` with the input channel innermost, which is what that GEMM wants as its
+K-major B operand.  CPU tensors take PyTorch reference paths (``F.conv2d`` and friends
 on permuted views), which the CPU test-suite and the GPU numerics tests compare against.
 
 These operators replace the cuDNN convolutions / batch norm / pooling the reference's CNN
