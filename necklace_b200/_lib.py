@@ -235,8 +235,11 @@ def call(name: str, *args) -> None:
 
 def value(name: str, *args) -> int:
     """What a native function that answers a question returns."""
-    lib = load()
-    return (_fast.get(name) or getattr(lib, name))(*args)
+    fn = _fast.get(name)
+    if fn is None:
+        lib = load()
+        fn = _fast.get(name) or getattr(lib, name)
+    return fn(*args)
 
 
 def stream_ptr() -> int:

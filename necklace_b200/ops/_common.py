@@ -8,6 +8,11 @@ import torch.autograd.forward_ad as _fwd_ad
 
 from .. import _lib
 
+_grad_on = torch.is_grad_enabled
+_trace = torch._C._get_tracing_state
+_transform = torch._C._functorch.peek_interpreter_stack
+_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", None)   # (CUDA builds)
+
 _status: dict[int, torch.Tensor] = {}
 _status_at: dict[int, int] = {}      # their addresses: the tensors live as long as the process
 _scratch: dict[tuple, object] = {}   # (tag, device, stream, capture) -> what `make` gave
@@ -51,9 +56,8 @@ def plain_call() -> bool:
     """Whether an operator may run its forward pass without an autograd node: gradients are off,
     and neither forward-mode differentiation, a trace nor a function transform is looking (the
     last refuse these operators, with a message of their own)."""
-    return not torch.is_grad_enabled() and _fwd_ad._current_level < 0 \
-        and torch._C._get_tracing_state() is None \
-        and torch._C._functorch.peek_interpreter_stack() is None
+    return not _grad_on() and _fwd_ad._current_level < 0 and _trace() is None \
+        and _transform() is None
 
 
 def check_status(reset: bool = True) -> None:
@@ -73,7 +77,7 @@ def stream_scratch(tag: str, device: torch.device, make):
     A graph being captured gets scratch of its own, cleared by the graph itself, because replays
     of two graphs may overlap wherever they were captured."""
     s = _lib.stream_ptr()
-    capture = _lib.value("nkb_capture_id", s)
+    capture = _lib.value("nkb_capture_id", s) if _capturing() else 0
     k = (tag, device.index, s, capture)
     t = _scratch.get(k)
     if t is None:
