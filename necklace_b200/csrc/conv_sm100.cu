@@ -803,7 +803,8 @@ extern "C" int nkb_conv_wgrad(const void* x, const void* dy, void* dw, float* ws
 // Times in us fitted to 502 layers (C, Cout 8 .. 1024, windows 1 .. 7, strides 1 and 2, 1 .. 256
 // images): choosing by them is 0.3 % (forward and weight gradient) and 2 % (data gradient) above
 // the quicker form on average; the image for all was 23 and 28 %.  The gathered form has another
-// kernel to launch, which costs the host about 4 us: it must win by more (3 % with that).
+// kernel and buffer, which cost the host 6 to 8 us a pass: it must win by more than that (with 4 and
+// 3 us a pass of ResNet-50 over 37 images, issued eagerly, took 3 % longer than all on the image).
 extern "C" int nkb_conv_route(int N, int H, int W, int C, int Cout, int KH, int KW, int stride,
                               int pad) {
   if (!conv_ok(N, H, W, C, Cout, KH, KW, stride, pad) || stride > 2) return -3;
@@ -854,7 +855,7 @@ extern "C" int nkb_conv_route(int N, int H, int W, int C, int Cout, int KH, int 
       image_dx += 3.2 + r * (taps * (mma > drain ? mma : drain) + 1.6);
     }
   const double gathered_dx = 4.9 + mb / 1.5 + gemm_time_us((int)P, (int)K, Cout);
-  return (image <= gathered + 4.0 ? 1 : 0) | (image_dx <= gathered_dx + 3.0 ? 2 : 0);
+  return (image <= gathered + 8.0 ? 1 : 0) | (image_dx <= gathered_dx + 6.0 ? 2 : 0);
 }
 
 NKB_DEFINE_WAIT_SETTER(conv)
