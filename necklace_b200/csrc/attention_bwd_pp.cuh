@@ -71,6 +71,7 @@ attn_bwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023) {
+    if (!grid_dep_wait()) return;
     if (threadIdx.x == 0 && a.status) atomicCAS(a.status, 0, (int)NKB_ERR_BOUNDS);
     return;
   }
@@ -143,6 +144,7 @@ attn_bwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!grid_dep_wait()) return;
 
   if (warp >= 12) {
     // =================================================================== control
@@ -171,6 +173,7 @@ attn_bwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_expect_tx(&do_full[o], TILE);
         load_tile(sDO + o * TILE, &tmDO, &do_full[o], (i0 + it) * 128);
       }
+      grid_dep_trigger();
     } else if (warp == 13 && lane == 0) {
       // -------------------------------------------------------------- MMA issuer
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);  // S^T, dP^T

@@ -97,6 +97,7 @@ attn_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     *abort_flag = 0;
     mbar_fence_init();
+    if (!grid_dep_wait()) return;
     mbar_expect_tx(q_full, 2 * TILE);
     load_tile(sQ, &tmQ, q_full, m0);
     load_tile(sQ + TILE, &tmQ, q_full, m0 + 128);
@@ -115,6 +116,7 @@ attn_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!grid_dep_wait()) return;
 
   if (warp >= 8) reg_alloc_dec<40>();
   if (warp == 8) {
@@ -136,6 +138,7 @@ attn_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_expect_tx(&v_full[st], TILE);
         load_tile(sV + st * TILE, &tmV, &v_full[st], j * 128);
       }
+      grid_dep_trigger();
     }
   } else if (warp == 9 || warp == 10) {
     // ------------------------------------------------- MMA issuer of half x = warp - 9

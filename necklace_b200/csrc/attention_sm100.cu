@@ -111,6 +111,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!grid_dep_wait()) return;
 
   if (warp == 4) {
     if (lane == 0) {
@@ -408,6 +409,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!grid_dep_wait()) return;
 
   if (warp == 4) {
     if (lane == 0) {
@@ -621,6 +623,7 @@ __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                   float* __restrict__ delta, int B, int H, int S, int D, long long ob, long long oh,
                   long long os, float* __restrict__ dq_acc) {
+  if (!grid_dep_begin()) return;
   // also clears the fp32 dQ accumulator [B*H*S, D] (each lane its D/8 floats of the row), so no
   // separate fill kernel runs before the backward kernel
   const long long slot = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
@@ -703,6 +706,7 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 __global__ void __launch_bounds__(256)
 attn_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B, int H,
                        int S, int D, long long sb, long long sh, long long ss) {
+  if (!grid_dep_begin()) return;
   const long long n8 = (long long)B * H * S * D / 8;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8;
        i += (long long)gridDim.x * blockDim.x) {
@@ -772,7 +776,7 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   static bool done[64];
   if (int e = allow_smem(attn_fwd_kernel<D, EXPM>, smem, done)) return e;
   dim3 grid(a.B * a.H, (a.S + 127) / 128);
-  attn_fwd_kernel<D, EXPM><<<grid, ATT_THREADS, smem, s>>>(tq, tk, tv, a);
+  launch_dep(attn_fwd_kernel<D, EXPM>, grid, ATT_THREADS, smem, s, tq, tk, tv, a);
   return (int)cudaGetLastError();
 }
 
@@ -786,7 +790,7 @@ static int launch_fwd_pp(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
   static bool done[64];
   if (int e = allow_smem(attn_fwd_pp_kernel<D, EXPM>, smem, done)) return e;
   dim3 grid(a.B * a.H, (a.S + 255) / 256);
-  attn_fwd_pp_kernel<D, EXPM><<<grid, ATT2_THREADS, smem, s>>>(tq, tk, tv, a);
+  launch_dep(attn_fwd_pp_kernel<D, EXPM>, grid, ATT2_THREADS, smem, s, tq, tk, tv, a);
   return (int)cudaGetLastError();
 }
 
@@ -810,7 +814,7 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   static bool done[64];
   if (int e = allow_smem(attn_bwd_kernel<D>, smem, done)) return e;
   dim3 grid(a.B * a.H, (a.S + 127) / 128);
-  attn_bwd_kernel<D><<<grid, ATT_THREADS, smem, s>>>(tq, tk, tv, tdo, a);
+  launch_dep(attn_bwd_kernel<D>, grid, ATT_THREADS, smem, s, tq, tk, tv, tdo, a);
   return (int)cudaGetLastError();
 }
 
@@ -840,7 +844,7 @@ static int launch_bwd_pp(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
   static bool done[64];
   if (int e = allow_smem(attn_bwd_pp_kernel<D>, smem, done)) return e;
   dim3 grid(a.B * a.H, (a.S + 127) / 128);
-  attn_bwd_pp_kernel<D><<<grid, BWD2_THREADS, smem, s>>>(tq, tk, tv, tdo, tdq, a);
+  launch_dep(attn_bwd_pp_kernel<D>, grid, BWD2_THREADS, smem, s, tq, tk, tv, tdo, tdq, a);
   return (int)cudaGetLastError();
 }
 
@@ -893,9 +897,9 @@ extern "C" int nkb_attn_bwd(const void* q, const void* k, const void* v, const v
   if ((rc = make_tmap_bshd(&tv, v, B, H, S, D, sb, sh, ss))) return rc;
   if ((rc = make_tmap_bshd(&tdo, dout, B, H, S, D, ob, oh, os))) return rc;
   const long long rows = (long long)B * H * S;
-  attn_delta_kernel<<<(unsigned)((rows * 8 + 256 * DELTA_ROWS - 1) / (256 * DELTA_ROWS)), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), delta, B, H, S,
-      D, ob, oh, os, dq_acc);
+  launch_dep(attn_delta_kernel, (unsigned)((rows * 8 + 256 * DELTA_ROWS - 1) / (256 * DELTA_ROWS)),
+             256, 0, s, static_cast<const __nv_bfloat16*>(o),
+             static_cast<const __nv_bfloat16*>(dout), delta, B, H, S, D, ob, oh, os, dq_acc);
   AttnBwdArgs a;
   a.lse = lse; a.delta = delta; a.dq_acc = dq_acc;
   a.dk = static_cast<__nv_bfloat16*>(dk);
@@ -918,8 +922,8 @@ extern "C" int nkb_attn_bwd(const void* q, const void* k, const void* v, const v
   long long n8 = rows * D / 8;
   int blocks = (int)((n8 + 255) / 256);
   if (blocks > 148 * 8) blocks = 148 * 8;
-  attn_dq_convert_kernel<<<blocks, 256, 0, s>>>(dq_acc, static_cast<__nv_bfloat16*>(dq), B, H, S, D,
-                                                sb, sh, ss);
+  launch_dep(attn_dq_convert_kernel, blocks, 256, 0, s, dq_acc, static_cast<__nv_bfloat16*>(dq), B,
+             H, S, D, sb, sh, ss);
   return (int)cudaGetLastError();
 }
 

@@ -35,6 +35,7 @@ struct ConvGeom {
 template <int VEC>
 __global__ void __launch_bounds__(256)
 im2col_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col, ConvGeom g) {
+  if (!grid_dep_begin()) return;
   const long long M = (long long)g.N * g.Ho * g.Wo;
   const int kchunks = g.Kpad / VEC;
   const int Kreal = g.KH * g.KW * g.C;
@@ -80,6 +81,7 @@ constexpr int IM2COL_TILE_SMEM = 40 * 1024;
 __global__ void __launch_bounds__(256)
 im2col_tile_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col, ConvGeom g,
                    int tw, int row_elems, int tiles_w) {
+  if (!grid_dep_begin()) return;
   extern __shared__ __align__(16) uint16_t ic_smem[];
   uint16_t* table = ic_smem;                       // [Kpad]: offset of entry k, pixel 0
   uint16_t* rows = ic_smem + g.Kpad;               // [KH][row_elems], then 8 zeros
@@ -131,6 +133,7 @@ im2col_tile_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
 template <int VEC>
 __global__ void __launch_bounds__(256)
 col2im_kernel(const __nv_bfloat16* __restrict__ dcol, __nv_bfloat16* __restrict__ dx, ConvGeom g) {
+  if (!grid_dep_begin()) return;
   const int cchunks = g.C / VEC;
   const long long total = (long long)g.N * g.H * g.W * cchunks;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -201,6 +204,7 @@ __global__ void __launch_bounds__(256)
 bn_sums_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ x,
                const uint8_t* __restrict__ mask, const float* __restrict__ stats,
                float* __restrict__ acc, long long M, int C, int cx) {
+  if (!grid_dep_begin()) return;
   __shared__ float sh[2][256][8 + 1];
   const int ry = 256 / cx;
   const int tx = threadIdx.x % cx, ty = threadIdx.x / cx;
@@ -285,6 +289,7 @@ bn_sums_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restr
 __global__ void bn_finalize_kernel(float* __restrict__ acc, float* __restrict__ stats,
                                    float* __restrict__ run_mean, float* __restrict__ run_var,
                                    long long M, int C, float eps, float momentum) {
+  if (!grid_dep_begin()) return;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const float inv = 1.f / (float)M;
@@ -310,6 +315,7 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ m
                 const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
                 const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ y,
                 uint8_t* __restrict__ mask, long long M, int C, int cx, int relu) {
+  if (!grid_dep_begin()) return;
   const int ry = 256 / cx;
   const int tx = threadIdx.x % cx, ty = threadIdx.x / cx;
   const int c = (blockIdx.x * cx + tx) * 8;
@@ -377,6 +383,7 @@ bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
                     const float* __restrict__ sums, const __nv_bfloat16* __restrict__ gamma,
                     __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dres, long long M,
                     int C, int cx) {
+  if (!grid_dep_begin()) return;
   const int ry = 256 / cx;
   const int tx = threadIdx.x % cx, ty = threadIdx.x / cx;
   const int c = (blockIdx.x * cx + tx) * 8;
@@ -440,6 +447,7 @@ bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
 __global__ void bn_param_grad_kernel(float* __restrict__ sums, __nv_bfloat16* __restrict__ dgamma,
                                      __nv_bfloat16* __restrict__ dbeta, int C, int acc_g,
                                      int acc_b) {
+  if (!grid_dep_begin()) return;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   float g = sums[C + c], b = sums[c];
@@ -460,6 +468,7 @@ __global__ void bn_param_grad_kernel(float* __restrict__ sums, __nv_bfloat16* __
 __global__ void __launch_bounds__(256)
 maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                    uint8_t* __restrict__ idx, int N, int H, int W, int C, int Ho, int Wo) {
+  if (!grid_dep_begin()) return;
   const int cch = C / 8;
   const long long total = (long long)N * Ho * Wo * cch;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -509,6 +518,7 @@ maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
 __global__ void __launch_bounds__(256)
 maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const uint8_t* __restrict__ idx,
                    __nv_bfloat16* __restrict__ dx, int N, int H, int W, int C, int Ho, int Wo) {
+  if (!grid_dep_begin()) return;
   const int cch = C / 8, Hb = (H + 1) / 2, Wb = (W + 1) / 2;
   const long long total = (long long)N * Hb * Wb * cch;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -570,6 +580,7 @@ maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const uint8_t* __restri
 __global__ void __launch_bounds__(256)
 avgpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int N,
                    int HW, int C) {
+  if (!grid_dep_begin()) return;
   const int cch = C / 8;
   const long long total = (long long)N * cch;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -599,6 +610,7 @@ avgpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
 __global__ void __launch_bounds__(256)
 avgpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx, int N,
                    int HW, int C) {
+  if (!grid_dep_begin()) return;
   const int cch = C / 8;
   const long long total = (long long)N * HW * cch;
   const float inv = 1.f / (float)HW;
@@ -654,17 +666,16 @@ extern "C" int nkb_im2col_nhwc(const void* x, void* col, int N, int H, int W, in
   const bool vec = (C % 8 == 0) && !(reinterpret_cast<uintptr_t>(x) & 15) &&
                    !(reinterpret_cast<uintptr_t>(col) & 15);
   if (vec) {
-    im2col_kernel<8><<<conv_grid(M * (Kpad / 8), 256), 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g);
+    launch_dep(im2col_kernel<8>, conv_grid(M * (Kpad / 8), 256), 256, 0, s,
+               static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g);
   } else if (int tw = im2col_tile(g); tw > 0 && !(reinterpret_cast<uintptr_t>(col) & 15)) {
     const int row_elems = ((tw - 1) * stride + KW) * C, tiles_w = (g.Wo + tw - 1) / tw;
-    im2col_tile_kernel<<<(unsigned)(tiles_w * (long long)g.Ho * N), 256,
-                         2 * (Kpad + KH * row_elems + 8), s>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g, tw, row_elems,
-        tiles_w);
+    launch_dep(im2col_tile_kernel, (unsigned)(tiles_w * (long long)g.Ho * N), 256,
+               2 * (Kpad + KH * row_elems + 8), s, static_cast<const __nv_bfloat16*>(x),
+               static_cast<__nv_bfloat16*>(col), g, tw, row_elems, tiles_w);
   } else {
-    im2col_kernel<1><<<conv_grid(M * Kpad, 256), 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g);
+    launch_dep(im2col_kernel<1>, conv_grid(M * Kpad, 256), 256, 0, s,
+               static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(col), g);
   }
   return (int)cudaGetLastError();
 }
@@ -678,11 +689,11 @@ extern "C" int nkb_col2im_nhwc(const void* dcol, void* dx, int N, int H, int W, 
                    !(reinterpret_cast<uintptr_t>(dcol) & 15);
   const long long px = (long long)N * H * W;
   if (vec)
-    col2im_kernel<8><<<conv_grid(px * (C / 8), 256), 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(dcol), static_cast<__nv_bfloat16*>(dx), g);
+    launch_dep(col2im_kernel<8>, conv_grid(px * (C / 8), 256), 256, 0, s,
+               static_cast<const __nv_bfloat16*>(dcol), static_cast<__nv_bfloat16*>(dx), g);
   else
-    col2im_kernel<1><<<conv_grid(px * C, 256), 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(dcol), static_cast<__nv_bfloat16*>(dx), g);
+    launch_dep(col2im_kernel<1>, conv_grid(px * C, 256), 256, 0, s,
+               static_cast<const __nv_bfloat16*>(dcol), static_cast<__nv_bfloat16*>(dx), g);
   return (int)cudaGetLastError();
 }
 
@@ -725,15 +736,14 @@ extern "C" int nkb_bn_fwd(const void* x, const void* gamma, const void* beta, co
   dim3 grid;
   bn_sums_dims(M, C, cx, grid);
   std::lock_guard<std::mutex> order(g_bn_order);
-  bn_sums_kernel<0><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), nullptr, nullptr,
-                                         nullptr, acc, M, C, cx);
-  bn_finalize_kernel<<<(C + 127) / 128, 128, 0, s>>>(acc, stats, run_mean, run_var, M, C, eps,
-                                                     momentum);
-  bn_apply_kernel<<<grid, 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(x), stats, stats + C, -1.f,
-      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
-      static_cast<const __nv_bfloat16*>(res),
-      static_cast<__nv_bfloat16*>(y), static_cast<uint8_t*>(mask), M, C, cx, relu);
+  launch_dep(bn_sums_kernel<0>, grid, 256, 0, s, static_cast<const __nv_bfloat16*>(x), nullptr,
+             nullptr, nullptr, acc, M, C, cx);
+  launch_dep(bn_finalize_kernel, (C + 127) / 128, 128, 0, s, acc, stats, run_mean, run_var, M, C,
+             eps, momentum);
+  launch_dep(bn_apply_kernel, grid, 256, 0, s, static_cast<const __nv_bfloat16*>(x), stats,
+             stats + C, -1.f, static_cast<const __nv_bfloat16*>(gamma),
+             static_cast<const __nv_bfloat16*>(beta), static_cast<const __nv_bfloat16*>(res),
+             static_cast<__nv_bfloat16*>(y), static_cast<uint8_t*>(mask), M, C, cx, relu);
   return (int)cudaGetLastError();
 }
 
@@ -744,11 +754,11 @@ extern "C" int nkb_bn_apply(const void* x, const float* stats, const void* gamma
   int cx;
   dim3 grid;
   bn_sums_dims(M, C, cx, grid);
-  bn_apply_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), stats, stats + C, -1.f,
-      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
-      static_cast<const __nv_bfloat16*>(res),
-      static_cast<__nv_bfloat16*>(y), nullptr, M, C, cx, relu);
+  launch_dep(bn_apply_kernel, grid, 256, 0, static_cast<cudaStream_t>(stream),
+             static_cast<const __nv_bfloat16*>(x), stats, stats + C, -1.f,
+             static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
+             static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(y), nullptr, M, C,
+             cx, relu);
   return (int)cudaGetLastError();
 }
 
@@ -761,11 +771,11 @@ extern "C" int nkb_bn_eval(const void* x, const float* run_mean, const float* ru
   int cx;
   dim3 grid;
   bn_sums_dims(M, C, cx, grid);
-  bn_apply_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), run_mean, run_var, eps,
-      static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
-      static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(y), nullptr, M, C, cx,
-      relu);
+  launch_dep(bn_apply_kernel, grid, 256, 0, static_cast<cudaStream_t>(stream),
+             static_cast<const __nv_bfloat16*>(x), run_mean, run_var, eps,
+             static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta),
+             static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(y), nullptr, M, C,
+             cx, relu);
   return (int)cudaGetLastError();
 }
 
@@ -783,17 +793,16 @@ extern "C" int nkb_bn_bwd(const void* dy, const void* x, const void* mask, const
   dim3 grid;
   bn_sums_dims(M, C, cx, grid);
   std::lock_guard<std::mutex> order(g_bn_order);
-  bn_sums_kernel<1><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(dy),
-                                         static_cast<const __nv_bfloat16*>(x),
-                                         static_cast<const uint8_t*>(mask), stats, acc, M, C,
-                                         cx);
-  bn_bwd_apply_kernel<<<grid, 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
-      static_cast<const uint8_t*>(mask), stats, acc, static_cast<const __nv_bfloat16*>(gamma),
-      static_cast<__nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(dres), M, C, cx);
-  bn_param_grad_kernel<<<(C + 127) / 128, 128, 0, s>>>(acc, static_cast<__nv_bfloat16*>(dgamma),
-                                                       static_cast<__nv_bfloat16*>(dbeta), C,
-                                                       acc_g, acc_b);
+  launch_dep(bn_sums_kernel<1>, grid, 256, 0, s, static_cast<const __nv_bfloat16*>(dy),
+             static_cast<const __nv_bfloat16*>(x), static_cast<const uint8_t*>(mask), stats, acc, M,
+             C, cx);
+  launch_dep(bn_bwd_apply_kernel, grid, 256, 0, s, static_cast<const __nv_bfloat16*>(dy),
+             static_cast<const __nv_bfloat16*>(x), static_cast<const uint8_t*>(mask), stats, acc,
+             static_cast<const __nv_bfloat16*>(gamma), static_cast<__nv_bfloat16*>(dx),
+             static_cast<__nv_bfloat16*>(dres), M, C, cx);
+  launch_dep(bn_param_grad_kernel, (C + 127) / 128, 128, 0, s, acc,
+             static_cast<__nv_bfloat16*>(dgamma), static_cast<__nv_bfloat16*>(dbeta), C, acc_g,
+             acc_b);
   return (int)cudaGetLastError();
 }
 
@@ -801,10 +810,9 @@ extern "C" int nkb_maxpool3x3s2_fwd(const void* x, void* y, void* idx, int N, in
                                     void* stream) {
   if (C % 8) return -3;
   const int Ho = (H + 2 - 3) / 2 + 1, Wo = (W + 2 - 3) / 2 + 1;
-  maxpool_fwd_kernel<<<conv_grid((long long)N * Ho * Wo * (C / 8), 256), 256, 0,
-                       static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y),
-      static_cast<uint8_t*>(idx), N, H, W, C, Ho, Wo);
+  launch_dep(maxpool_fwd_kernel, conv_grid((long long)N * Ho * Wo * (C / 8), 256), 256, 0,
+             static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x),
+             static_cast<__nv_bfloat16*>(y), static_cast<uint8_t*>(idx), N, H, W, C, Ho, Wo);
   return (int)cudaGetLastError();
 }
 
@@ -813,25 +821,25 @@ extern "C" int nkb_maxpool3x3s2_bwd(const void* dy, const void* idx, void* dx, i
   if (C % 8) return -3;
   const int Ho = (H + 2 - 3) / 2 + 1, Wo = (W + 2 - 3) / 2 + 1;
   const long long quads = (long long)N * ((H + 1) / 2) * ((W + 1) / 2) * (C / 8);
-  maxpool_bwd_kernel<<<conv_grid(quads, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const uint8_t*>(idx),
-      static_cast<__nv_bfloat16*>(dx), N, H, W, C, Ho, Wo);
+  launch_dep(maxpool_bwd_kernel, conv_grid(quads, 256), 256, 0, static_cast<cudaStream_t>(stream),
+             static_cast<const __nv_bfloat16*>(dy), static_cast<const uint8_t*>(idx),
+             static_cast<__nv_bfloat16*>(dx), N, H, W, C, Ho, Wo);
   return (int)cudaGetLastError();
 }
 
 extern "C" int nkb_avgpool_fwd(const void* x, void* y, int N, int HW, int C, void* stream) {
   if (C % 8) return -3;
-  avgpool_fwd_kernel<<<conv_grid((long long)N * (C / 8), 256), 256, 0,
-                       static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), N, HW, C);
+  launch_dep(avgpool_fwd_kernel, conv_grid((long long)N * (C / 8), 256), 256, 0,
+             static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x),
+             static_cast<__nv_bfloat16*>(y), N, HW, C);
   return (int)cudaGetLastError();
 }
 
 extern "C" int nkb_avgpool_bwd(const void* dy, void* dx, int N, int HW, int C, void* stream) {
   if (C % 8) return -3;
-  avgpool_bwd_kernel<<<conv_grid((long long)N * HW * (C / 8), 256), 256, 0,
-                       static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx), N, HW, C);
+  launch_dep(avgpool_bwd_kernel, conv_grid((long long)N * HW * (C / 8), 256), 256, 0,
+             static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(dy),
+             static_cast<__nv_bfloat16*>(dx), N, HW, C);
   return (int)cudaGetLastError();
 }
 

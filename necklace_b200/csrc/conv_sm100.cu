@@ -156,6 +156,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!grid_dep_wait()) return;
   const int boxes = g.nbw * g.nbh * g.nbn;
   const int tiles = g.tiles_m * g.tiles_n;
   const int units = KIND == CV_WGRAD ? tiles * g.split : tiles;
@@ -241,6 +242,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
       }
+      grid_dep_trigger();
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -480,6 +482,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 __global__ void __launch_bounds__(256)
 conv_dw_reduce_kernel(const float* __restrict__ ws, int S, long long n4,
                       __nv_bfloat16* __restrict__ dw, int accumulate) {
+  if (!grid_dep_begin()) return;
   __shared__ float4 sh[4][64];
   const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
   const long long i = (long long)blockIdx.x * 64 + tx;
@@ -573,7 +576,7 @@ static int launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap&
   static bool done[64];
   if (int e = allow_smem(kern, ConvCfg<KIND, BN>::SMEM, done)) return e;
   const int sms = num_sms();
-  kern<<<units < sms ? units : sms, CV_THREADS, ConvCfg<KIND, BN>::SMEM, s>>>(a, b, o, g);
+  launch_dep(kern, units < sms ? units : sms, CV_THREADS, ConvCfg<KIND, BN>::SMEM, s, a, b, o, g);
   return (int)cudaGetLastError();
 }
 
@@ -783,8 +786,8 @@ extern "C" int nkb_conv_wgrad(const void* x, const void* dy, void* dw, float* ws
                  : launch<CV_WGRAD, 256>(a, b, a, g, units, s);
   if (rc) return rc;
   const long long n4 = (long long)Cout * g.ntaps * C / 4;
-  conv_dw_reduce_kernel<<<(unsigned)((n4 + 63) / 64), 256, 0, s>>>(
-      ws, g.split, n4, static_cast<__nv_bfloat16*>(dw), accumulate);
+  launch_dep(conv_dw_reduce_kernel, (unsigned)((n4 + 63) / 64), 256, 0, s, ws, g.split, n4,
+             static_cast<__nv_bfloat16*>(dw), accumulate);
   return (int)cudaGetLastError();
 }
 

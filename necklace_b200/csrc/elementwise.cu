@@ -14,6 +14,7 @@ namespace nkb {
 __global__ void __launch_bounds__(256)
 rope_kernel(__nv_bfloat16* __restrict__ qkv, int T, int S, int H, int D, float base, float dir,
             int pos_offset) {
+  if (!grid_dep_begin()) return;
   const int half = D / 2;
   const int groups = half / 8;
   const long long total = (long long)T * 2 * H * groups;
@@ -54,6 +55,7 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long long T,
                   int F) {
+  if (!grid_dep_begin()) return;
   const int f8 = F / 8;
   const long long total = T * f8;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -76,6 +78,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
                   __nv_bfloat16* __restrict__ dgu, long long T, int F) {
+  if (!grid_dep_begin()) return;
   const int f8 = F / 8;
   const long long total = T * f8;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -116,24 +119,24 @@ extern "C" int nkb_rope(void* qkv, int T, int S, int H, int D, float base, int b
                         int pos_offset, void* stream) {
   if (D % 16) return -3;
   long long items = (long long)T * 2 * H * (D / 16);
-  rope_kernel<<<ew_grid(items), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(qkv), T, S, H, D, base, backward ? -1.f : 1.f, pos_offset);
+  launch_dep(rope_kernel, ew_grid(items), 256, 0, static_cast<cudaStream_t>(stream),
+             static_cast<__nv_bfloat16*>(qkv), T, S, H, D, base, backward ? -1.f : 1.f, pos_offset);
   return (int)cudaGetLastError();
 }
 
 extern "C" int nkb_swiglu_fwd(const void* gu, void* h, long long T, int F, void* stream) {
   if (F % 8) return -3;
-  swiglu_fwd_kernel<<<ew_grid(T * (F / 8)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), T, F);
+  launch_dep(swiglu_fwd_kernel, ew_grid(T * (F / 8)), 256, 0, static_cast<cudaStream_t>(stream),
+             static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), T, F);
   return (int)cudaGetLastError();
 }
 
 extern "C" int nkb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long long T, int F,
                               void* stream) {
   if (F % 8) return -3;
-  swiglu_bwd_kernel<<<ew_grid(T * (F / 8)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh),
-      static_cast<__nv_bfloat16*>(dgu), T, F);
+  launch_dep(swiglu_bwd_kernel, ew_grid(T * (F / 8)), 256, 0, static_cast<cudaStream_t>(stream),
+             static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh),
+             static_cast<__nv_bfloat16*>(dgu), T, F);
   return (int)cudaGetLastError();
 }
 

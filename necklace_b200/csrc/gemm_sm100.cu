@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, int S, long long MN, int N, void* out,
                      long long ldc, int c_fp32, int accumulate, float alpha,
                      const float* __restrict__ alpha_dev) {
+  if (!grid_dep_begin()) return;
   constexpr int GROUPS = 256 / LANES;
   __shared__ float4 sh[LANES > 1 ? LANES - 1 : 1][GROUPS];
   if (alpha_dev) alpha *= *alpha_dev;
@@ -939,6 +940,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!grid_dep_wait()) return;
   // The control warpgroup keeps GEMM_CTRL_REGS registers per thread and the epilogue warpgroups take
   // the rest; each setmaxnreg sits inside its own role branch so that no code is reachable
   // from both.
@@ -1003,6 +1005,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         }
       }
+      grid_dep_trigger();
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
@@ -1212,6 +1215,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   cluster_wait();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!grid_dep_wait()) return;
   if (warp < 4) {
     reg_alloc_dec<GEMM_CTRL_REGS>();
   }
@@ -1272,6 +1276,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
           }
         }
       }
+      grid_dep_trigger();
     }
   } else if (warp == 1) {
     if (lane == 0 && leader) {
@@ -1492,7 +1497,10 @@ static int launch_gemm_mode(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm
   if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
   if (tiles < ctas) ctas = tiles;
   g.rs_bn = BN;
-  kern<<<ctas + g.ag_ctas, GEMM_THREADS, smem_bytes, stream>>>(tmA, tmB, g);
+  if constexpr (MODE == 1)  // its copy CTAs take their role before the wait
+    kern<<<ctas + g.ag_ctas, GEMM_THREADS, smem_bytes, stream>>>(tmA, tmB, g);
+  else
+    launch_dep(kern, ctas, GEMM_THREADS, smem_bytes, stream, tmA, tmB, g);
   return (int)cudaGetLastError();
 }
 
@@ -1522,7 +1530,10 @@ static int launch_gemm_pair_mode(const CUtensorMap& tmA, const CUtensorMap& tmB,
   if (2 * tiles < ctas) ctas = 2 * tiles;
   if (ctas < 2) ctas = 2;
   g.rs_bn = 256;
-  kern<<<ctas + g.ag_ctas, GEMM_THREADS, smem_bytes, stream>>>(tmA, tmB, g);
+  if constexpr (MODE == 1)  // its copy CTAs take their role before the wait
+    kern<<<ctas + g.ag_ctas, GEMM_THREADS, smem_bytes, stream>>>(tmA, tmB, g);
+  else
+    launch_dep(kern, ctas, GEMM_THREADS, smem_bytes, stream, tmA, tmB, g);
   return (int)cudaGetLastError();
 }
 
@@ -1563,8 +1574,8 @@ static int gemm_run_splitk(GemmArgs g, const CUtensorMap& tmA, const CUtensorMap
   const long long MN = (long long)g.M * g.N;
   auto reduce = g.split_k > 8 ? splitk_reduce_kernel<4> : splitk_reduce_kernel<1>;
   const int per_block = 4 * 256 / (g.split_k > 8 ? 4 : 1);  // elements
-  reduce<<<(unsigned)((MN + per_block - 1) / per_block), 256, 0, s>>>(
-      g.splitk_ws, g.split_k, MN, g.N, g.C, g.ldc, g.c_fp32, g.accumulate, g.alpha, g.alpha_dev);
+  launch_dep(reduce, (unsigned)((MN + per_block - 1) / per_block), 256, 0, s, g.splitk_ws,
+             g.split_k, MN, g.N, g.C, g.ldc, g.c_fp32, g.accumulate, g.alpha, g.alpha_dev);
   return (int)cudaGetLastError();
 }
 

@@ -53,6 +53,7 @@ __device__ __forceinline__ void block_online_reduce(float& m, float& s, float* s
 __global__ void __launch_bounds__(1024)
 loss_mean_kernel(const float* __restrict__ losses, const long long* __restrict__ targets, int T,
                  float* __restrict__ loss, float* __restrict__ n_valid) {
+  if (!grid_dep_begin()) return;
   __shared__ float sh_s[32];
   __shared__ int sh_n[32];
   float s = 0.f;
@@ -86,6 +87,7 @@ loss_mean_kernel(const float* __restrict__ losses, const long long* __restrict__
 
 __global__ void loss_corr_kernel(const float* __restrict__ dloss, const float* __restrict__ n_valid,
                                  float T, float* __restrict__ out) {
+  if (!grid_dep_begin()) return;
   *out = *dloss * __fdiv_rn(T, *n_valid);
 }
 
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(CE_THREADS)
 ce_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
           float* __restrict__ out, const float* __restrict__ stats_g, int T, int V, long long ld,
           int vocab_start, float grad_scale, int use_smem) {
+  if (!grid_dep_begin()) return;
   extern __shared__ __align__(16) uint8_t ce_smem[];
   __shared__ float sh_m[32], sh_s[32];
   __nv_bfloat16* srow = reinterpret_cast<__nv_bfloat16*>(ce_smem);
@@ -209,6 +212,7 @@ __global__ void embed_fwd_kernel(const long long* __restrict__ idx,
                                  const __nv_bfloat16* __restrict__ wpe,
                                  __nv_bfloat16* __restrict__ out, int T, int S, int C,
                                  int vocab_start, int vocab_rows) {
+  if (!grid_dep_begin()) return;
   const int t = blockIdx.x;
   if (!NKB_IN_BOUNDS(t, T)) return;
   const long long id = idx[t] - vocab_start;
@@ -237,6 +241,7 @@ __global__ void embed_bwd_wte_kernel(const long long* __restrict__ idx,
                                      const __nv_bfloat16* __restrict__ dout,
                                      __nv_bfloat16* __restrict__ dwte, int T, int C,
                                      int vocab_start, int vocab_rows) {
+  if (!grid_dep_begin()) return;
   const int t = blockIdx.x;
   const long long id = idx[t] - vocab_start;
   if (id < 0 || id >= vocab_rows) return;
@@ -248,6 +253,7 @@ __global__ void embed_bwd_wte_kernel(const long long* __restrict__ idx,
 // dwpe[s, c] += sum_b dout[b*S + s, c]
 __global__ void embed_bwd_wpe_kernel(const __nv_bfloat16* __restrict__ dout,
                                      __nv_bfloat16* __restrict__ dwpe, int T, int S, int C) {
+  if (!grid_dep_begin()) return;
   const int s = blockIdx.x;
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
     float acc = 0.f;
@@ -272,8 +278,8 @@ static int launch_ce(void* logits, const long long* targets, float* out, const f
         if (int e = allow_smem(ce_kernel<MODE>, 200 * 1024, done)) return e;
     }
   }
-  ce_kernel<MODE><<<T, CE_THREADS, smem, s>>>(static_cast<__nv_bfloat16*>(logits), targets, out,
-                                              stats_g, T, V, ld, vocab_start, grad_scale, use_smem);
+  launch_dep(ce_kernel<MODE>, T, CE_THREADS, smem, s, static_cast<__nv_bfloat16*>(logits), targets,
+             out, stats_g, T, V, ld, vocab_start, grad_scale, use_smem);
   return (int)cudaGetLastError();
 }
 
@@ -302,24 +308,25 @@ extern "C" int nkb_ce_grad(void* logits, const long long* targets, const float* 
 extern "C" int nkb_loss_mean(const float* losses, const long long* targets, int T, float* loss,
                              float* n_valid, void* stream) {
   if (T <= 0) return -2;
-  loss_mean_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(losses, targets, T, loss,
-                                                                     n_valid);
+  launch_dep(loss_mean_kernel, 1, 1024, 0, static_cast<cudaStream_t>(stream), losses, targets, T,
+             loss, n_valid);
   return (int)cudaGetLastError();
 }
 
 // out = dloss * T / n_valid
 extern "C" int nkb_loss_corr(const float* dloss, const float* n_valid, int T, float* out,
                              void* stream) {
-  loss_corr_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(dloss, n_valid, (float)T, out);
+  launch_dep(loss_corr_kernel, 1, 1, 0, static_cast<cudaStream_t>(stream), dloss, n_valid, (float)T,
+             out);
   return (int)cudaGetLastError();
 }
 
 extern "C" int nkb_embed_fwd(const long long* idx, const void* wte, const void* wpe, void* out,
                              int T, int S, int C, int vocab_start, int vocab_rows, void* stream) {
   if (C % 8) return -3;
-  embed_fwd_kernel<<<T, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      idx, static_cast<const __nv_bfloat16*>(wte), static_cast<const __nv_bfloat16*>(wpe),
-      static_cast<__nv_bfloat16*>(out), T, S, C, vocab_start, vocab_rows);
+  launch_dep(embed_fwd_kernel, T, 128, 0, static_cast<cudaStream_t>(stream), idx,
+             static_cast<const __nv_bfloat16*>(wte), static_cast<const __nv_bfloat16*>(wpe),
+             static_cast<__nv_bfloat16*>(out), T, S, C, vocab_start, vocab_rows);
   return (int)cudaGetLastError();
 }
 extern "C" int nkb_embed_bwd(const long long* idx, const void* dout, void* dwte, void* dwpe, int T,
@@ -327,12 +334,11 @@ extern "C" int nkb_embed_bwd(const long long* idx, const void* dout, void* dwte,
   if (C % 2) return -3;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dwte)
-    embed_bwd_wte_kernel<<<T, 128, 0, s>>>(idx, static_cast<const __nv_bfloat16*>(dout),
-                                           static_cast<__nv_bfloat16*>(dwte), T, C, vocab_start,
-                                           vocab_rows);
+    launch_dep(embed_bwd_wte_kernel, T, 128, 0, s, idx, static_cast<const __nv_bfloat16*>(dout),
+               static_cast<__nv_bfloat16*>(dwte), T, C, vocab_start, vocab_rows);
   if (dwpe)
-    embed_bwd_wpe_kernel<<<S, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(dout),
-                                           static_cast<__nv_bfloat16*>(dwpe), T, S, C);
+    launch_dep(embed_bwd_wpe_kernel, S, 256, 0, s, static_cast<const __nv_bfloat16*>(dout),
+               static_cast<__nv_bfloat16*>(dwpe), T, S, C);
   return (int)cudaGetLastError();
 }
 

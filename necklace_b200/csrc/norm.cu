@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(128)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                 const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                 float* __restrict__ stats, int rows, int C, float eps, int rms) {
+  if (!grid_dep_begin()) return;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -95,6 +96,7 @@ norm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ stats,
                    __nv_bfloat16* __restrict__ dx, int rows, int C, int rms,
                    const __nv_bfloat16* __restrict__ dres) {
+  if (!grid_dep_begin()) return;
   // dres (optional): gradient that reaches x along the residual path; added here so that no
   // separate accumulation kernel runs
   const int lane = threadIdx.x & 31;
@@ -181,6 +183,7 @@ norm_bwd_all_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
                     int rows, int C, int rms, int tpr, float* __restrict__ acc,
                     int* __restrict__ ticket, __nv_bfloat16* __restrict__ dw,
                     __nv_bfloat16* __restrict__ db, int accum_w, int accum_b) {
+  if (!grid_dep_begin()) return;
   extern __shared__ __align__(16) float nb_smem[];
   // [2 buffers][warps][ROWS] row sums, then [threads][16] column sums of the groups
   float2* part = reinterpret_cast<float2*>(nb_smem);
@@ -364,11 +367,11 @@ static int launch_bwd_all(const void* dy, const void* x, const void* w, const fl
   size_t smem = sizeof(float2) * 2 * (threads / 32) * ROWS;
   const size_t cols = groups > 1 ? sizeof(float) * 16 * (size_t)(groups - 1) * tpr : 0;
   if (cols > smem) smem = cols;
-  norm_bwd_all_kernel<THREADS, ROWS><<<grid, threads, smem, s>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
-      static_cast<const __nv_bfloat16*>(w), stats, static_cast<__nv_bfloat16*>(dx),
-      static_cast<const __nv_bfloat16*>(dres), rows, C, rms, tpr, acc, ticket,
-      static_cast<__nv_bfloat16*>(dw), static_cast<__nv_bfloat16*>(db), accum_w, accum_b);
+  launch_dep(norm_bwd_all_kernel<THREADS, ROWS>, grid, threads, smem, s,
+             static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+             static_cast<const __nv_bfloat16*>(w), stats, static_cast<__nv_bfloat16*>(dx),
+             static_cast<const __nv_bfloat16*>(dres), rows, C, rms, tpr, acc, ticket,
+             static_cast<__nv_bfloat16*>(dw), static_cast<__nv_bfloat16*>(db), accum_w, accum_b);
   return (int)cudaGetLastError();
 }
 
@@ -390,6 +393,7 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restr
               const float* __restrict__ stats, float* __restrict__ acc, int rows, int C,
               long long ld, int rms, int* __restrict__ tickets, __nv_bfloat16* __restrict__ out,
               int accumulate) {
+  if (!grid_dep_begin()) return;
   // ring slots [which: dy | x][slot][thread] (16 bytes each); the reduction buffer reuses it
   extern __shared__ __align__(16) uint8_t colsum_smem[];  // COLSUM_SMEM_BYTES, dynamic
   uint4 (*ring)[COLSUM_RING][256] = reinterpret_cast<uint4 (*)[COLSUM_RING][256]>(colsum_smem);
@@ -497,6 +501,7 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restr
 
 __global__ void f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst,
                                    long long n, int accumulate) {
+  if (!grid_dep_begin()) return;
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (; i < n; i += stride) {
@@ -509,19 +514,18 @@ __global__ void f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16*
 template <int NCH>
 static int launch_fwd(const void* x, const void* w, const void* b, void* y, float* stats, int rows,
                       int C, float eps, int rms, cudaStream_t s) {
-  norm_fwd_kernel<NCH><<<(rows + 3) / 4, 128, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),
-      static_cast<const __nv_bfloat16*>(b), static_cast<__nv_bfloat16*>(y), stats, rows, C, eps,
-      rms);
+  launch_dep(norm_fwd_kernel<NCH>, (rows + 3) / 4, 128, 0, s, static_cast<const __nv_bfloat16*>(x),
+             static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(b),
+             static_cast<__nv_bfloat16*>(y), stats, rows, C, eps, rms);
   return (int)cudaGetLastError();
 }
 template <int NCH>
 static int launch_bwd(const void* dy, const void* x, const void* w, const float* stats, void* dx,
                       int rows, int C, int rms, const void* dres, cudaStream_t s) {
-  norm_bwd_dx_kernel<NCH><<<(rows + 3) / 4, 128, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
-      static_cast<const __nv_bfloat16*>(w), stats, static_cast<__nv_bfloat16*>(dx), rows, C, rms,
-      static_cast<const __nv_bfloat16*>(dres));
+  launch_dep(norm_bwd_dx_kernel<NCH>, (rows + 3) / 4, 128, 0, s,
+             static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+             static_cast<const __nv_bfloat16*>(w), stats, static_cast<__nv_bfloat16*>(dx), rows, C,
+             rms, static_cast<const __nv_bfloat16*>(dres));
   return (int)cudaGetLastError();
 }
 
@@ -608,9 +612,10 @@ extern "C" int nkb_colsum(const void* dy, const void* x, const float* stats, flo
   int gx = (C + 255) / 256;
   int gy = colsum_row_splits(gx, rows);
   if (colsum_configure()) return -6;
-  colsum_kernel<<<dim3(gx, gy), 256, nkb::COLSUM_SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, acc, rows,
-      C, ld, rms, nullptr, nullptr, 0);
+  launch_dep(colsum_kernel, dim3(gx, gy), 256, nkb::COLSUM_SMEM_BYTES,
+             static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(dy),
+             static_cast<const __nv_bfloat16*>(x), stats, acc, rows, C, ld, rms, nullptr, nullptr,
+             0);
   return (int)cudaGetLastError();
 }
 
@@ -623,9 +628,9 @@ extern "C" int nkb_colsum_fused(const void* dy, float* acc, int* tickets, void* 
   int gx = (C + 255) / 256;
   int gy = colsum_row_splits(gx, rows);
   if (colsum_configure()) return -6;
-  colsum_kernel<<<dim3(gx, gy), 256, nkb::COLSUM_SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(dy), nullptr, nullptr, acc, rows, C, ld, 0, tickets,
-      static_cast<__nv_bfloat16*>(out), accumulate);
+  launch_dep(colsum_kernel, dim3(gx, gy), 256, nkb::COLSUM_SMEM_BYTES,
+             static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(dy), nullptr,
+             nullptr, acc, rows, C, ld, 0, tickets, static_cast<__nv_bfloat16*>(out), accumulate);
   return (int)cudaGetLastError();
 }
 
@@ -634,8 +639,8 @@ extern "C" int nkb_f32_to_bf16(const float* src, void* dst, long long n, int acc
   if (n <= 0) return 0;
   int blocks = (int)((n + 255) / 256);
   if (blocks > 148 * 8) blocks = 148 * 8;
-  f32_to_bf16_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      src, static_cast<__nv_bfloat16*>(dst), n, accumulate);
+  launch_dep(f32_to_bf16_kernel, blocks, 256, 0, static_cast<cudaStream_t>(stream), src,
+             static_cast<__nv_bfloat16*>(dst), n, accumulate);
   return (int)cudaGetLastError();
 }
 

@@ -24,6 +24,7 @@ adam_flat_kernel(float* __restrict__ master, float* __restrict__ m, float* __res
                  const void* __restrict__ grad, int grad_fp32, __nv_bfloat16* __restrict__ pbf,
                  long long n, float lr, float b1, float b2, float eps, float wd, float c1,
                  float c2, float gscale, const float* __restrict__ hyper) {
+  if (!grid_dep_begin()) return;
   if (hyper) { lr = hyper[0]; c1 = hyper[1]; c2 = hyper[2]; gscale *= hyper[4]; }
   const long long n4 = n >> 2;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(256)
 sgd_flat_kernel(float* __restrict__ master, float* __restrict__ mom, const void* __restrict__ grad,
                 int grad_fp32, __nv_bfloat16* __restrict__ pbf, long long n, float lr, float mu,
                 float wd, float gscale, int first_step, const float* __restrict__ hyper) {
+  if (!grid_dep_begin()) return;
   if (hyper) { lr = hyper[0]; gscale *= hyper[4]; }
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -127,6 +129,7 @@ __device__ __forceinline__ void load8(const void* p, long long i, int fp32, floa
 __global__ void __launch_bounds__(256)
 quant2_flat_kernel(const void* __restrict__ g, int g_fp32, float* __restrict__ residual,
                    uint32_t* __restrict__ codes, long long n, float thr) {
+  if (!grid_dep_begin()) return;
   const long long halves = ((n + 15) >> 4) << 1;
   const long long stride = (long long)gridDim.x * blockDim.x;
   // the number of half words is even and so is the stride: both lanes of a pair take part
@@ -161,6 +164,7 @@ quant2_flat_kernel(const void* __restrict__ g, int g_fp32, float* __restrict__ r
 __global__ void __launch_bounds__(256)
 dequant2_flat_kernel(const uint32_t* __restrict__ codes, void* __restrict__ out, int out_fp32,
                      long long n, float thr, float scale, int accumulate, int vec) {
+  if (!grid_dep_begin()) return;
   const long long halves = (n + 7) >> 3;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x; h < halves; h += stride) {
@@ -203,6 +207,7 @@ dequant2_flat_kernel(const uint32_t* __restrict__ codes, void* __restrict__ out,
 __global__ void __launch_bounds__(256)
 quant2_matrix_kernel(const float* __restrict__ A, uint32_t* __restrict__ codes,
                      float* __restrict__ R, int n, int ncol, float thr) {
+  if (!grid_dep_begin()) return;
   const long long nwords = (long long)((n + 15) / 16) * ncol;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += stride) {
@@ -237,6 +242,7 @@ quant2_matrix_kernel(const float* __restrict__ A, uint32_t* __restrict__ codes,
 __global__ void __launch_bounds__(256)
 dequant2_matrix_kernel(float* __restrict__ A, const uint32_t* __restrict__ codes, int n, int ncol,
                        float thr) {
+  if (!grid_dep_begin()) return;
   const long long nwords = (long long)((n + 15) / 16) * ncol;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += stride) {
@@ -253,6 +259,7 @@ dequant2_matrix_kernel(float* __restrict__ A, const uint32_t* __restrict__ codes
 __global__ void __launch_bounds__(256)
 scale_cast_kernel(const void* __restrict__ src, int src_fp32, void* __restrict__ dst, int dst_fp32,
                   long long n, float scale, int accumulate) {
+  if (!grid_dep_begin()) return;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     float v = load_as_float(src, i, src_fp32) * scale;
@@ -268,6 +275,7 @@ scale_cast_kernel(const void* __restrict__ src, int src_fp32, void* __restrict__
 
 __global__ void __launch_bounds__(256)
 sumsq_kernel(const void* __restrict__ src, int src_fp32, long long n, float* __restrict__ out) {
+  if (!grid_dep_begin()) return;
   __shared__ float sh[8];
   float acc = 0.f;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -309,6 +317,7 @@ static int grid_for(long long work_items) {
 // hyper[4] = min(1, max_norm / (sqrt(sumsq) * gscale)): the multiplier that clips the global
 // gradient norm; applied inside the optimizer kernels.
 __global__ void clip_coef_kernel(float* hyper, const float* sumsq, float max_norm, float gscale) {
+  if (!grid_dep_begin()) return;
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     const float nrm = sqrtf(sumsq[0]) * gscale;
     hyper[4] = fminf(1.f, max_norm / (nrm + 1e-6f));
@@ -322,6 +331,7 @@ __global__ void clip_coef_kernel(float* hyper, const float* sumsq, float max_nor
 // not of when the host last rewrote a staging buffer (the host may enqueue many steps, or
 // replay a CUDA graph, far ahead of the device).
 __global__ void hyper_advance_kernel(float* hyper, float beta1, float beta2) {
+  if (!grid_dep_begin()) return;
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     const float t = hyper[3] + 1.f;
     hyper[3] = t;
@@ -337,12 +347,14 @@ using namespace nkb;
 
 extern "C" int nkb_clip_coef(float* hyper, const float* sumsq, float max_norm, float gscale,
                              void* stream) {
-  clip_coef_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(hyper, sumsq, max_norm, gscale);
+  launch_dep(clip_coef_kernel, 1, 32, 0, static_cast<cudaStream_t>(stream), hyper, sumsq, max_norm,
+             gscale);
   return (int)cudaGetLastError();
 }
 
 extern "C" int nkb_hyper_advance(float* hyper, float beta1, float beta2, void* stream) {
-  hyper_advance_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(hyper, beta1, beta2);
+  launch_dep(hyper_advance_kernel, 1, 32, 0, static_cast<cudaStream_t>(stream), hyper, beta1,
+             beta2);
   return (int)cudaGetLastError();
 }
 
@@ -357,9 +369,9 @@ extern "C" int nkb_adam_flat(float* master, float* m, float* v, const void* grad
     return -3;
   if (reinterpret_cast<uintptr_t>(grad) & (grad_fp32 ? 15 : 7)) return -3;
   if (param_bf16 && (reinterpret_cast<uintptr_t>(param_bf16) & 7)) return -3;
-  adam_flat_kernel<<<grid_for(n / 4 + 1), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      master, m, v, grad, grad_fp32, static_cast<__nv_bfloat16*>(param_bf16), n, lr, beta1, beta2,
-      eps, weight_decay, bias_c1, bias_c2, grad_scale, hyper_dev);
+  launch_dep(adam_flat_kernel, grid_for(n / 4 + 1), 256, 0, static_cast<cudaStream_t>(stream),
+             master, m, v, grad, grad_fp32, static_cast<__nv_bfloat16*>(param_bf16), n, lr, beta1,
+             beta2, eps, weight_decay, bias_c1, bias_c2, grad_scale, hyper_dev);
   return (int)cudaGetLastError();
 }
 
@@ -368,9 +380,9 @@ extern "C" int nkb_sgd_flat(float* master, float* mom, const void* grad, int gra
                             float weight_decay, float grad_scale, int first_step,
                             const float* hyper_dev, void* stream) {
   if (n <= 0) return 0;
-  sgd_flat_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      master, mom, grad, grad_fp32, static_cast<__nv_bfloat16*>(param_bf16), n, lr, momentum,
-      weight_decay, grad_scale, first_step, hyper_dev);
+  launch_dep(sgd_flat_kernel, grid_for(n), 256, 0, static_cast<cudaStream_t>(stream), master, mom,
+             grad, grad_fp32, static_cast<__nv_bfloat16*>(param_bf16), n, lr, momentum,
+             weight_decay, grad_scale, first_step, hyper_dev);
   return (int)cudaGetLastError();
 }
 
@@ -378,44 +390,44 @@ extern "C" int nkb_quant2_flat(const void* g, int g_fp32, float* residual, uint3
                                long long n, float thr, void* stream) {
   if (n <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(residual)) & 15) return -3;
-  quant2_flat_kernel<<<grid_for((n + 15) / 16 * 2), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      g, g_fp32, residual, codes, n, thr);
+  launch_dep(quant2_flat_kernel, grid_for((n + 15) / 16 * 2), 256, 0,
+             static_cast<cudaStream_t>(stream), g, g_fp32, residual, codes, n, thr);
   return (int)cudaGetLastError();
 }
 extern "C" int nkb_dequant2_flat(const uint32_t* codes, void* out, int out_fp32, long long n,
                                  float thr, float scale, int accumulate, void* stream) {
   if (n <= 0) return 0;
   const int vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-  dequant2_flat_kernel<<<grid_for((n + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      codes, out, out_fp32, n, thr, scale, accumulate, vec);
+  launch_dep(dequant2_flat_kernel, grid_for((n + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream),
+             codes, out, out_fp32, n, thr, scale, accumulate, vec);
   return (int)cudaGetLastError();
 }
 extern "C" int nkb_quant2_matrix(const float* A, uint32_t* codes, float* R, int n, int ncol,
                                  float thr, void* stream) {
   if (n <= 0 || ncol <= 0) return 0;
-  quant2_matrix_kernel<<<grid_for((long long)((n + 15) / 16) * ncol), 256, 0,
-                         static_cast<cudaStream_t>(stream)>>>(A, codes, R, n, ncol, thr);
+  launch_dep(quant2_matrix_kernel, grid_for((long long)((n + 15) / 16) * ncol), 256, 0,
+             static_cast<cudaStream_t>(stream), A, codes, R, n, ncol, thr);
   return (int)cudaGetLastError();
 }
 extern "C" int nkb_dequant2_matrix(float* A, const uint32_t* codes, int n, int ncol, float thr,
                                    void* stream) {
   if (n <= 0 || ncol <= 0) return 0;
-  dequant2_matrix_kernel<<<grid_for((long long)((n + 15) / 16) * ncol), 256, 0,
-                           static_cast<cudaStream_t>(stream)>>>(A, codes, n, ncol, thr);
+  launch_dep(dequant2_matrix_kernel, grid_for((long long)((n + 15) / 16) * ncol), 256, 0,
+             static_cast<cudaStream_t>(stream), A, codes, n, ncol, thr);
   return (int)cudaGetLastError();
 }
 extern "C" int nkb_scale_cast(const void* src, int src_fp32, void* dst, int dst_fp32, long long n,
                               float scale, int accumulate, void* stream) {
   if (n <= 0) return 0;
-  scale_cast_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      src, src_fp32, dst, dst_fp32, n, scale, accumulate);
+  launch_dep(scale_cast_kernel, grid_for(n), 256, 0, static_cast<cudaStream_t>(stream), src,
+             src_fp32, dst, dst_fp32, n, scale, accumulate);
   return (int)cudaGetLastError();
 }
 extern "C" int nkb_sumsq(const void* src, int src_fp32, long long n, float* out_accum,
                          void* stream) {
   if (n <= 0) return 0;
-  sumsq_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(src, src_fp32, n,
-                                                                          out_accum);
+  launch_dep(sumsq_kernel, grid_for(n), 256, 0, static_cast<cudaStream_t>(stream), src, src_fp32, n,
+             out_accum);
   return (int)cudaGetLastError();
 }
 
