@@ -167,13 +167,41 @@ norm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // as fit 512 threads, one CTA per SM: each adds its columns to the fp32 accumulator once
 // and the last one (ticket) writes the bf16 gradients and leaves both at zero.
 // Bound by memory: dy, x, dres in, dx out.  With a kernel for dx and one for the column sums, which
-// read dy and x again: 8192 x 1024 15.6 + 12.8 us, 4096 x 4096 47.5 + 32.1 us, 512 x 256 2.1 + 4.8 us;
-// now 24.0, 53.7 and 6.3 us.
+// read dy and x again: 8192 x 1024 15.6 + 12.8 us, 4096 x 4096 47.5 + 32.1 us, 512 x 256 2.1 + 4.8 us.
+// In one, the 41 instructions per value set the pace (48 % of the issue slots with a quarter of the
+// warps); with packed pairs, sums that halve what a lane carries at every exchange and the two factors
+// kept between their uses: 8192 x 1024 21.0 -> 16.7 us, 4096 x 4096 41.6 -> 30.3, 4001 x 5120
+// 75.3 -> 70.8, 512 x 256 6.0.
 constexpr int NB_MAX_C = 8192;
 __device__ __forceinline__ void nb_red_add_v4(float* p, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
                "f"(d)
                : "memory");
+}
+// The warp's sums of s1 and s2 of every row go to out[row * pitch] (x, y).  Every exchange halves
+// the values that a lane still carries: 6 shuffles for two rows, where one sum after the other
+// takes 20.
+template <int ROWS>
+__device__ __forceinline__ void nb_warp_sums(const float* s1, const float* s2, int lane, float2* out,
+                                             int pitch) {
+  static_assert(ROWS == 1 || ROWS == 2, "rows per batch");
+  float a, b;  // s1 and s2 of the lane's row
+  if constexpr (ROWS == 2) {
+    const bool up = lane & 16;  // lanes 16 and up take the second row
+    a = (up ? s1[1] : s1[0]) + __shfl_xor_sync(0xffffffffu, up ? s1[0] : s1[1], 16);
+    b = (up ? s2[1] : s2[0]) + __shfl_xor_sync(0xffffffffu, up ? s2[0] : s2[1], 16);
+  } else {
+    a = s1[0];
+    b = s2[0];
+  }
+  const bool second = lane & 8;  // of the two sums
+  float v = (second ? b : a) + __shfl_xor_sync(0xffffffffu, second ? a : b, 8);
+  if constexpr (ROWS == 1) v += __shfl_xor_sync(0xffffffffu, v, 16);
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  if ((lane & 7) == 0 && (ROWS == 2 || lane < 16))
+    reinterpret_cast<float*>(out + (ROWS == 2 ? lane >> 4 : 0) * pitch)[second] = v;
 }
 template <int THREADS, int ROWS>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -194,18 +222,14 @@ norm_bwd_all_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
   const int col = t * 8;
   const bool on = col < C;
   const float inv_c = 1.f / (float)C;
-  float wf[8], sw[8], sb[8];
+  f32x2_t wf[4], sw2[4], sb2[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) wf[j] = sw[j] = sb[j] = 0.f;
+  for (int j = 0; j < 4; ++j) wf[j] = sw2[j] = sb2[j] = f2_pack(0.f, 0.f);
   if (on) {
     const uint4 v = __ldg(reinterpret_cast<const uint4*>(w + col));
     const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = unpack_bf16x2(u[j]);
-      wf[2 * j] = f.x;
-      wf[2 * j + 1] = f.y;
-    }
+    for (int j = 0; j < 4; ++j) wf[j] = f2_from_bf16x2(u[j]);
   }
   int buf = 0;
   const int step = gridDim.x * groups * ROWS;
@@ -236,54 +260,67 @@ norm_bwd_all_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
     float mn[ROWS], sn[ROWS];
     fetch(row0 + step, xn, gn, rn, mn, sn);  // the next batch is on its way meanwhile
     float2* mine = part + (size_t)(buf * warps + grp * wpg) * ROWS;
+    // dy w and the normalised x of pair j of row r; kept between the two uses where there are
+    // registers for it (the form with 64 of them spilled: 4001 x 5120 took 78 us for 71)
+    constexpr bool KEEP = THREADS <= 512;
+    f32x2_t ka[KEEP ? ROWS : 1][4], kh[KEEP ? ROWS : 1][4];
+    auto norm2 = [&](int r, uint32_t xu) {
+      return f2_mul(f2_add(f2_from_bf16x2(xu), f2_pack(-mean[r], -mean[r])),
+                    f2_pack(rstd[r], rstd[r]));
+    };
+    float s1[ROWS], s2[ROWS];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
       const uint32_t xu[4] = {xv[r].x, xv[r].y, xv[r].z, xv[r].w};
       const uint32_t gu[4] = {gv[r].x, gv[r].y, gv[r].z, gv[r].w};
-      float s1 = 0.f, s2 = 0.f;
-      if (on) {
+      f32x2_t t1 = f2_pack(0.f, 0.f), t2 = t1;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 xf = unpack_bf16x2(xu[j]), gf = unpack_bf16x2(gu[j]);
-          const float h0 = (xf.x - mean[r]) * rstd[r], h1 = (xf.y - mean[r]) * rstd[r];
-          const float a0 = gf.x * wf[2 * j], a1 = gf.y * wf[2 * j + 1];
-          s1 += a0 + a1;
-          s2 += a0 * h0 + a1 * h1;
-          sw[2 * j] += gf.x * h0;
-          sw[2 * j + 1] += gf.y * h1;
-          sb[2 * j] += gf.x;
-          sb[2 * j + 1] += gf.y;
+      for (int j = 0; j < 4; ++j) {  // columns behind the last one have dy = w = 0
+        const f32x2_t g = f2_from_bf16x2(gu[j]);
+        const f32x2_t h = norm2(r, xu[j]), a = f2_mul(g, wf[j]);
+        t1 = f2_add(t1, a);
+        t2 = f2_fma(a, h, t2);
+        sw2[j] = f2_fma(g, h, sw2[j]);
+        sb2[j] = f2_add(sb2[j], g);
+        if constexpr (KEEP) {
+          ka[r][j] = a;
+          kh[r][j] = h;
         }
       }
-      s1 = warp_sum(s1);
-      s2 = warp_sum(s2);
-      if (lane == 0) mine[r * wpg + wg] = make_float2(s1, s2);
+      float lo, hi;
+      f2_unpack(t1, lo, hi);
+      s1[r] = lo + hi;
+      f2_unpack(t2, lo, hi);
+      s2[r] = lo + hi;
     }
+    nb_warp_sums<ROWS>(s1, s2, lane, mine + wg, wpg);
     // one meeting per batch: the next batch writes the other buffer
     if (wpg > 1) asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(tpr) : "memory");
     else __syncwarp();
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
-      float s1 = 0.f, s2 = 0.f;
+      float m1 = 0.f, m2 = 0.f;
       for (int k = 0; k < wpg; ++k) {
         const float2 p = mine[r * wpg + k];
-        s1 += p.x;
-        s2 += p.y;
+        m1 += p.x;
+        m2 += p.y;
       }
-      s1 = rms ? 0.f : s1 * inv_c;
-      s2 *= inv_c;
+      m1 = rms ? 0.f : -m1 * inv_c;
+      m2 *= -inv_c;
       if (on && row0 + r < rows) {
+        const uint32_t ru[4] = {rv[r].x, rv[r].y, rv[r].z, rv[r].w};
+        if (!KEEP)  // (the compiler would keep them all the same)
+          asm volatile("" : "+r"(xv[r].x), "+r"(xv[r].y), "+r"(xv[r].z), "+r"(xv[r].w),
+                            "+r"(gv[r].x), "+r"(gv[r].y), "+r"(gv[r].z), "+r"(gv[r].w));
         const uint32_t xu[4] = {xv[r].x, xv[r].y, xv[r].z, xv[r].w};
         const uint32_t gu[4] = {gv[r].x, gv[r].y, gv[r].z, gv[r].w};
-        const uint32_t ru[4] = {rv[r].x, rv[r].y, rv[r].z, rv[r].w};
+        const f32x2_t n1 = f2_pack(m1, m1), n2 = f2_pack(m2, m2), rs = f2_pack(rstd[r], rstd[r]);
         uint32_t o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float2 xf = unpack_bf16x2(xu[j]), gf = unpack_bf16x2(gu[j]);
-          const float2 rf = unpack_bf16x2(ru[j]);
-          const float h0 = (xf.x - mean[r]) * rstd[r], h1 = (xf.y - mean[r]) * rstd[r];
-          o[j] = pack_bf16x2(rstd[r] * (gf.x * wf[2 * j] - s1 - h0 * s2) + rf.x,
-                             rstd[r] * (gf.y * wf[2 * j + 1] - s1 - h1 * s2) + rf.y);
+          const f32x2_t h = KEEP ? kh[KEEP ? r : 0][j] : norm2(r, xu[j]);
+          const f32x2_t a = KEEP ? ka[KEEP ? r : 0][j] : f2_mul(f2_from_bf16x2(gu[j]), wf[j]);
+          o[j] = f2_to_bf16x2(f2_fma(rs, f2_fma(h, n2, f2_add(a, n1)), f2_from_bf16x2(ru[j])));
         }
         *reinterpret_cast<uint4*>(dx + (long long)(row0 + r) * C + col) =
             make_uint4(o[0], o[1], o[2], o[3]);
@@ -291,6 +328,12 @@ norm_bwd_all_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
       xv[r] = xn[r]; gv[r] = gn[r]; rv[r] = rn[r];
       mean[r] = mn[r]; rstd[r] = sn[r];
     }
+  }
+  float sw[8], sb[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    f2_unpack(sw2[j], sw[2 * j], sw[2 * j + 1]);
+    f2_unpack(sb2[j], sb[2 * j], sb[2 * j + 1]);
   }
   // column sums: groups of the CTA through shared memory, then one vector reduction per four
   if (groups > 1) {
@@ -377,17 +420,27 @@ static int launch_bwd_all(const void* dy, const void* x, const void* w, const fl
 
 // Column sums.  Block = 32 x 8 threads: a lane owns 8 adjacent columns (one 16-byte piece
 // per row), the 8 warps take interleaved rows; grid = (ceil(C/256), row_splits).
-// Each thread streams its pieces through a private ring of COLSUM_RING shared-memory slots
-// filled by cp.async (no registers held while in flight, no barriers: a thread only reads
-// what it copied itself), so a CTA keeps COLSUM_RING x 4 KB (x2 with the norm input) in
-// flight; plain register loads kept only ~1 load per warp outstanding at 2.4 TB/s.
+//
+// Plain sums (bias gradients): a thread loads COLSUM_UNROLL rows before it adds the first, as pairs:
+// 12 instructions for 8 values (through the ring, one by one: 8192 x 1024 6.5 -> 5.8 us, 8192 x 4096
+// 14.5 -> 10.5, 2313 x 3072 6.1 -> 5.4; 512 x 256 3.9 -> 4.3).
+//
+// With the norm input (NORM): each thread streams its pieces through a private ring of COLSUM_RING
+// shared-memory slots filled by cp.async (no registers held while in flight, no barriers: a thread
+// only reads what it copied itself), so a CTA keeps COLSUM_RING x 8 KB in flight; plain register
+// loads kept only ~1 load per warp outstanding at 2.4 TB/s.
 constexpr int COLSUM_RING = 8;
-constexpr int COLSUM_UNROLL = COLSUM_RING;  // rows per warp the row split aims for
-constexpr int COLSUM_SMEM_BYTES = 2 * COLSUM_RING * 256 * 16;
+constexpr int COLSUM_UNROLL = 8;  // rows in flight per thread, and per warp at least
+// the ring, or the reduction buffer alone
+template <bool NORM>
+constexpr int colsum_smem_bytes() {
+  return NORM ? 2 * COLSUM_RING * 256 * 16 : 8 * (256 + 8) * 4;
+}
 __device__ __forceinline__ void colsum_cp16(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc)
                : "memory");
 }
+template <bool NORM>
 __global__ void __launch_bounds__(256)
 colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
               const float* __restrict__ stats, float* __restrict__ acc, int rows, int C,
@@ -395,7 +448,7 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restr
               int accumulate) {
   if (!grid_dep_begin()) return;
   // ring slots [which: dy | x][slot][thread] (16 bytes each); the reduction buffer reuses it
-  extern __shared__ __align__(16) uint8_t colsum_smem[];  // COLSUM_SMEM_BYTES, dynamic
+  extern __shared__ __align__(16) uint8_t colsum_smem[];  // colsum_smem_bytes<NORM>(), dynamic
   uint4 (*ring)[COLSUM_RING][256] = reinterpret_cast<uint4 (*)[COLSUM_RING][256]>(colsum_smem);
   float (*sh)[256 + 8] = reinterpret_cast<float (*)[256 + 8]>(colsum_smem);
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
@@ -405,16 +458,37 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restr
   for (int k = 0; k < 8; ++k) a[k] = b[k] = 0.f;
   const bool vec = (col + 8 <= C) && ((ld & 7) == 0) &&
                    ((reinterpret_cast<uintptr_t>(dy) & 15) == 0) &&
-                   (!x || (reinterpret_cast<uintptr_t>(x) & 15) == 0);
+                   (!NORM || (reinterpret_cast<uintptr_t>(x) & 15) == 0);
   const int stride = gridDim.y * 8;
   const int r0 = blockIdx.y * 8 + wy;
-  if (col < C && vec) {
+  if (!NORM && col < C && vec) {
+    f32x2_t t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) t[j] = f2_pack(0.f, 0.f);
+    for (long long r = r0; r < rows; r += COLSUM_UNROLL * stride) {
+      uint4 v[COLSUM_UNROLL];
+#pragma unroll
+      for (int u = 0; u < COLSUM_UNROLL; ++u) {
+        v[u] = make_uint4(0, 0, 0, 0);
+        if (r + u * stride < rows) v[u] = ld_nc_v4(dy + (r + u * stride) * ld + col);
+      }
+#pragma unroll
+      for (int u = 0; u < COLSUM_UNROLL; ++u) {
+        t[0] = f2_add(t[0], f2_from_bf16x2(v[u].x));
+        t[1] = f2_add(t[1], f2_from_bf16x2(v[u].y));
+        t[2] = f2_add(t[2], f2_from_bf16x2(v[u].z));
+        t[3] = f2_add(t[3], f2_from_bf16x2(v[u].w));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) f2_unpack(t[j], b[2 * j], b[2 * j + 1]);
+  } else if (NORM && col < C && vec) {
     const int n = r0 < rows ? (rows - r0 + stride - 1) / stride : 0;  // rows of this thread
     auto issue = [&](int k) {
       if (k < n) {
         const long long off = (long long)(r0 + (long long)k * stride) * ld + col;
         colsum_cp16(&ring[0][k % COLSUM_RING][threadIdx.x], dy + off);
-        if (x) colsum_cp16(&ring[1][k % COLSUM_RING][threadIdx.x], x + off);
+        colsum_cp16(&ring[1][k % COLSUM_RING][threadIdx.x], x + off);
       }
       asm volatile("cp.async.commit_group;" ::: "memory");  // one group per step, empty or not
     };
@@ -424,27 +498,18 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restr
       asm volatile("cp.async.wait_group %0;" ::"n"(COLSUM_RING - 1) : "memory");
       const uint4 gu = ring[0][k % COLSUM_RING][threadIdx.x];
       const uint32_t w[4] = {gu.x, gu.y, gu.z, gu.w};
-      if (x) {
-        const uint4 xu = ring[1][k % COLSUM_RING][threadIdx.x];
-        const uint32_t v[4] = {xu.x, xu.y, xu.z, xu.w};
-        const long long rr = r0 + (long long)k * stride;
-        const float mean = rms ? 0.f : stats[2 * rr];
-        const float rstd = stats[2 * rr + 1];
+      const uint4 xu = ring[1][k % COLSUM_RING][threadIdx.x];
+      const uint32_t v[4] = {xu.x, xu.y, xu.z, xu.w};
+      const long long rr = r0 + (long long)k * stride;
+      const float mean = rms ? 0.f : stats[2 * rr];
+      const float rstd = stats[2 * rr + 1];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = unpack_bf16x2(w[j]), xf = unpack_bf16x2(v[j]);
-          b[2 * j] += f.x;
-          b[2 * j + 1] += f.y;
-          a[2 * j] += f.x * (xf.x - mean) * rstd;
-          a[2 * j + 1] += f.y * (xf.y - mean) * rstd;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = unpack_bf16x2(w[j]);
-          b[2 * j] += f.x;
-          b[2 * j + 1] += f.y;
-        }
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = unpack_bf16x2(w[j]), xf = unpack_bf16x2(v[j]);
+        b[2 * j] += f.x;
+        b[2 * j + 1] += f.y;
+        a[2 * j] += f.x * (xf.x - mean) * rstd;
+        a[2 * j + 1] += f.y * (xf.y - mean) * rstd;
       }
       issue(k + COLSUM_RING);  // refill the slot just read
     }
@@ -455,11 +520,11 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restr
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         g[k] = (col + k < C) ? __bfloat162float(dy[(long long)r * ld + col + k]) : 0.f;
-        xv[k] = (x && col + k < C) ? __bfloat162float(x[(long long)r * ld + col + k]) : 0.f;
+        xv[k] = (NORM && col + k < C) ? __bfloat162float(x[(long long)r * ld + col + k]) : 0.f;
       }
 #pragma unroll
       for (int k = 0; k < 8; ++k) b[k] += g[k];
-      if (x) {
+      if (NORM) {
         const float mean = rms ? 0.f : stats[2 * r];
         const float rstd = stats[2 * r + 1];
 #pragma unroll
@@ -468,7 +533,7 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restr
     }
   }
   for (int which = 0; which < 2; ++which) {
-    if (which == 0 && !x) continue;
+    if (which == 0 && !NORM) continue;
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 8; ++k) sh[wy][lane * 8 + k] = which == 0 ? a[k] : b[k];
@@ -590,33 +655,33 @@ extern "C" int nkb_norm_bwd_all(const void* dy, const void* x, const void* w, co
                                 accum_w, accum_b, s);
 }
 
-// the ring needs more than the 48 KB a kernel gets without opting in
-static int colsum_configure() {
-  static bool done[64];
-  return nkb::allow_smem(nkb::colsum_kernel, nkb::COLSUM_SMEM_BYTES, done);
+// row splits: about three CTAs per SM (64 KB of ring each; four without), and whole turns of
+// COLSUM_UNROLL rows per warp
+static int colsum_row_splits(int gx, int rows, int per_sm) {
+  const int most = (per_sm * 148 + gx - 1) / gx, turn = 8 * nkb::COLSUM_UNROLL;
+  const int turns = (int)((rows + (long long)turn * most - 1) / ((long long)turn * most));
+  return (int)((rows + (long long)turn * turns - 1) / ((long long)turn * turns));
 }
 
-// row splits: about three CTAs per SM (64 KB of ring each), and at least COLSUM_UNROLL rows per
-// warp when possible
-static int colsum_row_splits(int gx, int rows) {
-  int gy = (3 * 148 + gx - 1) / gx;
-  int max_gy = rows / (8 * nkb::COLSUM_UNROLL);
-  if (max_gy < 1) max_gy = 1;
-  if (gy > max_gy) gy = max_gy;
-  return gy < 1 ? 1 : gy;
+template <bool NORM>
+static int launch_colsum(const void* dy, const void* x, const float* stats, float* acc, int rows,
+                         int C, long long ld, int rms, int* tickets, void* out, int accumulate,
+                         void* stream) {
+  constexpr int smem = nkb::colsum_smem_bytes<NORM>();
+  static bool done[64];
+  if (nkb::allow_smem(nkb::colsum_kernel<NORM>, smem, done)) return -6;
+  const int gx = (C + 255) / 256, gy = rows > 0 ? colsum_row_splits(gx, rows, NORM ? 3 : 4) : 1;
+  launch_dep(colsum_kernel<NORM>, dim3(gx, gy), 256, smem, static_cast<cudaStream_t>(stream),
+             static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats, acc,
+             rows, C, ld, rms, tickets, static_cast<__nv_bfloat16*>(out), accumulate);
+  return (int)cudaGetLastError();
 }
 
 extern "C" int nkb_colsum(const void* dy, const void* x, const float* stats, float* acc, int rows,
                           int C, long long ld, int rms, void* stream) {
   if ((C & 1) || (ld & 1)) return -3;
-  int gx = (C + 255) / 256;
-  int gy = colsum_row_splits(gx, rows);
-  if (colsum_configure()) return -6;
-  launch_dep(colsum_kernel, dim3(gx, gy), 256, nkb::COLSUM_SMEM_BYTES,
-             static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(dy),
-             static_cast<const __nv_bfloat16*>(x), stats, acc, rows, C, ld, rms, nullptr, nullptr,
-             0);
-  return (int)cudaGetLastError();
+  return x ? launch_colsum<true>(dy, x, stats, acc, rows, C, ld, rms, nullptr, nullptr, 0, stream)
+           : launch_colsum<false>(dy, x, stats, acc, rows, C, ld, rms, nullptr, nullptr, 0, stream);
 }
 
 // Column sums of dy straight to a bf16 output in one launch.  acc: fp32 [2][C] (the second half
@@ -625,13 +690,8 @@ extern "C" int nkb_colsum(const void* dy, const void* x, const float* stats, flo
 extern "C" int nkb_colsum_fused(const void* dy, float* acc, int* tickets, void* out,
                                 int accumulate, int rows, int C, long long ld, void* stream) {
   if ((C & 1) || (ld & 1) || !acc || !tickets || !out) return -3;
-  int gx = (C + 255) / 256;
-  int gy = colsum_row_splits(gx, rows);
-  if (colsum_configure()) return -6;
-  launch_dep(colsum_kernel, dim3(gx, gy), 256, nkb::COLSUM_SMEM_BYTES,
-             static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(dy), nullptr,
-             nullptr, acc, rows, C, ld, 0, tickets, static_cast<__nv_bfloat16*>(out), accumulate);
-  return (int)cudaGetLastError();
+  return launch_colsum<false>(dy, nullptr, nullptr, acc, rows, C, ld, 0, tickets, out, accumulate,
+                              stream);
 }
 
 extern "C" int nkb_f32_to_bf16(const float* src, void* dst, long long n, int accumulate,
