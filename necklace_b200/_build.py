@@ -23,6 +23,8 @@ LIB = os.path.join(HERE, "_nkb200.so")
 # the same entry points as a Python extension (csrc/pycall.cpp), linked to LIB; the suffix names
 # the interpreter, so another Python version in the same checkout does not load it
 EXT = os.path.join(HERE, "_nkpy" + sysconfig.get_config_var("EXT_SUFFIX"))
+# operators on torch tensors (csrc/pytensor.cpp), linked to LIB and torch's libraries
+OPS = os.path.join(HERE, "_nkops" + sysconfig.get_config_var("EXT_SUFFIX"))
 # the bounds-checked debug variant (-DNKB_DEBUG_BOUNDS): ``--debug-bounds``
 BUILD_DBG = os.path.join(os.path.dirname(HERE), "build", "nkb200_dbg")
 LIB_DBG = os.path.join(HERE, "_nkb200_dbg.so")
@@ -86,6 +88,7 @@ def build(force: bool = False, verbose: bool = False, debug_bounds: bool = False
             raise RuntimeError(f"link failed:\n{p.stdout}{p.stderr}")
     if not debug_bounds:
         build_ext(force)
+        build_ops(force)
     return lib
 
 
@@ -95,29 +98,49 @@ def build_ext(force: bool = False) -> bool:
     untagged = os.path.join(os.path.dirname(EXT), "_nkpy.so")
     if os.path.exists(untagged):           # as it was named before, for any interpreter
         os.remove(untagged)
-    src = os.path.join(CSRC, "pycall.cpp")
+    return _build_extension(EXT, "pycall.cpp", [], force, "calls go through ctypes")
+
+
+def build_ops(force: bool = False) -> bool:
+    """Compile the operators on tensors; whether there are any.  Without them the operators do the
+    same in Python, so a failure is a warning."""
+    import torch
+    from torch.utils import cpp_extension
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    flags = [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for d in [*cpp_extension.include_paths(), os.path.join(cuda, "include")]:
+        flags += ["-isystem", d]
+    for d in cpp_extension.library_paths():
+        flags += ["-L", d]
+    flags += ["-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    return _build_extension(OPS, "pytensor.cpp", flags, force,
+                            "operators take the way through Python")
+
+
+def _build_extension(target: str, source: str, flags: list[str], force: bool, without: str) -> bool:
+    src = os.path.join(CSRC, source)
     newest = max(os.path.getmtime(src), _headers_mtime())
-    if not force and os.path.exists(EXT) and os.path.getmtime(EXT) >= newest:
+    if not force and os.path.exists(target) and os.path.getmtime(target) >= newest:
         return True
     inc = sysconfig.get_paths()["include"]
     # built under another name and moved: a process may be importing it
-    tmp = EXT + f".{os.getpid()}"
+    tmp = target + f".{os.getpid()}"
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-I", inc, "-I",
            CSRC, src, "-o", tmp, "-L", HERE, "-l:" + os.path.basename(LIB),
-           "-Wl,-rpath,$ORIGIN"]
+           "-Wl,-rpath,$ORIGIN", *flags]
     try:
         p = subprocess.run(cmd, capture_output=True, text=True)
         log = f"exit code {p.returncode}\n{p.stdout}{p.stderr}" if p.returncode else ""
     except OSError as e:
         log = str(e)
     if not log:
-        os.replace(tmp, EXT)
+        os.replace(tmp, target)
         return True
     # one that was built for other signatures must not stay
-    for old in (tmp, EXT):
+    for old in (tmp, target):
         if os.path.exists(old):
             os.remove(old)
-    warnings.warn(f"building {EXT} failed, calls go through ctypes:\n{log[-2000:]}", stacklevel=2)
+    warnings.warn(f"building {target} failed, {without}:\n{log[-2000:]}", stacklevel=3)
     return False
 
 

@@ -170,9 +170,48 @@ def _load_fast(build_if_missing: bool) -> dict:
     return {n: getattr(_nkpy, n) for n in dir(_nkpy) if n.startswith("nkb_")}
 
 
+# operators on tensors (csrc/pytensor.cpp), None where there is no such module
+_ops = None
+
+
+def _load_ops(build_if_missing: bool):
+    if DEBUG_BOUNDS:
+        return None         # linked to the normal library, like _nkpy
+    try:
+        from . import _nkops
+        from torch import __version__
+        return _nkops if _nkops.torch_version == __version__.split("+")[0] else None
+    except ImportError:
+        if build_if_missing:
+            from . import _build
+            if _build.build_ops():
+                importlib.invalidate_caches()
+                return _load_ops(False)
+    return None
+
+
+def ops():
+    """The compiled operators, or None: then every operator takes its general way."""
+    if _lib is None:
+        load()
+    return _ops
+
+
+def done(r, name: str, launches: int = 1) -> bool:
+    """Whether a compiled operator has done its work: None is left to the general way, an int is a
+    native error code."""
+    global launch_count
+    if r is None:
+        return False
+    if type(r) is int:
+        check(r, name)
+    launch_count += launches
+    return True
+
+
 def load(build_if_missing: bool = True):
     """Load (building first if needed and possible) and return the ctypes handle."""
-    global _lib, _load_error
+    global _lib, _ops, _load_error
     if _lib is not None:
         return _lib
     with _lock:
@@ -191,6 +230,7 @@ def load(build_if_missing: bool = True):
             if hasattr(lib, "nkb_build_info"):
                 lib.nkb_build_info.restype = C.c_char_p
             _fast.update(_load_fast(build_if_missing))
+            _ops = _load_ops(build_if_missing)
             _lib = lib
         except Exception as e:  # noqa: BLE001
             _load_error = e

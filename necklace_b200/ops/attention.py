@@ -64,6 +64,10 @@ def _split(qkv, H):
 
 def attn_fwd(qkv: torch.Tensor, H: int, causal: bool = True):
     """Returns (out [B,S,C], lse [B,H,S] fp32)."""
+    if qkv.is_cuda and (ops := _lib.ops()) is not None:
+        r = ops.attn(qkv, H, causal, status_ptr(qkv))
+        if _lib.done(r, "nkb_attn_fwd"):
+            return r
     B, S, C3 = qkv.shape
     C = C3 // 3
     D = C // H
@@ -91,6 +95,10 @@ def attn_fwd(qkv: torch.Tensor, H: int, causal: bool = True):
 
 def attn_bwd(qkv, out, lse, dout, H: int, causal: bool = True):
     """Returns dqkv [B,S,3C]."""
+    if qkv.is_cuda and (ops := _lib.ops()) is not None:
+        r = ops.attn_bwd(qkv, out, lse, dout, H, causal, status_ptr(qkv))
+        if _lib.done(r, "nkb_attn_bwd", 3):
+            return r
     B, S, C3 = qkv.shape
     C = C3 // 3
     D = C // H

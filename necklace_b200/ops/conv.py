@@ -234,6 +234,14 @@ def conv2d(x, w, KH, KW, stride=1, pad=0):
 
 def _conv2d_plain(x, w, KH, KW, stride, pad):
     """The forward pass by itself."""
+    if x.is_cuda and x.dim() == 4 and (ops := _lib.ops()) is not None:
+        y = None
+        if KH == 1 and KW == 1 and stride == 1 and pad == 0:
+            y = ops.linear(x, w, None, None, status_ptr(x))
+        elif _image_route(x, w, KH, KW, stride, pad) & 1:
+            y = ops.conv(x, w, KH, KW, stride, pad, status_ptr(x))
+        if _lib.done(y, "convolution"):
+            return y
     N, H, W, C = x.shape
     direct = KH == 1 and KW == 1 and stride == 1 and pad == 0 and C % 8 == 0
     if not direct and _image_route(x, w, KH, KW, stride, pad) & 1:
@@ -402,6 +410,11 @@ class BatchNorm2d(nn.Module):
             return BatchNormFn.apply(x, self.weight, self.bias, residual, self.running_mean,
                                      self.running_var, self.eps, self.momentum, self.relu)
         C = self.C
+        if x.is_cuda and (ops := _lib.ops()) is not None:
+            y = ops.bn_eval(x, self.running_mean, self.running_var, self.eps, self.weight, self.bias,
+                            residual, self.relu)
+            if _lib.done(y, "nkb_bn_eval"):
+                return y
         x2 = x.reshape(-1, C)
         if not on_gpu(x):
             stats = torch.stack([self.running_mean, torch.rsqrt(self.running_var + self.eps)])

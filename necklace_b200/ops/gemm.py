@@ -37,6 +37,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          alpha_dev: torch.Tensor | None = None) -> torch.Tensor:
     """``a`` is stored ``[M,K]`` (or ``[K,M]`` when ``a_mn``); ``b`` is stored ``[N,K]``
     (or ``[K,N]`` when ``b_mn``).  Both must be 2-D with unit inner stride."""
+    if a.is_cuda and ready_flags is None and max_ctas == 0 \
+            and (out_dtype is None or out_dtype is torch.bfloat16 or out_dtype is torch.float32):
+        ops = _lib.ops()
+        if ops is not None:
+            y = ops.gemm(a, b, a_mn, b_mn, out, out_dtype is torch.float32, accumulate, alpha, bias,
+                         res, epi, aux, bn, alpha_dev, status_ptr(a))
+            if _lib.done(y, "nkb_gemm_bf16_ws"):
+                return y
     sa, sb = a.shape, b.shape
     assert len(sa) == 2 and len(sb) == 2
     M, K = (sa[1], sa[0]) if a_mn else sa
@@ -176,6 +184,27 @@ def _deliver_grad(p: torch.Tensor, compute):
     return None
 
 
+def _grad_target(p):
+    """(tensor the kernel writes, accumulate?, what autograd gets) for parameter ``p``."""
+    buf = getattr(p, "_nkb_grad", None)
+    if buf is None:
+        out = torch.empty_like(p)
+        return out, False, out
+    return buf, bool(getattr(p, "_nkb_grad_has", False)), None
+
+
+def _grad_done(p):
+    if getattr(p, "_nkb_grad", None) is None:
+        return
+    p._nkb_grad_has = True
+    cb = getattr(p, "_nkb_grad_ready", None)
+    if cb is not None:
+        cb(p)
+
+
+_NO_TARGET = (None, False, None)
+
+
 def _deliver_nothing(p: torch.Tensor):
     """The gradient of a parameter whose output nobody used: zeros, delivered like any other."""
     return _deliver_grad(p, lambda out, acc: torch.zeros_like(p) if out is None
@@ -187,18 +216,33 @@ class LinearFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w, b, residual):
-        x2 = x.reshape(-1, x.shape[-1])
-        r2 = residual.reshape(-1, w.shape[0]) if residual is not None else None
-        y = gemm(x2, w, bias=b, res=r2)
+        x2 = x if x.is_contiguous() else x.reshape(-1, x.shape[-1])
+        y = _linear(x2, w, b, residual)
         ctx.save_for_backward(x2, w)
         ctx.has_b = b is not None
         ctx.has_r = residual is not None
         ctx.b_ref = b
-        return y.view(*x.shape[:-1], w.shape[0])
+        return y if x2 is x else y.view(*x.shape[:-1], w.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
-        x2, w = ctx.saved_tensors
+        x, w = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        dres = dy if ctx.has_r and need[3] else None
+        if dy.is_cuda and (ops := _lib.ops()) is not None:
+            b, bias = ctx.b_ref, ctx.has_b and need[2]
+            tw, acc_w, dw = _grad_target(w) if need[1] else _NO_TARGET
+            tb, acc_b, db = _grad_target(b) if bias else _NO_TARGET
+            acc, tickets = colsum_scratch(w.shape[0], dy.device) if bias else (None, None)
+            r = ops.linear_bwd(dy, x, w, need[0], tw, acc_w, tb, acc_b, acc, tickets,
+                               status_ptr(dy))
+            if _lib.done(r, "nkb_gemm_bf16_ws", need[0] + need[1] + bias):
+                if need[1]:
+                    _grad_done(w)
+                if bias:
+                    _grad_done(b)
+                return r[0] if need[0] else None, dw, db, dres
+        x2 = x.reshape(-1, x.shape[-1])
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
@@ -210,7 +254,6 @@ class LinearFn(torch.autograd.Function):
                                                         accumulate=acc))
         if ctx.has_b and ctx.needs_input_grad[2]:
             db = _deliver_grad(ctx.b_ref, lambda out, acc: colsum(dy2, out, acc))
-        dres = dy if ctx.has_r and ctx.needs_input_grad[3] else None
         return dx, dw, db, dres
 
 
@@ -224,25 +267,33 @@ class MLPFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w1, b1, w2, b2, residual, act):
-        x2 = x.reshape(-1, x.shape[-1])
-        r2 = residual.reshape(-1, w2.shape[0]) if residual is not None else None
-        if act == "gelu":
-            z = torch.empty(x2.shape[0], w1.shape[0], dtype=x2.dtype, device=x2.device)
-            h = gemm(x2, w1, bias=b1, epi=EPI_GELU_FWD, aux=z)
-        else:
-            z = None
-            h = gemm(x2, w1, bias=b1, epi=EPI_RELU)
-        y = gemm(h, w2, bias=b2, res=r2)
+        x2 = x if x.is_contiguous() else x.reshape(-1, x.shape[-1])
+        y, h, z = _mlp(x2, w1, b1, w2, b2, residual, act)
         ctx.save_for_backward(x2, w1, w2, h, z)
         ctx.act = act
         ctx.refs = (b1, b2)
         ctx.has_r = residual is not None
-        return y.view(*x.shape[:-1], w2.shape[0])
+        return y if x2 is x else y.view(*x.shape[:-1], w2.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
-        x2, w1, w2, h, z = ctx.saved_tensors
+        x, w1, w2, h, z = ctx.saved_tensors
         b1, b2 = ctx.refs
+        need_x = ctx.needs_input_grad[0]
+        if dy.is_cuda and ctx.act == "gelu" and w1 is not w2 and (b1 is None or b1 is not b2) \
+                and (ops := _lib.ops()) is not None:
+            t = [_grad_target(p) if p is not None else _NO_TARGET for p in (w1, b1, w2, b2)]
+            acc, tickets = (None, None) if b1 is None and b2 is None else \
+                colsum_scratch(max(w1.shape[0], w2.shape[0]), dy.device)
+            r = ops.mlp_bwd(dy, x, w1, w2, h, z, need_x, t[0][0], t[0][1], t[1][0], t[1][1], t[2][0],
+                            t[2][1], t[3][0], t[3][1], acc, tickets, status_ptr(dy))
+            if _lib.done(r, "nkb_gemm_bf16_ws", 3 + need_x + (b1 is not None) + (b2 is not None)):
+                for p in (w2, b2, w1, b1):
+                    if p is not None:
+                        _grad_done(p)
+                return (r[0] if need_x else None, t[0][2], t[1][2], t[2][2], t[3][2],
+                        dy if ctx.has_r else None, None)
+        x2 = x.reshape(-1, x.shape[-1])
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
@@ -257,7 +308,7 @@ class MLPFn(torch.autograd.Function):
         if b2 is not None:
             db2 = _deliver_grad(b2, lambda out, acc: colsum(dy2, out, acc))
         dx = gemm(dz, w1, b_mn=True).view(*dy.shape[:-1], w1.shape[1]) \
-            if ctx.needs_input_grad[0] else None
+            if need_x else None
         dw1 = _deliver_grad(w1, lambda out, acc: gemm(dz, x2, a_mn=True, b_mn=True, out=out,
                                                       accumulate=acc))
         db1 = None
@@ -267,24 +318,43 @@ class MLPFn(torch.autograd.Function):
         return dx, dw1, db1, dw2, db2, dres, None
 
 
+def _linear(x, w, b, residual):
+    """The forward pass by itself."""
+    if x.is_cuda and (ops := _lib.ops()) is not None:
+        y = ops.linear(x, w, b, residual, status_ptr(x))
+        if _lib.done(y, "nkb_gemm_bf16_ws"):
+            return y
+    r2 = residual.reshape(-1, w.shape[0]) if residual is not None else None
+    y = gemm(x.reshape(-1, x.shape[-1]), w, bias=b, res=r2)
+    return y.view(*x.shape[:-1], w.shape[0])
+
+
+def _mlp(x, w1, b1, w2, b2, residual, act):
+    """(output, activation, pre-activation or None) of the forward pass by itself."""
+    if act == "gelu" and x.is_cuda and (ops := _lib.ops()) is not None:
+        r = ops.mlp(x, w1, b1, w2, b2, residual, status_ptr(x))
+        if _lib.done(r, "nkb_gemm_bf16_ws", 2):
+            return r
+    x2 = x.reshape(-1, x.shape[-1])
+    r2 = residual.reshape(-1, w2.shape[0]) if residual is not None else None
+    z = None
+    if act == "gelu":
+        z = torch.empty(x2.shape[0], w1.shape[0], dtype=x2.dtype, device=x2.device)
+        h = gemm(x2, w1, bias=b1, epi=EPI_GELU_FWD, aux=z)
+    else:
+        h = gemm(x2, w1, bias=b1, epi=EPI_RELU)
+    return gemm(h, w2, bias=b2, res=r2).view(*x.shape[:-1], w2.shape[0]), h, z
+
+
 def linear(x, w, b=None, residual=None):
     if plain_call():
-        r2 = residual.reshape(-1, w.shape[0]) if residual is not None else None
-        y = gemm(x.reshape(-1, x.shape[-1]), w, bias=b, res=r2)
-        return y.view(*x.shape[:-1], w.shape[0])
+        return _linear(x, w, b, residual)
     return LinearFn.apply(x, w, b, residual)
 
 
 def mlp(x, w1, b1, w2, b2, residual=None, act="gelu"):
     if plain_call():
-        x2 = x.reshape(-1, x.shape[-1])
-        r2 = residual.reshape(-1, w2.shape[0]) if residual is not None else None
-        if act == "gelu":
-            z = torch.empty(x2.shape[0], w1.shape[0], dtype=x2.dtype, device=x2.device)
-            h = gemm(x2, w1, bias=b1, epi=EPI_GELU_FWD, aux=z)
-        else:
-            h = gemm(x2, w1, bias=b1, epi=EPI_RELU)
-        return gemm(h, w2, bias=b2, res=r2).view(*x.shape[:-1], w2.shape[0])
+        return _mlp(x, w1, b1, w2, b2, residual, act)[0]
     return MLPFn.apply(x, w1, b1, w2, b2, residual, act)
 
 

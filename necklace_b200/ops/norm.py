@@ -6,7 +6,8 @@ import torch.nn as nn
 
 from .. import _lib
 from ._common import on_gpu, plain_call, ptr
-from .gemm import _deliver_grad, _deliver_nothing, colsum_scratch
+from .gemm import (_deliver_grad, _deliver_nothing, _grad_done, _grad_target,
+                   colsum_scratch)
 
 
 def norm_fwd(x2: torch.Tensor, w: torch.Tensor, b: torch.Tensor | None, eps: float, rms: bool):
@@ -83,18 +84,28 @@ def _store_f32_grad(p, g32):
 class NormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b, eps, rms):
-        x2 = x.reshape(-1, x.shape[-1])
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        y, stats = norm_fwd(x2, w, b, eps, rms)
-        ctx.save_for_backward(x2, w, stats)
+        y, stats, kept = _norm(x, w, b, eps, rms)
+        ctx.save_for_backward(kept, w, stats)
         ctx.rms = rms
         ctx.b_ref = b
-        return y.view(x.shape)
+        return y
 
     @staticmethod
     def backward(ctx, dy, dres=None):
-        x2, w, stats = ctx.saved_tensors
+        x, w, stats = ctx.saved_tensors
+        if dy.is_cuda and (ops := _lib.ops()) is not None:
+            b = ctx.b_ref
+            tgt_w, acc_w, ret_w = _grad_target(w)
+            tgt_b, acc_b, ret_b = _grad_target(b) if b is not None else (None, False, None)
+            acc, tickets = colsum_scratch(w.shape[0], dy.device)
+            dx = ops.norm_bwd(dy, x, w, stats, dres, ctx.rms, tgt_w, acc_w, tgt_b, acc_b, acc,
+                              tickets)
+            if _lib.done(dx, "nkb_norm_bwd_all"):
+                _grad_done(w)
+                if b is not None:
+                    _grad_done(b)
+                return dx, ret_w, ret_b, None, None
+        x2 = x.reshape(-1, x.shape[-1])
         dy2 = dy.reshape(-1, dy.shape[-1])
         if dres is not None:
             dres = dres.reshape(-1, dres.shape[-1])
@@ -133,29 +144,23 @@ def _rows16(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-def _norm_plain(x, w, b, eps, rms):
+def _norm(x, w, b, eps, rms):
+    """(output, row statistics, x without gaps) of the forward pass by itself."""
+    if x.is_cuda and (ops := _lib.ops()) is not None:
+        r = ops.norm(x, w, b, eps, rms)
+        if _lib.done(r, "nkb_norm_fwd"):
+            return r[0], r[1], x
     x2 = x.reshape(-1, x.shape[-1])
     if not x2.is_contiguous():
         x2 = x2.contiguous()
-    return norm_fwd(x2, w, b, eps, rms)[0].view(x.shape)
+    y, stats = norm_fwd(x2, w, b, eps, rms)
+    return y.view(x.shape), stats, x2
 
 
-def _grad_target(p):
-    """(tensor the kernel writes, accumulate?, what autograd gets) for parameter ``p``."""
-    buf = getattr(p, "_nkb_grad", None)
-    if buf is None:
-        out = torch.empty_like(p)
-        return out, False, out
-    return buf, bool(getattr(p, "_nkb_grad_has", False)), None
+def _norm_plain(x, w, b, eps, rms):
+    return _norm(x, w, b, eps, rms)[0]
 
 
-def _grad_done(p):
-    if getattr(p, "_nkb_grad", None) is None:
-        return
-    p._nkb_grad_has = True
-    cb = getattr(p, "_nkb_grad_ready", None)
-    if cb is not None:
-        cb(p)
 
 
 class NormSplitFn(torch.autograd.Function):

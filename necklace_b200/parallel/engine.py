@@ -44,6 +44,11 @@ from ..ops._common import check_status
 from ..ops.optim import clip_coef, hyper_advance, sumsq
 from .flat import FlatParams
 
+# A step's backward pass is a chain of short host calls: run in the calling thread it needs no
+# hand-over of the interpreter lock to the device's autograd thread (step of a two-layer GPT-2 over
+# 2 x 256 tokens: 1.51 -> 1.24 ms).
+_one_thread = torch.autograd.set_multithreading_enabled
+
 HYPER_LR, HYPER_C1, HYPER_C2, HYPER_T, HYPER_GMUL = 0, 1, 2, 3, 4
 
 
@@ -340,7 +345,8 @@ class TrainEngine:
         if k == 1:
             self._armed = True
             loss = self.model(*inputs)
-            loss.backward()
+            with _one_thread(False):
+                loss.backward()
             self._armed = False
             total = loss.detach()
         else:
@@ -349,7 +355,8 @@ class TrainEngine:
             for j in range(k):
                 self._armed = j == k - 1
                 loss = self.model(*(c[j] for c in chunks))
-                loss.backward()
+                with _one_thread(False):
+                    loss.backward()
                 total = loss.detach() if total is None else total + loss.detach()
             self._armed = False
             total = total / k
