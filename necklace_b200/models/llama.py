@@ -118,18 +118,25 @@ class LlamaBlock(nn.Module):
     def forward(self, x, batch=None):
         if self.cfg.tp_group is not None:
             return self.forward_sp(x, batch)
-        h = self._copy(self.ln1(x))
+        # the gradient that reaches x along the residual path is added in the norm's backward
+        x, h = _norm_split(self.ln1, x)
+        h = self._copy(h)
         qkv = linear_rope(h, self.w_qkv, self.n_head_local, self.cfg.rope_base)
         a = attention_qkv(qkv, self.n_head_local, True)
         if self.cfg.mp == 1:
             x = linear(a, self.w_o, None, residual=x)
         else:
             x = x + self._reduce(linear(a, self.w_o))
-        h = self._copy(self.ln2(x))
+        x, h = _norm_split(self.ln2, x)
+        h = self._copy(h)
         f = swiglu(linear(h, self.w_gu))
         if self.cfg.mp == 1:
             return linear(f, self.w_down, None, residual=x)
         return x + self._reduce(linear(f, self.w_down))
+
+
+def _norm_split(norm, x):
+    return norm.split(x) if isinstance(norm, RMSNorm) else (x, norm(x))
 
 
 def _padded_vocab(cfg) -> int:

@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import _lib
 from ._common import on_gpu, plain_call, ptr
@@ -183,6 +184,15 @@ class NormSplitFn(torch.autograd.Function):
         return NormFn.backward(ctx, dy, dres)
 
 
+def _observed(m, cls) -> bool:
+    """Whether something would notice that the module is not called: hooks of its own or global ones,
+    or a forward of a subclass or of this instance."""
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks
+                or m._backward_pre_hooks or _has_any_global_hook()
+                or type(m).forward is not cls.forward or type(m).__call__ is not nn.Module.__call__
+                or "forward" in m.__dict__)
+
+
 class LayerNorm(nn.Module):
     def __init__(self, dim: int, eps: float = 1e-5, bias: bool = True, dtype=torch.bfloat16,
                  device=None):
@@ -216,6 +226,8 @@ class RMSNorm(nn.Module):
 
     def split(self, x):
         """``(x, norm(x))`` for a pre-norm residual block (see ``NormSplitFn``)."""
+        if _observed(self, RMSNorm):
+            return x, self(x)
         if plain_call():
             return x, _norm_plain(x, self.weight, None, self.eps, True)
         return NormSplitFn.apply(x, self.weight, None, self.eps, True)
