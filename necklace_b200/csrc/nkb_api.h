@@ -26,8 +26,8 @@ int nkb_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long lo
                   void* aux, long long ldaux, int* status, const int* ready_flags,
                   int rows_per_flag, int ready_target, int max_ctas, int bn_hint,
                   const float* alpha_dev, void* stream);
-// The number of slices (>= 1) into which a GEMM of these sizes without bias, residual and
-// activation cuts K, and the same GEMM with that number and the fp32 [slices][M][N] workspace of
+// The number of slices (>= 1) into which a GEMM of these sizes without activation cuts K (bias and
+// residual: 8-byte aligned, rows of the latter a multiple of 4 apart), and the same GEMM with that number and the fp32 [slices][M][N] workspace of
 // its partial sums.  The workspace is the call's own: no other work may use it before both of
 // the call's kernels have run.
 int nkb_gemm_slices(int M, int N, int K, long long ldc, int bn_hint);

@@ -126,8 +126,9 @@ struct Gemm {
   int run(const Tensor& like, int* status) const {
     int slices = 1;
     Tensor ws;  // the call's own: the allocator orders its reuse on the stream
-    if (K >= 2048 && epi == NKB_EPI_NONE && !bias && !res &&
-        !(reinterpret_cast<uintptr_t>(c) & (fp32 ? 15 : 7))) {
+    auto at = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
+    if (K >= 2048 && epi == NKB_EPI_NONE && !(at(c) & (fp32 ? 15 : 7)) &&
+        !((at(bias) | at(res)) & 7) && !(ldres & 3)) {
       slices = nkb_gemm_slices((int)M, (int)N, (int)K, ldc, bn);
       if (slices > 1) ws = at::empty({slices * M * N}, of(like, at::kFloat));
     }

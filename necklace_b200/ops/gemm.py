@@ -99,8 +99,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         b = _repack(b)
         pb, ldb = b.data_ptr(), b.stride(0)
     slices, ws = 1, None
-    if K >= 2048 and epi == EPI_NONE and bias is None and res is None \
-            and out.data_ptr() % (16 if fp32 else 8) == 0:
+    if K >= 2048 and epi == EPI_NONE and out.data_ptr() % (16 if fp32 else 8) == 0 \
+            and (bias is None or bias.data_ptr() % 8 == 0) \
+            and (res is None or (res.data_ptr() % 8 == 0 and res.stride(0) % 4 == 0)):
         slices = _lib.value("nkb_gemm_slices", M, N, K, out.stride(0), bn)
         if slices > 1:
             # the partial sums' memory belongs to this call: the allocator orders its reuse on

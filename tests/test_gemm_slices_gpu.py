@@ -63,3 +63,29 @@ def test_reduction_of_few_and_many_slices(M, N, K, fp32):
     bound = want.abs() * 4 * rel + mag * (K + 16) * 2.0 ** -21
     assert bool(((out.double() - 2.5 * want).abs() <= bound).all())
     assert bool((wide[:, N:] == 3).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(333, 1024, 4096), (64, 68, 2048), (129, 260, 4608)])
+@pytest.mark.parametrize("bias,res,pitch,shift", [(True, False, 0, 0), (True, True, 0, 0),
+                                                  (False, True, 4, 0), (True, True, 2, 0),
+                                                  (True, True, 0, 1)])
+def test_slices_with_bias_and_residual(M, N, K, bias, res, pitch, shift):
+    """The kernel that adds the slices adds bias and residual; rows or bases that it cannot read four
+    values at a time go through one slice."""
+    from necklace_b200 import _lib
+    from necklace_b200.ops.gemm import gemm
+    assert _lib.value("nkb_gemm_slices", M, N, K, N, 0) > 1
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    b = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    # (a bias is contiguous in any case; rows of the residual may lie apart)
+    bv = torch.randn(N + shift, generator=g, device="cuda").bfloat16()[shift:] if bias else None
+    r = torch.randn(M, N + pitch, generator=g, device="cuda").bfloat16()[:, :N] if res else None
+    want, mag = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    if bias:
+        want, mag = want + bv.double(), mag + bv.double().abs()
+    if res:
+        want, mag = want + r.double(), mag + r.double().abs()
+    _close(gemm(a, b, bias=bv, res=r), want, mag, K)
+    out32 = gemm(a, b, bias=bv, res=r, out_dtype=torch.float32)
+    assert bool(((out32.double() - want).abs() <= mag * (K + 16) * 2.0 ** -24).all())
