@@ -27,7 +27,9 @@
 // block's S^T issued after dV and dK a block took 7.6 k cycles (head dim 64), of which the
 // compute is about 2.1 k and the 32 MMAs (at least 60 cycles each) about 2 k.  Causal, 8 x 16
 // heads, 1024 positions, head dim 64: 167 -> 112 us; full, 3 x 12, 1111: 111 -> 73 us; causal,
-// 2 x 32, 2048, head dim 128: 568 (one tile at a time, dQ by atomics) -> 338 us.
+// 2 x 32, 2048, head dim 128: 568 (one tile at a time, dQ by atomics) -> 338 us.  With packed pairs in the
+// compute warps (the staged lse and delta negated for it) another 2 % with head dim 64 (106.8 -> 105.0,
+// 69.3 -> 67.9 us in later timings), nothing with 128.
 //
 // lse / delta of the query block are staged in shared memory (they index columns here),
 // fetched one block ahead.  All waits are bounded.  The reference has no attention layer.
@@ -48,7 +50,7 @@ struct AttnBwd2Smem {
   static constexpr int DO_OFF = Q_OFF + QST * TILE;
   static constexpr int DS_OFF = DO_OFF + OST * TILE;  // 32 KB (dS^T, two 64-query sub-tiles)
   static constexpr int DQ_OFF = DS_OFF + 32768;   // 32 KB fp32 staging (two 32-column sub-tiles)
-  static constexpr int LD_OFF = DQ_OFF + 32768;   // [2][256] floats: lse*log2e | delta
+  static constexpr int LD_OFF = DQ_OFF + 32768;   // [2][256] floats: -lse*log2e | -delta
   static constexpr int BAR_OFF = LD_OFF + 2048;
   // the buffer starts on 1024 bytes (checked in the kernel): there is no room for slack
   static constexpr int BYTES = BAR_OFF + 256;
@@ -355,11 +357,11 @@ attn_bwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int r = (warp & 3) * 32 + lane;    // key row inside the block (TMEM lane)
     const int tid = threadIdx.x;             // 0..255
     const uint32_t t_lane = tmem_base + (uint32_t((warp & 3) * 32) << 16);
-    // lse * log2(e) (threads 0-127) / delta (threads 128-255) of query (block, tid & 127)
+    // -lse * log2(e) (threads 0-127) / -delta (threads 128-255) of query (block, tid & 127)
     auto fetch_ld = [&](int it) -> float {
       const int qi = (i0 + it) * 128 + (tid & 127);
-      if (qi >= a.S) return tid < 128 ? INFINITY : 0.f;
-      return tid < 128 ? a.lse[bh_off + qi] * LOG2E : a.delta[bh_off + qi];
+      if (qi >= a.S) return tid < 128 ? -INFINITY : 0.f;
+      return tid < 128 ? -(a.lse[bh_off + qi] * LOG2E) : -a.delta[bh_off + qi];
     };
     if (niter > 0) {
       sLD[tid] = fetch_ld(0);
@@ -393,14 +395,20 @@ attn_bwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       __syncwarp();
       if (lane == 0) mbar_arrive(s_read);
       const bool diag = a.causal && i == j;
+      const f32x2_t scale2 = f2_pack(a.scale_log2, a.scale_log2);
       float p[64];
 #pragma unroll
       for (int e = 0; e < 64; e += 4) {
         const float4 l4 = *reinterpret_cast<const float4*>(sL + e);
-        p[e] = ex2_f32(fmaf(__uint_as_float(s[e]), a.scale_log2, -l4.x));
-        p[e + 1] = ex2_f32(fmaf(__uint_as_float(s[e + 1]), a.scale_log2, -l4.y));
-        p[e + 2] = ex2_f32(fmaf(__uint_as_float(s[e + 2]), a.scale_log2, -l4.z));
-        p[e + 3] = ex2_f32(fmaf(__uint_as_float(s[e + 3]), a.scale_log2, -l4.w));
+        float x0, x1, x2, x3;
+        f2_unpack(f2_fma(f2_pack(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), scale2,
+                         f2_pack(l4.x, l4.y)), x0, x1);
+        f2_unpack(f2_fma(f2_pack(__uint_as_float(s[e + 2]), __uint_as_float(s[e + 3])), scale2,
+                         f2_pack(l4.z, l4.w)), x2, x3);
+        p[e] = ex2_f32(x0);
+        p[e + 1] = ex2_f32(x1);
+        p[e + 2] = ex2_f32(x2);
+        p[e + 3] = ex2_f32(x3);
       }
       if (diag) {  // key r may only see queries >= r
 #pragma unroll
@@ -455,11 +463,14 @@ attn_bwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const float4 d0 = *reinterpret_cast<const float4*>(sDl + hf * 32 + q * 8);
           const float4 d1 = *reinterpret_cast<const float4*>(sDl + hf * 32 + q * 8 + 4);
           const uint32_t* v = dp + q * 8;
-          *reinterpret_cast<uint4*>(ds_tile + sw128_off(r, hf * 4 + q)) = make_uint4(
-              pack_bf16x2(pe[0] * (__uint_as_float(v[0]) - d0.x), pe[1] * (__uint_as_float(v[1]) - d0.y)),
-              pack_bf16x2(pe[2] * (__uint_as_float(v[2]) - d0.z), pe[3] * (__uint_as_float(v[3]) - d0.w)),
-              pack_bf16x2(pe[4] * (__uint_as_float(v[4]) - d1.x), pe[5] * (__uint_as_float(v[5]) - d1.y)),
-              pack_bf16x2(pe[6] * (__uint_as_float(v[6]) - d1.z), pe[7] * (__uint_as_float(v[7]) - d1.w)));
+          auto ds2 = [&](int e, float n0, float n1) {  // P^T (dP^T - delta), two columns
+            return f2_to_bf16x2(f2_mul(
+                f2_pack(pe[e], pe[e + 1]),
+                f2_add(f2_pack(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), f2_pack(n0, n1))));
+          };
+          *reinterpret_cast<uint4*>(ds_tile + sw128_off(r, hf * 4 + q)) =
+              make_uint4(ds2(0, d0.x, d0.y), ds2(2, d0.z, d0.w), ds2(4, d1.x, d1.y),
+                         ds2(6, d1.z, d1.w));
         }
       }
       tmem_st_wait();

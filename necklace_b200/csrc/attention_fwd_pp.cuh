@@ -24,6 +24,8 @@
 //     O rescaled through tcgen05.ld / st) when it grew by more than 2^8 since the last
 //     move; until then probabilities are taken against the older maximum, which keeps
 //     them below 256 and leaves the result unchanged after the final division.
+//   * The exponents and the row sums are packed pairs (half of the instructions, the same bits): causal,
+//     40 heads, 4001 positions, D = 128 247 -> 235 us, 8 x 16, 1024, D = 64 52.9 -> 51.3.
 //   * EXPM 0: fp32 ex2 per element; EXPM 1: packed half ex2 (two per MUFU op).
 //
 // All waits are bounded; a failed wait sets the status word and the abort flag.
@@ -286,15 +288,16 @@ attn_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       }
       const float mneg = -m_ref * a.scale_log2;
-      float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+      const f32x2_t scale2 = f2_pack(a.scale_log2, a.scale_log2), mneg2 = f2_pack(mneg, mneg);
+      f32x2_t sum01 = f2_pack(0.f, 0.f), sum23 = sum01;
       uint32_t pk[64];
 #pragma unroll
       for (int i = 0; i < 128; i += 4) {
-        const float x0 = fmaf(__uint_as_float(s[i]), a.scale_log2, mneg);
-        const float x1 = fmaf(__uint_as_float(s[i + 1]), a.scale_log2, mneg);
-        const float x2 = fmaf(__uint_as_float(s[i + 2]), a.scale_log2, mneg);
-        const float x3 = fmaf(__uint_as_float(s[i + 3]), a.scale_log2, mneg);
-        float p0, p1, p2, p3;
+        float x0, x1, x2, x3, p0, p1, p2, p3;
+        f2_unpack(f2_fma(f2_pack(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), scale2, mneg2),
+                  x0, x1);
+        f2_unpack(f2_fma(f2_pack(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3])), scale2,
+                         mneg2), x2, x3);
         if (EXPM == 0) {
           p0 = ex2_f32(x0);
           p1 = ex2_f32(x1);
@@ -304,10 +307,8 @@ attn_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           unpack_f16x2(ex2_f16x2(x0, x1), p0, p1);
           unpack_f16x2(ex2_f16x2(x2, x3), p2, p3);
         }
-        sum0 += p0;
-        sum1 += p1;
-        sum2 += p2;
-        sum3 += p3;
+        sum01 = f2_add(sum01, f2_pack(p0, p1));
+        sum23 = f2_add(sum23, f2_pack(p2, p3));
         pk[i >> 1] = pack_bf16x2(p0, p1);
         pk[(i >> 1) + 1] = pack_bf16x2(p2, p3);
       }
@@ -317,8 +318,8 @@ attn_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_st_32x16(t_p + c * 16, pk + c * 16);
-      sum0 += sum2;
-      sum1 += sum3;
+      float sum0, sum1;
+      f2_unpack(f2_add(sum01, sum23), sum0, sum1);
       l += sum0 + sum1;
       tmem_st_wait();
       tc_fence_before();
