@@ -105,14 +105,13 @@ def build_ops(force: bool = False) -> bool:
     """Compile the operators on tensors; whether there are any.  Without them the operators do the
     same in Python, so a failure is a warning."""
     import torch
-    from torch.utils import cpp_extension
-    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    root = os.path.dirname(torch.__file__)
     flags = [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
-    for d in [*cpp_extension.include_paths(), os.path.join(cuda, "include")]:
+    for d in (os.path.join(root, "include"),
+              os.path.join(root, "include", "torch", "csrc", "api", "include"),
+              os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")):
         flags += ["-isystem", d]
-    for d in cpp_extension.library_paths():
-        flags += ["-L", d]
-    flags += ["-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    flags += ["-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
     return _build_extension(OPS, "pytensor.cpp", flags, force,
                             "operators take the way through Python")
 
