@@ -69,7 +69,7 @@ inline int allow_smem(K kern, int bytes, bool (&done)[64]) {
 // 134 -> 125 us; the 2-bit codec's two kernels 71.7 -> 68.7 us, ResNet-50 over 37 images 1.86 -> 1.80
 // ms, its training step of 256 images 23.3 -> 22.97 ms.  A graph being captured gets plain edges: the
 // same step's graph takes 22.1 ms with those and 22.6 with programmatic ones (memory-bound kernels,
-// whose CTAs start early wherever an SM is free, end up unevenly spread), and 1.0 s for 0.45 to build.
+// whose CTAs start early wherever an SM is free, end up unevenly spread).
 __device__ __forceinline__ void grid_dep_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
